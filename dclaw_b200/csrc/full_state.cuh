@@ -161,13 +161,17 @@ DC_HD bool full_b4(const dclaw_params& P, const Geom& g, const double* __restric
     return nan;
 }
 
-// Stage B. calc_taudir on the bed less the bed change
+// Stage B. calc_taudir on the bed less the bed change, and tau of the rpn2
+// states. The two tau planes lie where the x-fluxes go later in the step
+// (the solves, which read them, come before the fluxes).
+DC_HD double* full_tau(const WorkF& W) { return W.fx; }
+
 DC_HD void full_taudir(const dclaw_params& P, const Geom& g, const WorkF& W, int i, int j) {
     const WorkF w = W;
-    taudir_cell(P, g, W.qB, W.npad, W.td, [w](size_t q) { return w.beff(q); }, i, j);
+    taudir_cell(P, g, W.qB, W.npad, W.td, [w](size_t q) { return w.beff(q); }, i, j, full_tau(W));
 }
 
-// solver side after one or two rpn2 qfix passes, with chi (load_side)
+// solver side after one or two rpn2 qfix passes, with chi (load_side_sv)
 DC_HD Side full_load_side(const dclaw_params& P, const WorkF& W, size_t pi, int comp_n, int comp_t, bool twice,
                           int taudir_plane) {
     Side s;
@@ -196,9 +200,8 @@ DC_HD Side full_load_side(const dclaw_params& P, const WorkF& W, size_t pi, int 
     s.h = h; s.hn = hn; s.ht = ht; s.hm = hm; s.p = p; s.m = m; s.chi = chi;
     s.un = hn / h;
     s.ut = ht / h;
-    SetVars sv = setvars<false>(P, P.phi, h, s.un, s.ut, m, p, P.grav);
-    s.rho_sv = sv.rho;
-    s.tau_sv = sv.tau;
+    s.rho_sv = m * (P.rho_s - P.rho_f) + P.rho_f;
+    s.tau_sv = full_tau(W)[(twice ? W.npad : 0) + pi];
     return s;
 }
 

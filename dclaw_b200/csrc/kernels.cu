@@ -107,6 +107,28 @@ constexpr int SRC2_MINB = DCLAW_PLAIN_CELL_MINB * 256 / DCLAW_SRC2_TPB;
 constexpr int RECORDS_TPB = DCLAW_RECORDS_TPB;
 constexpr int RECORDS_MINB = DCLAW_PLAIN_CELL_MINB * 256 / DCLAW_RECORDS_TPB;
 
+// Threads per CTA, and resident CTAs the registers are sized for, of the
+// staged per-interface kernels (patch calls, full state), which wait on
+// FP64 latency. Their solves and fluxes need 125-160 registers: CTAs of 256
+// threads left one CTA (8 warps) on an SM as soon as a kernel passed 128.
+// With 128 threads and 128 registers, and tau once per cell, two 1024^2
+// steps of the full state take 1.22 ms (1.68 before) and two 500 x 300
+// rounds of the patch calls 0.39 ms (0.48). 3, 5 and 6 CTAs for the solves
+// and fluxes, and 64 threads, came out 0-6 % slower.
+#ifndef DCLAW_STAGE_TPB
+#define DCLAW_STAGE_TPB 128
+#endif
+#ifndef DCLAW_STAGE_SOLVE_MINB
+#define DCLAW_STAGE_SOLVE_MINB 4
+#endif
+#ifndef DCLAW_STAGE_FLUX_MINB
+#define DCLAW_STAGE_FLUX_MINB 4
+#endif
+#ifndef DCLAW_STAGE_FINAL_MINB
+#define DCLAW_STAGE_FINAL_MINB 4
+#endif
+constexpr int STAGE_TPB = DCLAW_STAGE_TPB;
+
 __device__ __forceinline__ double warp_max(double v) {
     for (int o = 16; o > 0; o >>= 1) {
         double w = __shfl_xor_sync(0xffffffffu, v, o);
@@ -126,6 +148,17 @@ __device__ __forceinline__ void block_max_to(double v, unsigned long long* acc) 
         double x = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
         x = warp_max(x);
         if (lane == 0 && x > 0.0) atomicMax(acc, (unsigned long long)__double_as_longlong(x));
+    }
+}
+
+// warp-wide max of a non-negative value into *acc, with an atomic only where
+// it raises *acc: no barrier, so a warp of dry interfaces leaves its SM
+// without waiting for the wet ones of its CTA
+__device__ __forceinline__ void warp_max_to(double v, unsigned long long* acc) {
+    v = warp_max(v);
+    if ((threadIdx.x & 31) == 0 && v > 0.0) {
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+        if (bits > *(volatile unsigned long long*)acc) atomicMax(acc, bits);
     }
 }
 
@@ -227,15 +260,6 @@ __device__ __forceinline__ bool tile_active(const uint32_t* __restrict__ tflag, 
 }
 
 // ---- fused step (interior layout) -----------------------------------------
-__global__ void __launch_bounds__(TPB) k_b4(dclaw_params P, Geom g, const double* __restrict__ q_in,
-                                            const double* __restrict__ b, Work W, dclaw_clock* clk) {
-    const long long n = (long long)g.PX * g.PY;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n) return;
-    int i = (int)(idx % g.PX) - 1, j = (int)(idx / g.PX) - 1;
-    if (stage_b4(P, g, q_in, b, W, i, j)) flag_status(clk, DCLAW_ERR_NAN);
-}
-
 __global__ void __launch_bounds__(TPB) k_taudir(dclaw_params P, Geom g, Work W, int inner_only) {
     const long long n = (long long)g.PX * g.PY;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -245,9 +269,17 @@ __global__ void __launch_bounds__(TPB) k_taudir(dclaw_params P, Geom g, Work W, 
     stage_taudir(P, g, W, i, j);
 }
 
+// tau of every wet padded cell's two rpn2 states, for the solves: one setvars
+// a cell instead of one per interface side
+__global__ void __launch_bounds__(STAGE_TPB) k_taus(dclaw_params P, Work W, double* __restrict__ tau) {
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx < (long long)W.npad) cell_taus(P, W.qB, W.npad, (size_t)idx, tau);
+}
+
 template <int DIR>
-__global__ void __launch_bounds__(TPB) k_riemann(dclaw_params P, Geom g, Work W, dclaw_clock* clk,
-                                                 uint32_t* __restrict__ brlog) {
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_riemann(dclaw_params P, Geom g, Work W,
+                                                                              const double* __restrict__ tau,
+                                                                              double dt, dclaw_clock* clk) {
     // DIR 0: rows r = 0..my+1, interfaces i = 0..mx+2 (x fastest)
     // DIR 1: interfaces k = 0..my+2, columns c = 0..mx+1 (column fastest)
     const int nfast = DIR == 0 ? g.mx + 3 : g.mx + 2;
@@ -256,57 +288,31 @@ __global__ void __launch_bounds__(TPB) k_riemann(dclaw_params P, Geom g, Work W,
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double cflv = 0.0;
     if (idx < n) {
-        int a = (int)(idx % nfast), s = (int)(idx / nfast);
+        int a, s;
+        split_index(idx, nfast, a, s);
         int r = DIR == 0 ? s : a;   // slice
         int i = DIR == 0 ? a : s;   // interface along the slice
         const int nlen = DIR == 0 ? g.mx : g.my;
-        uint32_t bits = 0;
-        double smax = stage_riemann<DIR>(P, g, W, r, i, &bits);
-        if (i >= 1 && i <= nlen + 1) {
-            const double dt = clk->dt;
-            const double dtdx = DIR == 0 ? dt / g.dx : dt / g.dy;
-            cflv = dtdx * smax;
-            if (brlog) {
-                size_t off = DIR == 0 ? (size_t)r * (g.mx + 1) + (size_t)(i - 1)
-                                      : (size_t)(g.my + 2) * (g.mx + 1) + (size_t)r * (g.my + 1) + (size_t)(i - 1);
-                brlog[off] = bits;
-            }
-        }
+        double smax = stage_riemann<DIR>(P, g, W, r, i, nullptr, tau, 1);
+        if (i >= 1 && i <= nlen + 1) cflv = (DIR == 0 ? dt / g.dx : dt / g.dy) * smax;
         if (!(cflv == cflv)) cflv = 0.0;
     }
-    block_max_to(cflv, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
+    warp_max_to(cflv, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
 }
 
 template <int DIR>
-__global__ void __launch_bounds__(TPB) k_flux(dclaw_params P, Geom g, Work W, const dclaw_clock* clk,
-                                              uint32_t* __restrict__ brlog) {
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_flux(dclaw_params P, Geom g, Work W, double dt) {
     // DIR 0: rows 0..my+1, interfaces 1..mx+1; DIR 1: interfaces 1..my+1, columns 0..mx+1
     const int nfast = DIR == 0 ? g.mx + 1 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 1;
     const long long n = (long long)nfast * nslow;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
-    int a = (int)(idx % nfast), s = (int)(idx / nfast);
+    int a, s;
+    split_index(idx, nfast, a, s);
     int r = DIR == 0 ? s : a;
     int i = DIR == 0 ? a + 1 : s + 1;
-    const double dt = clk->dt;
-    const double dtdx = DIR == 0 ? dt / g.dx : dt / g.dy;
-    uint32_t bits = 0;
-    stage_flux<DIR>(P, g, W, r, i, dtdx, brlog ? &bits : nullptr);
-    if (brlog) {
-        size_t off = DIR == 0 ? (size_t)r * (g.mx + 1) + (size_t)(i - 1)
-                              : (size_t)(g.my + 2) * (g.mx + 1) + (size_t)r * (g.my + 1) + (size_t)(i - 1);
-        brlog[off] |= bits;
-    }
-}
-
-__global__ void __launch_bounds__(TPB) k_final(dclaw_params P, Geom g, Work W, double* __restrict__ q_out,
-                                               dclaw_clock* clk) {
-    const long long n = (long long)g.mx * g.my;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n) return;
-    int i = (int)(idx % g.mx) + 1, j = (int)(idx / g.mx) + 1;
-    if (stage_finalize(P, g, W, q_out, i, j, clk->dt)) flag_status(clk, DCLAW_ERR_NAN);
+    stage_flux<DIR>(P, g, W, r, i, DIR == 0 ? dt / g.dx : dt / g.dy, nullptr);
 }
 
 // ---- the full-state step (segregation, entrainment) -------------------------
@@ -356,7 +362,7 @@ __global__ void __launch_bounds__(TPB) k_full_taudir(dclaw_params P, Geom g, Wor
 }
 
 template <int DIR>
-__global__ void __launch_bounds__(TPB) k_full_riemann(dclaw_params P, Geom g, WorkF W, dclaw_clock* clk,
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_full_riemann(dclaw_params P, Geom g, WorkF W, dclaw_clock* clk,
                                                       uint32_t* __restrict__ brlog,
                                                       const uint32_t* __restrict__ tflag) {
     const int nfast = DIR == 0 ? g.mx + 3 : g.mx + 2;
@@ -365,7 +371,8 @@ __global__ void __launch_bounds__(TPB) k_full_riemann(dclaw_params P, Geom g, Wo
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double cflv = 0.0;
     if (idx < n) {
-        int a = (int)(idx % nfast), s = (int)(idx / nfast);
+        int a, s;
+        split_index(idx, nfast, a, s);
         int r = DIR == 0 ? s : a;
         int i = DIR == 0 ? a : s;
         const int nlen = DIR == 0 ? g.mx : g.my;
@@ -390,18 +397,19 @@ __global__ void __launch_bounds__(TPB) k_full_riemann(dclaw_params P, Geom g, Wo
             if (!(cflv == cflv)) cflv = 0.0;
         }
     }
-    block_max_to(cflv, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
+    warp_max_to(cflv, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
 }
 
 template <int DIR>
-__global__ void __launch_bounds__(TPB) k_full_flux(dclaw_params P, Geom g, WorkF W, const dclaw_clock* clk,
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_full_flux(dclaw_params P, Geom g, WorkF W, const dclaw_clock* clk,
                                                    uint32_t* __restrict__ brlog, const uint32_t* __restrict__ tflag) {
     const int nfast = DIR == 0 ? g.mx + 1 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 1;
     const long long n = (long long)nfast * nslow;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
-    int a = (int)(idx % nfast), s = (int)(idx / nfast);
+    int a, s;
+    split_index(idx, nfast, a, s);
     int r = DIR == 0 ? s : a;
     int i = DIR == 0 ? a + 1 : s + 1;
     // read by the updates of cells i-1, i along the slice, one slice either side
@@ -422,7 +430,7 @@ __global__ void __launch_bounds__(TPB) k_full_flux(dclaw_params P, Geom g, WorkF
     }
 }
 
-__global__ void __launch_bounds__(TPB) k_full_final(dclaw_params P, Geom g, WorkF W, const double* __restrict__ he,
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_full_final(dclaw_params P, Geom g, WorkF W, const double* __restrict__ he,
                                                     double* __restrict__ q_out, dclaw_clock* clk,
                                                     const uint32_t* __restrict__ tflag);
 
@@ -515,14 +523,19 @@ __device__ __forceinline__ void last_block_tick(const dclaw_params& P, dclaw_clo
     }
 }
 
-// update + src2 of the full state; the last block applies the tick
-__global__ void __launch_bounds__(TPB) k_full_final(dclaw_params P, Geom g, WorkF W, const double* __restrict__ he,
+// update + src2 of the full state; the tick is a launch of its own (a block
+// that counts itself finished holds its dry warps at a barrier until its wet
+// ones are through src2: 1.25 against 1.22 ms for two steps at 1024^2)
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_full_final(dclaw_params P, Geom g, WorkF W, const double* __restrict__ he,
                                                     double* __restrict__ q_out, dclaw_clock* clk,
                                                     const uint32_t* __restrict__ tflag) {
     const long long n = (long long)g.mx * g.my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < n) {
-        int i = (int)(idx % g.mx) + 1, j = (int)(idx / g.mx) + 1;
+        int i, j;
+        split_index(idx, g.mx, i, j);
+        i += 1;
+        j += 1;
         if (tflag && !full_any_active(tflag, clk->nsteps + 1u, g, i, i, j, j)) {
             // a cell of an inactive tile: zero, its eroded depth passed through
             const size_t plane = (size_t)g.mx * g.my;
@@ -532,7 +545,6 @@ __global__ void __launch_bounds__(TPB) k_full_final(dclaw_params P, Geom g, Work
             flag_status(clk, DCLAW_ERR_NAN);
         }
     }
-    last_block_tick(P, clk);
 }
 
 // One tile of the fused step (all threads of the CTA call it). smem holds
@@ -1209,7 +1221,7 @@ __global__ void __launch_bounds__(TPB) k_b4_padded(dclaw_params P, int mx, int m
     q[idx] = h; q[npad + idx] = hu; q[2 * npad + idx] = hv; q[3 * npad + idx] = hm; q[4 * npad + idx] = p;
 }
 
-__global__ void __launch_bounds__(TPB) k_update_padded(Geom g, Work W, double dt, double* q, double* fluxes,
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_update_padded(Geom g, Work W, double dt, double* q, double* fluxes,
                                                        dclaw_clock* clk) {
     const long long n = (long long)g.mx * g.my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1231,7 +1243,7 @@ __global__ void __launch_bounds__(TPB) k_update_padded(Geom g, Work W, double dt
     }
 }
 
-__global__ void __launch_bounds__(TPB) k_src2_padded(dclaw_params P, int mx, int my, double dt, double* q) {
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_src2_padded(dclaw_params P, int mx, int my, double dt, double* q) {
     const long long n = (long long)mx * my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
@@ -1329,6 +1341,7 @@ __global__ void k_cfl_from_bits(dclaw_clock* clk) {
 
 // ---- host helpers ----------------------------------------------------------
 inline unsigned nblocks(long long n) { return (unsigned)((n + TPB - 1) / TPB); }
+inline unsigned stage_blocks(long long n) { return (unsigned)((n + STAGE_TPB - 1) / STAGE_TPB); }
 inline unsigned src2_blocks(long long n) { return (unsigned)((n + SRC2_TPB - 1) / SRC2_TPB); }
 
 struct Layout : StagedLayout {
@@ -1841,14 +1854,17 @@ int dclaw_step2(double* q, const double* aux, int mx, int my, int mbc, double dx
     W.qB = q;
     W.bP = const_cast<double*>(aux);
     W.td = const_cast<double*>(aux) + 3 * L.npad;
-    // the kernels read dt from the clock: use a clock set to this dt
+    // the caller reads cflgrid from the clock: a clock set to this dt
     k_clock_init<<<1, 32, 0, s>>>(clock, 0.0, dt, 0.0, 1);
     const dclaw_params P = *p;
-    k_riemann<0><<<nblocks((long long)L.nxi), TPB, 0, s>>>(P, g, W, clock, nullptr);
-    k_riemann<1><<<nblocks((long long)(mx + 2) * (my + 3)), TPB, 0, s>>>(P, g, W, clock, nullptr);
-    k_flux<0><<<nblocks((long long)(mx + 1) * (my + 2)), TPB, 0, s>>>(P, g, W, clock, nullptr);
-    k_flux<1><<<nblocks((long long)(mx + 2) * (my + 1)), TPB, 0, s>>>(P, g, W, clock, nullptr);
-    k_update_padded<<<nblocks((long long)mx * my), TPB, 0, s>>>(g, W, dt, q, fluxes, clock);
+    // the tau planes lie where the x-fluxes go after the solves have read them
+    double* tau = W.fx;
+    k_taus<<<stage_blocks((long long)L.npad), STAGE_TPB, 0, s>>>(P, W, tau);
+    k_riemann<0><<<stage_blocks((long long)L.nxi), STAGE_TPB, 0, s>>>(P, g, W, tau, dt, clock);
+    k_riemann<1><<<stage_blocks((long long)L.nyi), STAGE_TPB, 0, s>>>(P, g, W, tau, dt, clock);
+    k_flux<0><<<stage_blocks((long long)(mx + 1) * (my + 2)), STAGE_TPB, 0, s>>>(P, g, W, dt);
+    k_flux<1><<<stage_blocks((long long)(mx + 2) * (my + 1)), STAGE_TPB, 0, s>>>(P, g, W, dt);
+    k_update_padded<<<stage_blocks((long long)mx * my), STAGE_TPB, 0, s>>>(g, W, dt, q, fluxes, clock);
     k_cfl_from_bits<<<1, 32, 0, s>>>(clock);
     return cuda_status();
 }
@@ -1859,7 +1875,7 @@ int dclaw_src2(double* q, const double* aux, int mx, int my, int mbc, double dx,
     if (!q || !p || mbc != 2 || !sizes_ok(mx, my)) return DCLAW_ERR_ARG;
     int rc = dclaw_params_check_5(p);
     if (rc) return rc;
-    k_src2_padded<<<nblocks((long long)mx * my), TPB, 0, (cudaStream_t)stream>>>(*p, mx, my, dt, q);
+    k_src2_padded<<<stage_blocks((long long)mx * my), STAGE_TPB, 0, (cudaStream_t)stream>>>(*p, mx, my, dt, q);
     return cuda_status();
 }
 
@@ -1959,11 +1975,12 @@ int dclaw_step_full(const double* q_in, double* q_out, const double* b, const do
     const long long npad = (long long)g.PX * g.PY;
     k_full_b4<<<nblocks(npad), TPB, 0, s>>>(P, g, q_in, b, W, clock, tflag);
     k_full_taudir<<<nblocks(npad), TPB, 0, s>>>(P, g, W);
-    k_full_riemann<0><<<nblocks((long long)(mx + 3) * (my + 2)), TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_riemann<1><<<nblocks((long long)(mx + 2) * (my + 3)), TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_flux<0><<<nblocks((long long)(mx + 1) * (my + 2)), TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_flux<1><<<nblocks((long long)(mx + 2) * (my + 1)), TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_final<<<nblocks((long long)mx * my), TPB, 0, s>>>(P, g, W, h_e, q_out, clock, tflag);
+    k_full_riemann<0><<<stage_blocks((long long)(mx + 3) * (my + 2)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
+    k_full_riemann<1><<<stage_blocks((long long)(mx + 2) * (my + 3)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
+    k_full_flux<0><<<stage_blocks((long long)(mx + 1) * (my + 2)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
+    k_full_flux<1><<<stage_blocks((long long)(mx + 2) * (my + 1)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
+    k_full_final<<<stage_blocks((long long)mx * my), STAGE_TPB, 0, s>>>(P, g, W, h_e, q_out, clock, tflag);
+    k_tick<<<1, 32, 0, s>>>(P, clock);
     return cuda_status();
 }
 

@@ -104,21 +104,49 @@ DC_HD bool stage_b4(const dclaw_params& P, const Geom& g, const double* __restri
 }
 
 // ---------------------------------------------------------------------------
+// tau of a wet cell's two rpn2 states, once per cell instead of once per
+// interface side (setvars, with its atan, tan and tanh, is over half of an
+// interface's work when both sides evaluate it): plane 0 after one qfix pass
+// (A1), plane 1 after two (A2). setvars reads the velocity only through
+// u^2 + v^2, so one value serves both sweep directions.
+// put_taus: from the state after the first pass and its tau1.
+DC_HD void put_taus(const dclaw_params& P, double h, double u, double v, double hm, double p, double m, double tau1,
+                    size_t npad, size_t pi, double* tau) {
+    const double m1 = m, p1 = p;
+    qfix_mp(P, h, hm, p, m, P.grav);
+    tau[pi] = tau1;
+    tau[npad + pi] = m == m1 && p == p1 ? tau1 : setvars<false>(P, P.phi, h, u, v, m, p, P.grav).tau;
+}
+
+// cell_taus: from the b4step2 state's padded planes; a dry cell has none
+DC_HD void cell_taus(const dclaw_params& P, const double* __restrict__ qB, size_t npad, size_t pi, double* tau) {
+    const double h = qB[pi];
+    if (h <= P.dry_tolerance) return;
+    double hm = qB[3 * npad + pi], p = qB[4 * npad + pi], m;
+    qfix_mp(P, h, hm, p, m, P.grav);
+    const double u = qB[npad + pi] / h, v = qB[2 * npad + pi] / h;
+    put_taus(P, h, u, v, hm, p, m, setvars<false>(P, P.phi, h, u, v, m, p, P.grav).tau, npad, pi, tau);
+}
+
+// ---------------------------------------------------------------------------
 // Stage B. calc_taudir on cell (i, j) of the padded patch. Cells of the outer
 // ghost ring keep fsphi = taudir = 0 (setaux zeroes them, calc_taudir covers
 // only 2-mbc..m+mbc-1).
 // qB: the b4step2 state's padded planes (h, hu, hv, hm, pb first), td the
 // three output planes, bed(pi) the bed of padded cell pi (the bed less the
-// bed change on the full state: digclaw_module.f90:555-613).
+// bed change on the full state: digclaw_module.f90:555-613). tau (nullable):
+// two planes that receive tau of the cell's rpn2 states where it is wet
+// (cell_taus).
 template <typename Bed>
 DC_HD void taudir_cell(const dclaw_params& P, const Geom& g, const double* __restrict__ qB, size_t npad,
-                       double* td, Bed bed, int i, int j) {
+                       double* td, Bed bed, int i, int j, double* tau = nullptr) {
     const size_t pi = pidx(g, i, j);
     double* fs = td;
     double* tx = td + npad;
     double* ty = td + 2 * npad;
     if (i < 0 || j < 0 || i > g.mx + 1 || j > g.my + 1) {
         fs[pi] = 0.0; tx[pi] = 0.0; ty[pi] = 0.0;
+        if (tau) cell_taus(P, qB, npad, pi, tau);
         return;
     }
     const double dry = P.dry_tolerance;
@@ -151,6 +179,7 @@ DC_HD void taudir_cell(const dclaw_params& P, const Geom& g, const double* __res
     double u, v, m;
     qfix(P, h, hu, hv, hm, p, u, v, m, gz);
     SetVars sv = setvars<false>(P, P.phi, h, u, v, m, p, gz);
+    if (tau && h > 0.0) put_taus(P, h, u, v, hm, p, m, sv.tau, npad, pi, tau);
     const double dx = g.dx, dy = g.dy;
     const double sint = 0.0;  // sin(theta), theta = 0
     double FxL = -gz * 0.5 * (h + hL) * (eta - etaL) / (dx) + gz * 0.5 * (h + hL) * sint;
@@ -232,9 +261,11 @@ constexpr int SV_N = 8;
 constexpr int NSV = 2 * SV_N;
 enum { SV_TAU = 0, SV_DH, SV_DU, SV_DV, SV_DM, SV_DP, SV_DPHI, SV_DMU };
 
-// load_side with tau read from the record instead of recomputed (same bits)
+// load_side with tau read from a record instead of recomputed (same bits):
+// plane 0 of sv after one qfix pass, plane `second` after two (SV_N in the
+// adjoint's records, 1 in cell_taus' planes)
 DC_HD Side load_side_sv(const dclaw_params& P, const Work& W, const double* __restrict__ sv, size_t pi,
-                        int comp_n, int comp_t, bool twice, int taudir_plane) {
+                        int comp_n, int comp_t, bool twice, int taudir_plane, int second = SV_N) {
     Side s;
     double h = W.qB[pi];
     s.b = W.bP[pi];
@@ -257,17 +288,17 @@ DC_HD Side load_side_sv(const dclaw_params& P, const Work& W, const double* __re
     s.un = hn / h;
     s.ut = ht / h;
     s.rho_sv = m * (P.rho_s - P.rho_f) + P.rho_f;
-    s.tau_sv = sv[(size_t)((twice ? SV_N : 0) + SV_TAU) * W.npad + pi];
+    s.tau_sv = sv[(size_t)(twice ? second : 0) * W.npad + pi];
     return s;
 }
 
 // Stage C. Interface `i` (0..n+2) of slice `r` (x: row 0..my+1; y: column
 // 0..mx+1). Writes the compact waves; returns max |s| over the waves for the
-// Courant number and ORs branch bits into *br (nullable). sv (nullable):
-// setvars records to read tau from instead of recomputing it.
+// Courant number and ORs branch bits into *br (nullable). sv (nullable), second:
+// the records load_side_sv reads tau from instead of recomputing it.
 template <int DIR>
 DC_HD double stage_riemann(const dclaw_params& P, const Geom& g, const Work& W, int r, int i, uint32_t* br,
-                           const double* __restrict__ sv = nullptr) {
+                           const double* __restrict__ sv = nullptr, int second = SV_N) {
     size_t pL, pR, oi;
     double* wv;
     size_t nplane;
@@ -284,8 +315,9 @@ DC_HD double stage_riemann(const dclaw_params& P, const Geom& g, const Work& W, 
         zero_waves(w);
         if (br) *br |= BR_DRY;
     } else {
-        Side R = sv ? load_side_sv(P, W, sv, pR, cn, ct, false, 1 + DIR) : load_side(P, W, pR, cn, ct, false, 1 + DIR);
-        Side L = sv ? load_side_sv(P, W, sv, pL, cn, ct, i - 1 >= 0, 1 + DIR)
+        Side R = sv ? load_side_sv(P, W, sv, pR, cn, ct, false, 1 + DIR, second)
+                    : load_side(P, W, pR, cn, ct, false, 1 + DIR);
+        Side L = sv ? load_side_sv(P, W, sv, pL, cn, ct, i - 1 >= 0, 1 + DIR, second)
                     : load_side(P, W, pL, cn, ct, i - 1 >= 0, 1 + DIR);
         w = riemann_solve(P, L, R, br);
     }
