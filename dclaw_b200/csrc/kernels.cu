@@ -764,7 +764,8 @@ __global__ void __launch_bounds__(TPB, DCLAW_SCAN_MINB) k_scan_patch(dclaw_param
                                                                     unsigned int* counters,
                                                                     uint32_t* __restrict__ tflag, size_t s0,
                                                                     size_t s1, size_t z0, size_t z1) {
-    if (blockIdx.x == 0 && threadIdx.x < 3) counters[threadIdx.x] = 0u;  // tile queue and list lengths
+    // tile queue, list lengths, src2method 2's cell counter
+    if (blockIdx.x == 0 && threadIdx.x < 6) counters[threadIdx.x] = 0u;
     const size_t n = (size_t)mx * my;
     const int ntx = (mx + TILE_X - 1) / TILE_X, nty = (my + TILE_Y - 1) / TILE_Y;
     const size_t lo = s0 < z0 ? s0 : z0, hi = s1 > z1 ? s1 : z1;
@@ -888,6 +889,108 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_list(dclaw_params 
     if (tick) last_block_tick(P, clk);
 }
 
+// src2 of the active tiles' cells with src2method 2. A cell takes between 1
+// and 100 substeps (2.4 on average over the flows in motion that were
+// counted, 16 in the 99th percentile; the longest lie within 4 dry tolerances
+// of dry), so a warp bound to 32 cells mostly waits for its longest one. Here
+// a lane that is done takes the next cell of all the active tiles' from a
+// counter. Cells are started and finished when `refill` lanes of the warp
+// wait for it, so that those parts (friction, with its setvars, and the
+// stores) run on many lanes at once. The counter passes over the cells
+// twice, the shallow ones first: the longest of them takes 300 us by itself
+// (5900 cycles a substep, a chain of divisions and roots), and a warp that
+// holds such cells takes no others until they are through. On the 777 x 1024
+// flow in motion two steps take 1.61 ms, 2.28 ms with k_src2_list (with
+// the quadrants' shared evaluations in mp_update_fe4quad; 1.68 ms without
+// them, 1.67 ms without the shallow pass). A queue of wet cells per warp, so
+// that it starts 28 of them at once, took 1.80 ms: what is left is latency,
+// and fewer, fuller warps hide less of it.
+#ifndef DCLAW_QUAD_REFILL
+#define DCLAW_QUAD_REFILL 16
+#endif
+#ifndef DCLAW_QUAD_SHALLOW
+#define DCLAW_QUAD_SHALLOW 6.0
+#endif
+#ifndef DCLAW_QUAD_TPB
+#define DCLAW_QUAD_TPB 128
+#endif
+#ifndef DCLAW_QUAD_MINB
+#define DCLAW_QUAD_MINB 4
+#endif
+constexpr double QUAD_SHALLOW = DCLAW_QUAD_SHALLOW;  // in dry tolerances
+__global__ void __launch_bounds__(DCLAW_QUAD_TPB, DCLAW_QUAD_MINB) k_src2_quad_list(
+    dclaw_params P, Geom g, const double* __restrict__ q_star, double* __restrict__ q_out, dclaw_clock* clk,
+    unsigned int* counters, const uint32_t* __restrict__ list_act, int tick) {
+    constexpr unsigned CELLS = TILE_X * TILE_Y;
+    const unsigned long long ncell = (unsigned long long)counters[1] * CELLS;
+    const uint32_t ntx = (uint32_t)((g.mx + TILE_X - 1) / TILE_X);
+    const size_t plane = (size_t)g.mx * g.my;
+    const double dt = clk->dt;
+    const int lane = threadIdx.x & 31;
+    unsigned long long* next = reinterpret_cast<unsigned long long*>(counters + 4);
+    Src2State s;
+    size_t c = 0;
+    bool busy = false, done = false;  // in its substeps; through them
+    // the same for the whole warp: cells may be left to take, idle lanes that
+    // make it refill
+    bool left = true;
+    int refill = 1;
+    auto put = [&](double a, double b, double d, double e, double f) {
+        q_out[c] = a;
+        q_out[plane + c] = b;
+        q_out[2 * plane + c] = d;
+        q_out[3 * plane + c] = e;
+        q_out[4 * plane + c] = f;
+    };
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !busy);
+        if (idle == 0xffffffffu || (left && __popc(idle) >= refill)) {
+            if (done) {
+                double a, b, d, e, f;
+                src2_substeps_end(P, s);
+                src2_end(P, dt, s, a, b, d, e, f);
+                put(a, b, d, e, f);
+                done = false;
+            }
+            if (!left) break;  // every lane is idle and has stored its cell
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(next, (unsigned long long)__popc(idle));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            left = base + __popc(idle) < 2 * ncell;
+            refill = base < ncell ? 32 : DCLAW_QUAD_REFILL;
+            unsigned long long k = base + __popc(idle & ((1u << lane) - 1u));
+            const bool deep = k >= ncell;
+            if (deep) k -= ncell;
+            if (!busy && k < ncell) {
+                const uint32_t t = list_act[k / CELLS];
+                const int o = (int)(k % CELLS);
+                const int i = 1 + (int)(t % ntx) * TILE_X + o % TILE_X, j = 1 + (int)(t / ntx) * TILE_Y + o / TILE_X;
+                if (i <= g.mx && j <= g.my) {
+                    c = (size_t)(j - 1) * g.mx + (size_t)(i - 1);
+                    double a = q_star[c];
+                    // a dry cell keeps the zeros k_scan_patch wrote
+                    if (!(a <= P.dry_tolerance) && (a > QUAD_SHALLOW * P.dry_tolerance) == deep) {
+                        double b = q_star[plane + c], d = q_star[2 * plane + c], e = q_star[3 * plane + c],
+                               f = q_star[4 * plane + c];
+                        if (src2_begin(P, P.phi, dt, a, b, d, e, f, s)) {
+                            busy = src2_more(s);
+                            done = !busy;
+                        } else {
+                            put(a, b, d, e, f);
+                        }
+                    }
+                }
+            }
+            continue;
+        }
+        if (busy) {
+            busy = src2_substep(P, P.phi, s);
+            done = !busy;
+        }
+    }
+    if (tick) last_block_tick(P, clk);
+}
+
 // ---- batched ensemble -------------------------------------------------------
 // the ensemble's tile shapes: 14 x 13 (the single patch's), 13 x 14, 16 x 14
 constexpr int NBATCH_SHAPES = 3;
@@ -991,7 +1094,8 @@ __global__ void __launch_bounds__(TPB, DCLAW_SCAN_MINB) k_scan_batch(int nmem, u
                                                     const double* __restrict__ q_in, double* __restrict__ q_out,
                                                     unsigned int* counters, uint32_t* __restrict__ tflag, int TX,
                                                     int TY) {
-    if (blockIdx.x == 0 && threadIdx.x < 3) counters[threadIdx.x] = 0u;  // tile queue and list lengths
+    // tile queue, list lengths, src2method 2's cell counter
+    if (blockIdx.x == 0 && threadIdx.x < 6) counters[threadIdx.x] = 0u;
     int m = -1;
     for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         m = member_of(nmem, nchunks, ch, m, [&](int k) { return mem[k].schunk0; });
@@ -1397,6 +1501,21 @@ inline int ensure_tile_smem_attr() {
     return DCLAW_OK;
 }
 
+// src2 over the active list (g3: k_src2_list's grid)
+inline void launch_src2_list(const dclaw_params& P, const Geom& g, const double* qstar, double* q_out,
+                             dclaw_clock* clock, unsigned int* counters, const uint32_t* list_act, unsigned g3,
+                             int nsm, unsigned ntiles, int tick, cudaStream_t s) {
+    if (P.src2method == 2) {
+        const unsigned long long all =
+            ((unsigned long long)ntiles * (TILE_X * TILE_Y) + DCLAW_QUAD_TPB - 1) / DCLAW_QUAD_TPB;
+        const unsigned most = (unsigned)(nsm * DCLAW_QUAD_MINB);
+        k_src2_quad_list<<<all < most ? (unsigned)all : most, DCLAW_QUAD_TPB, 0, s>>>(P, g, qstar, q_out, clock, counters,
+                                                                           list_act, tick);
+        return;
+    }
+    k_src2_list<<<g3, SRC2_TPB, 0, s>>>(P, g, qstar, q_out, clock, counters, list_act, tick);
+}
+
 inline bool sizes_ok(int mx, int my) {
     return mx >= 2 && my >= 2 && (long long)(mx + 4) * (my + 4) < (1LL << 40);
 }
@@ -1635,7 +1754,7 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
         k_tile_list<false><<<g2, TILE_TPB, TG::SMEM_BYTES, s>>>(P, g, R, b, qstar, clock, counters, list_act);
         unsigned g3 = (unsigned)(nsm * SRC2_MINB);
         if (g3 > ntiles) g3 = ntiles;
-        k_src2_list<<<g3, SRC2_TPB, 0, s>>>(P, g, qstar, q_out, clock, counters, list_act);
+        launch_src2_list(P, g, qstar, q_out, clock, counters, list_act, g3, nsm, ntiles, 1, s);
         return cuda_status();
     }
     k_records<<<nblocks((long long)L.npad), TPB, 0, s>>>(P, g, q_in, b, R, clock, tflag);
@@ -1794,7 +1913,7 @@ int dclaw_step_rows(const double* q_in, double* q_out, const double* b, int mx, 
     k_tile_list<false><<<g2, TILE_TPB, TG::SMEM_BYTES, s>>>(P, g, R, b, qstar, clock, counters, list_act);
     unsigned g3 = (unsigned)(sm * SRC2_MINB);
     if (g3 > ntiles) g3 = ntiles;
-    k_src2_list<<<g3, SRC2_TPB, 0, s>>>(P, g, qstar, q_out, clock, counters, list_act, 0);
+    launch_src2_list(P, g, qstar, q_out, clock, counters, list_act, g3, sm, ntiles, 0, s);
     return cuda_status();
 }
 

@@ -718,183 +718,226 @@ DC_BIG double mp_update_fe4quad(const dclaw_params& P, double phi, double dtr, d
     else if ((m > m_c) && (p <= p_eq_c)) quad0 = 3;
     else if ((m <= m_c) && (p < p_eq_c)) quad0 = 4;
     if (quad0 == 0) return 0.0;
-    // p_exc(t) = (1/kp0) ((kp0 p_exc0 - c_d0) e^{-kp0 t} + c_d0)
-    auto pexc_at = [&](double t) { return (1.0 / kp0) * ((kp0 * p_exc0 - c_d0) * em::d_exp(-kp0 * t) + c_d0); };
-    double dtm, dtp, dts, p_exc_ave;
-    if (quad0 == 1) {
-        if (p_exc0 < -1.0e-3 * rhoh * gz) {  // region 1A
-            if (c_d0 > 0.0) dtp = -(1.0 / kp0) * em::d_log(c_d0 / (c_d0 - kp0 * p_exc0));
-            else dtp = dtr;
-            dtm = em::d_log(0.98) / (kp0 * p_exc0);
+    // The quadrants' regions. They differ in what goes into one logarithm (the
+    // time p_exc takes to an isocline), one quotient (the time m takes), the
+    // time p_exc(t) is taken at and the update of m; written as operands
+    // chosen per region, the lanes of a warp share those evaluations whatever
+    // regions their cells are in.
+    enum { R1A, R1B, R1CL, R1CR, R2, R3A, R3B, R3CB, R3CL, R4 };
+    // the p-nullcline's side (also written -kp0 p_exc0 + c_d0, the same value)
+    const double side = c_d0 - kp0 * p_exc0;
+    int reg;
+    if (quad0 == 1) reg = p_exc0 < -1.0e-3 * rhoh * gz ? R1A : side > 0.0 ? R1B : c_d0 > 0.0 ? R1CL : R1CR;
+    else if (quad0 == 2) reg = R2;
+    else if (quad0 == 3) reg = p_exc0 > 1.0e-3 * rhoh * gz ? R3A : side < 0.0 ? R3B : c_d0 < 0.0 ? R3CB : R3CL;
+    else reg = R4;
+    // dtp: dtr, or -(1/kp0) log(num / side) where the region takes it
+    double num = c_d0;
+    if (reg == R1B) num = -kp0 * rhoh * gz + kp0 * p_eq_c + c_d0;
+    else if (reg == R2 || reg == R4) num = c_d0 - kp0 * (p_eq_c - p_eq0);
+    else if (reg == R3B) num = c_d0 + kp0 * p_eq0;
+    const double ratio = num / side;
+    bool take;
+    switch (reg) {
+        case R1A: take = c_d0 > 0.0; break;
+        case R1B: take = (c_d0 / kp0) > (rhoh * gz - p_eq_c); break;
+        case R1CR:
+            take = (kp0 * p_exc0 - c_d0) != 0.0 && (-kp0 * p_eq0 - c_d0) / (kp0 * p_exc0 - c_d0) > 1.0e-99;
+            break;
+        case R2: case R3A: case R4: take = ratio > 1.0e-99; break;
+        case R3B: take = c_d0 / kp0 < -p_eq0 && ratio > 1.0e-99; break;
+        case R3CL: take = (-c_d0 / (kp0 * p_exc0 - c_d0)) > 1.0e-99; break;
+        default: take = false; break;
+    }
+    double dtp = dtr;
+    if (take) {
+        const double t = -(1.0 / kp0) * em::d_log(ratio);
+        dtp = reg == R1A || reg == R3CL ? t : fmin2(dtr, t);
+    }
+    // dtm: from K, m's rate at p_exc0 (or kp0 p_exc0 with log 0.98)
+    const bool log98 = reg == R1A || reg == R4;
+    const double K = log98 ? kp0 * p_exc0 : km0 * p_exc0 * m_0;
+    const double way = log98 ? em::d_log(0.98) : reg == R2 || reg == R3A ? fmin2(1.0 - m_0, 0.02) : m_c - m_0;
+    const double mtime = way / K;
+    double dtm = dtp, dts, t_p;
+    switch (reg) {
+        case R1A:
+            dtm = mtime;
             dts = fmin2(fmin2(dtr, dtp), dtm);
             dts = fmax2(dts, 0.0);
-            p_exc = pexc_at(dts);
-            m = m_0 * em::d_exp(dts * km0 * p_exc);
-        } else if ((-kp0 * p_exc0 + c_d0) > 0.0) {  // region 1B
-            if ((c_d0 / kp0) > (rhoh * gz - p_eq_c))
-                dtp = fmin2(dtr, -(1.0 / kp0) * em::d_log((-kp0 * rhoh * gz + kp0 * p_eq_c + c_d0) / (-kp0 * p_exc0 + c_d0)));
-            else
-                dtp = dtr;
-            p_exc = pexc_at(dtp);
-            p_exc_ave = 0.5 * (p_exc + p_exc0);
-            if (p_exc_ave <= 0.0) dtm = dtr;
-            else if ((km0 * p_exc_ave * m_0) < 1.0e-99) dtm = dtp;
-            else dtm = fmin2(dtp, (m_eq - m_0) / (km0 * p_exc_ave * m_0));
-            m = m_0 + km0 * m_0 * p_exc_ave * dtm;
-            dts = dtm;
-        } else if (c_d0 > 0.0) {  // region 1C, left of m_eq
-            dtp = dtr;
-            if ((km0 * p_exc0 * m_0) > 1.0e-99) dtm = (m_c - m_0) / (km0 * p_exc0 * m_0);
-            else dtm = dtp;
+            t_p = dts;
+            break;
+        case R1CL:  // left of m_eq
+            if (K > 1.0e-99) dtm = mtime;
             dts = fmin2(dtm, dtp);
             dts = fmax2(dts, 0.0);
-            m = m_0 + km0 * m_0 * p_exc0 * dts;
-            p_exc = pexc_at(dts);
-        } else {  // region 1C, right of m_eq
+            t_p = dts;
+            break;
+        case R1CR:  // right of m_eq
             dts = dtr;
-            dtp = dtr;
-            if ((km0 * p_exc0 * m_0) > 1.0e-99) dts = fmin2(dtr, (m_c - m_0) / (km0 * p_exc0 * m_0));
-            if ((kp0 * p_exc0 - c_d0) != 0.0) {
-                if ((-kp0 * p_eq0 - c_d0) / (kp0 * p_exc0 - c_d0) > 1.0e-99)
-                    dtp = fmin2(dtr, -(1.0 / kp0) * em::d_log((c_d0) / (c_d0 - kp0 * p_exc0)));
-            }
+            if (K > 1.0e-99) dts = fmin2(dtr, mtime);
             dts = fmin2(dts, dtp);
             dts = fmax2(dts, 0.0);
-            m = m_0 + km0 * m_0 * p_exc0 * dts;
-            p_exc = pexc_at(dts);
-        }
-    } else if (quad0 == 2) {
-        dtp = dtr;
-        if ((c_d0 - kp0 * (p_eq_c - p_eq0)) / (c_d0 - kp0 * p_exc0) > 1.0e-99)
-            dtp = fmin2(dtr, -(1.0 / kp0) * em::d_log((c_d0 - kp0 * (p_eq_c - p_eq0)) / (c_d0 - kp0 * p_exc0)));
-        dtm = dtp;
-        if (km0 * p_exc0 * m_0 > 1.0e-99) dtm = fmin2(dtp, (fmin2(1.0 - m_0, 0.02) / (km0 * p_exc0 * m_0)));
-        dts = fmin2(dtp, dtm);
-        p_exc = pexc_at(dts);
-        m = m_0 + km0 * m_0 * p_exc * dts;
-    } else if (quad0 == 3) {
-        if (p_exc0 > 1.0e-3 * rhoh * gz) {  // region 3A
-            dtp = dtr;
-            if ((c_d0 / (-kp0 * p_exc0 + c_d0)) > 1.0e-99)
-                dtp = fmin2(dtr, -(1.0 / kp0) * em::d_log(c_d0 / (c_d0 - kp0 * p_exc0)));
-            dtm = dtp;
-            if ((km0 * p_exc0 * m_0) > 1.0e-99) dtm = fmin2(dtp, (fmin2(1.0 - m_0, 0.02)) / (km0 * p_exc0 * m_0));
-            p_exc = pexc_at(dtp);
-            m = m_0 + km0 * m_0 * 0.5 * (p_exc0 + p_exc) * dtm;
+            t_p = dts;
+            break;
+        case R2:
+            if (K > 1.0e-99) dtm = fmin2(dtp, mtime);
+            dts = fmin2(dtp, dtm);
+            t_p = dts;
+            break;
+        case R3A:
+            if (K > 1.0e-99) dtm = fmin2(dtp, mtime);
             dts = dtp;
-        } else if ((-kp0 * p_exc0 + c_d0) < 0.0) {  // region 3B
-            dtp = dtr;
-            if (c_d0 / kp0 < -p_eq0) {
-                if (((c_d0 + kp0 * p_eq0) / (-kp0 * p_exc0 + c_d0)) > 1.0e-99)
-                    dtp = fmin2(dtr, -(1.0 / kp0) * em::d_log((c_d0 + kp0 * p_eq0) / (-kp0 * p_exc0 + c_d0)));
-            }
-            p_exc = pexc_at(dtp);
-            p_exc_ave = 0.5 * (p_exc + p_exc0);
-            if (p_exc_ave > 0.0) {
-                dtm = fmin2(dtr, (0.02) / (km0 * p_exc_ave * m_0));
-            } else {
-                const double m_lower = m_eq + fmax2(0.0, (1.0 / 3.0) * kp0 * h0 * (-p_exc_ave) / (vnorm * sv.alphainv));
-                dtm = fmin2(dtr, (m_lower - m_0) / (km0 * p_exc_ave * m_0));
-            }
-            m = m_0 + km0 * m_0 * p_exc_ave * dtm;
-            dts = dtm;
-        } else if (c_d0 < 0.0) {  // region 3C, between the p-nullcline and m_eq
-            dtp = dtr;
+            t_p = dtp;
+            break;
+        case R3CB:  // between the p-nullcline and m_eq
+        case R3CL:  // left of m_eq
             dtm = dtr;
-            if (-(km0 * p_exc0 * m_0) > 1.0e-99) dtm = (m_c - m_0) / (km0 * p_exc0 * m_0);
+            if ((reg == R3CB ? -K : K) > 1.0e-99) dtm = mtime;
             dts = fmin2(dtp, dtm);
             dts = fmax2(dts, 0.0);
-            p_exc = pexc_at(dts);
-            m = m_0 + km0 * m_0 * p_exc0 * dts;
-        } else {  // region 3C, left of m_eq
-            dtm = dtr;
-            dtp = dtr;
-            if ((km0 * p_exc0 * m_0) > 1.0e-99) dtm = (m_c - m_0) / (km0 * p_exc0 * m_0);
-            if ((-c_d0 / (kp0 * p_exc0 - c_d0)) > 1.0e-99) dtp = -(1.0 / kp0) * em::d_log(c_d0 / (c_d0 - kp0 * p_exc0));
-            dts = fmin2(dtp, dtm);
-            dts = fmax2(dts, 0.0);
-            p_exc = pexc_at(dts);
-            m = m_0 + km0 * m_0 * p_exc0 * dts;
+            t_p = dts;
+            break;
+        case R4:
+            dtm = mtime;
+            dts = fmin2(dtr, fmin2(dtp, dtm));
+            t_p = dts;
+            break;
+        default:  // R1B, R3B: dtm follows from p_exc's average
+            dts = dtp;
+            t_p = dtp;
+            break;
+    }
+    // p_exc(t) = (1/kp0) ((kp0 p_exc0 - c_d0) e^{-kp0 t} + c_d0)
+    p_exc = (1.0 / kp0) * ((kp0 * p_exc0 - c_d0) * em::d_exp(-kp0 * t_p) + c_d0);
+    if (reg == R1B || reg == R3B) {
+        const double p_exc_ave = 0.5 * (p_exc + p_exc0);
+        const double rate = km0 * p_exc_ave * m_0;
+        if (reg == R1B) {
+            if (p_exc_ave <= 0.0) dtm = dtr;
+            else if (rate < 1.0e-99) dtm = dtp;
+            else dtm = fmin2(dtp, (m_eq - m_0) / rate);
+        } else if (p_exc_ave > 0.0) {
+            dtm = fmin2(dtr, (0.02) / rate);
+        } else {
+            const double m_lower = m_eq + fmax2(0.0, (1.0 / 3.0) * kp0 * h0 * (-p_exc_ave) / (vnorm * sv.alphainv));
+            dtm = fmin2(dtr, (m_lower - m_0) / rate);
         }
-    } else {  // quad0 == 4
-        dtp = dtr;
-        if ((c_d0 - kp0 * (p_eq_c - p_eq0)) / (c_d0 - kp0 * p_exc0) > 1.0e-99)
-            dtp = fmin2(dtr, -(1.0 / kp0) * em::d_log((c_d0 - kp0 * (p_eq_c - p_eq0)) / (c_d0 - kp0 * p_exc0)));
-        dtm = em::d_log(0.98) / (kp0 * p_exc0);
-        dts = fmin2(dtr, fmin2(dtp, dtm));
-        p_exc = pexc_at(dts);
-        m = m_0 * em::d_exp(dts * km0 * 0.5 * (p_exc0 + p_exc));
-        dts = dtp;  // the reference reports dtp as the time covered
+        m = m_0 + km0 * m_0 * p_exc_ave * dtm;
+        dts = dtm;
+    } else if (log98) {
+        m = m_0 * em::d_exp(reg == R1A ? dts * km0 * p_exc : dts * km0 * 0.5 * (p_exc0 + p_exc));
+        if (reg == R4) dts = dtp;  // the reference reports dtp as the time covered
+    } else if (reg == R2) {
+        m = m_0 + km0 * m_0 * p_exc * dts;
+    } else if (reg == R3A) {
+        m = m_0 + km0 * m_0 * 0.5 * (p_exc0 + p_exc) * dtm;
+    } else {
+        m = m_0 + km0 * m_0 * p_exc0 * dts;
     }
     qfix_cmass(P, h, m, p, rho, p_exc, hu, hv, hm, u, v, rhoh, gz);
     return dts;
 }
 
-// src2 on one interior cell (in place on the 5 conserved fields)
-DC_BIG void src2_cell(const dclaw_params& P, double phi, double dt, double& qh, double& qhu,
-                                          double& qhv, double& qhm, double& qp) {
-    double h = qh;
-    if (h <= P.dry_tolerance) {
+// src2 on one interior cell, in the parts a kernel may run apart: the
+// friction (src2_begin), the substeps of src2method 2 (src2_substep) and what
+// follows them (src2_end).
+struct Src2State {
+    double h, hu, hv, hm, p, u, v, m, rhoh;
+    double left;   // src2method 2: the time its substeps have yet to cover
+    int count;     // and the substeps taken
+};
+
+// dry (q zeroed), or returned as it is (hm < 0): false; else true, with the
+// state after friction in s
+DC_HD bool src2_begin(const dclaw_params& P, double phi, double dt, double& qh, double& qhu, double& qhv, double& qhm,
+                      double& qp, Src2State& s) {
+    s.h = qh;
+    if (s.h <= P.dry_tolerance) {
         qh = 0.0; qhu = 0.0; qhv = 0.0; qhm = 0.0; qp = 0.0;
-        return;
+        return false;
     }
-    double hu = qhu, hv = qhv, hm = qhm, p = qp;
-    double rhoh = hm * P.rho_s + (h - hm) * P.rho_f;
-    if (hm < 0.0) return;
+    s.hu = qhu; s.hv = qhv; s.hm = qhm; s.p = qp;
+    s.rhoh = s.hm * P.rho_s + (s.h - s.hm) * P.rho_f;
+    if (s.hm < 0.0) return false;
     const double gz = P.grav;
     const double gx = 0.0;
-    double u, v, m;
-    qfix(P, h, hu, hv, hm, p, u, v, m, gz);
-    SetVars sv = setvars<false>(P, phi, h, u, v, m, p, gz);
-    double hvnorm0 = sqrt(sq(hu) + sq(hv));
-    double vnorm = hvnorm0 / h;
+    qfix(P, s.h, s.hu, s.hv, s.hm, s.p, s.u, s.v, s.m, gz);
+    SetVars sv = setvars<false>(P, phi, s.h, s.u, s.v, s.m, s.p, gz);
+    double hvnorm0 = sqrt(sq(s.hu) + sq(s.hv));
+    double vnorm = hvnorm0 / s.h;
     if (hvnorm0 > 0.0) {
-        vnorm = fmax2(0.0, vnorm - dt * sv.tau / rhoh);
-        vnorm = vnorm * em::d_exp(-(1.0 - m) * 2.0 * P.mu * dt / (h * rhoh));
-        double hvnorm = h * vnorm;
-        hu = hvnorm * hu / hvnorm0 + gx * h * dt;
-        hv = hvnorm * hv / hvnorm0;
-        u = hu / h;
-        v = hv / h;
+        vnorm = fmax2(0.0, vnorm - dt * sv.tau / s.rhoh);
+        vnorm = vnorm * em::d_exp(-(1.0 - s.m) * 2.0 * P.mu * dt / (s.h * s.rhoh));
+        double hvnorm = s.h * vnorm;
+        s.hu = hvnorm * s.hu / hvnorm0 + gx * s.h * dt;
+        s.hv = hvnorm * s.hv / hvnorm0;
+        s.u = s.hu / s.h;
+        s.v = s.hv / s.h;
     }
-    if (P.src2method == -1) {
-        hu = h * u; hv = h * v; hm = h * m;
-    } else if (P.src2method == 2) {
-        // src2.f90:206-229: substeps until dt is covered, at most 100
-        double dtremaining = dt;
-        int itercount = 0;
-        while (dtremaining > 1.0e-99) {
-            const double dtk = mp_update_fe4quad(P, phi, dtremaining, h, u, v, m, p, rhoh, gz);
-            dtremaining = dtremaining - dtk;
-            itercount = itercount + 1;
-            if (dtk == 0.0) break;
-            if (h < P.dry_tolerance) break;
-            if (itercount >= 100) break;
-        }
-        hu = h * u; hv = h * v; hm = h * m;
-        qfix(P, h, hu, hv, hm, p, u, v, m, gz);
-    } else {
-        mp_update_relax(P, phi, dt, h, u, v, m, p, rhoh, gz);
-        hu = h * u; hv = h * v; hm = h * m;
-    }
-    if (h <= P.dry_tolerance) {
+    s.left = dt;
+    s.count = 0;
+    return true;
+}
+
+// one substep of src2method 2 (src2.f90:206-229: until dt is covered, at most
+// 100); whether another follows
+DC_HD bool src2_more(const Src2State& s) { return s.left > 1.0e-99; }
+DC_HD bool src2_substep(const dclaw_params& P, double phi, Src2State& s) {
+    const double dtk = mp_update_fe4quad(P, phi, s.left, s.h, s.u, s.v, s.m, s.p, s.rhoh, P.grav);
+    s.left = s.left - dtk;
+    s.count = s.count + 1;
+    if (dtk == 0.0) return false;
+    if (s.h < P.dry_tolerance) return false;
+    if (s.count >= 100) return false;
+    return src2_more(s);
+}
+
+// after the substeps of src2method 2
+DC_HD void src2_substeps_end(const dclaw_params& P, Src2State& s) {
+    s.hu = s.h * s.u; s.hv = s.h * s.v; s.hm = s.h * s.m;
+    qfix(P, s.h, s.hu, s.hv, s.hm, s.p, s.u, s.v, s.m, P.grav);
+}
+
+DC_HD void src2_end(const dclaw_params& P, double dt, Src2State& s, double& qh, double& qhu, double& qhv, double& qhm,
+                    double& qp) {
+    if (s.h <= P.dry_tolerance) {
         qh = 0.0; qhu = 0.0; qhv = 0.0; qhm = 0.0; qp = 0.0;
         return;
     }
     if (P.friction_forcing && P.manning_coefficient > 0.0) {
-        if (h <= P.friction_depth) {
+        if (s.h <= P.friction_depth) {
             double cm = P.manning_coefficient;
             if (P.dd_manning)
-                cm = P.manning_max + (P.manning_coefficient - P.manning_max) * 0.5 * (1.0 + em::d_tanh(300.0 * (h - 0.05)));
+                cm = P.manning_max +
+                     (P.manning_coefficient - P.manning_max) * 0.5 * (1.0 + em::d_tanh(300.0 * (s.h - 0.05)));
             double beta = 1.0;
-            double gamma = beta * sqrt(sq(hu) + sq(hv)) * (gz * sq(cm)) / (em::d_pow_7_3(h));
+            double gamma = beta * sqrt(sq(s.hu) + sq(s.hv)) * (P.grav * sq(cm)) / (em::d_pow_7_3(s.h));
             double dgamma = 1.0 + dt * gamma;
-            hu = hu / dgamma;
-            hv = hv / dgamma;
-            qfix(P, h, hu, hv, hm, p, u, v, m, gz);
+            s.hu = s.hu / dgamma;
+            s.hv = s.hv / dgamma;
+            qfix(P, s.h, s.hu, s.hv, s.hm, s.p, s.u, s.v, s.m, P.grav);
         }
     }
-    qh = h; qhu = hu; qhv = hv; qhm = hm; qp = p;
+    qh = s.h; qhu = s.hu; qhv = s.hv; qhm = s.hm; qp = s.p;
+}
+
+// the whole of src2 (in place on the 5 conserved fields)
+DC_BIG void src2_cell(const dclaw_params& P, double phi, double dt, double& qh, double& qhu, double& qhv, double& qhm,
+                      double& qp) {
+    Src2State s;
+    if (!src2_begin(P, phi, dt, qh, qhu, qhv, qhm, qp, s)) return;
+    if (P.src2method == -1) {
+        s.hu = s.h * s.u; s.hv = s.h * s.v; s.hm = s.h * s.m;
+    } else if (P.src2method == 2) {
+        bool more = src2_more(s);
+        while (more) more = src2_substep(P, phi, s);
+        src2_substeps_end(P, s);
+    } else {
+        mp_update_relax(P, phi, dt, s.h, s.u, s.v, s.m, s.p, s.rhoh, P.grav);
+        s.hu = s.h * s.u; s.hv = s.h * s.v; s.hm = s.h * s.m;
+    }
+    src2_end(P, dt, s, qh, qhu, qhv, qhm, qp);
 }
 
 }  // namespace dclaw
