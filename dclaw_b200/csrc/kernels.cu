@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "full_state.cuh"
+#include "launch.cuh"
 #include "stages.cuh"
 #include "tile.cuh"
 #include "workspace.cuh"
@@ -261,6 +262,7 @@ __device__ __forceinline__ bool tile_active(const uint32_t* __restrict__ tflag, 
 
 // ---- fused step (interior layout) -----------------------------------------
 __global__ void __launch_bounds__(TPB) k_taudir(dclaw_params P, Geom g, Work W, int inner_only) {
+    pdl_wait();
     const long long n = (long long)g.PX * g.PY;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
@@ -272,6 +274,7 @@ __global__ void __launch_bounds__(TPB) k_taudir(dclaw_params P, Geom g, Work W, 
 // tau of every wet padded cell's two rpn2 states, for the solves: one setvars
 // a cell instead of one per interface side
 __global__ void __launch_bounds__(STAGE_TPB) k_taus(dclaw_params P, Work W, double* __restrict__ tau) {
+    pdl_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < (long long)W.npad) cell_taus(P, W.qB, W.npad, (size_t)idx, tau);
 }
@@ -280,6 +283,7 @@ template <int DIR>
 __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_riemann(dclaw_params P, Geom g, Work W,
                                                                               const double* __restrict__ tau,
                                                                               double dt, dclaw_clock* clk) {
+    pdl_wait();
     // DIR 0: rows r = 0..my+1, interfaces i = 0..mx+2 (x fastest)
     // DIR 1: interfaces k = 0..my+2, columns c = 0..mx+1 (column fastest)
     const int nfast = DIR == 0 ? g.mx + 3 : g.mx + 2;
@@ -302,6 +306,7 @@ __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_riemann(d
 
 template <int DIR>
 __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_flux(dclaw_params P, Geom g, Work W, double dt) {
+    pdl_wait();
     // DIR 0: rows 0..my+1, interfaces 1..mx+1; DIR 1: interfaces 1..my+1, columns 0..mx+1
     const int nfast = DIR == 0 ? g.mx + 1 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 1;
@@ -343,6 +348,7 @@ __device__ __forceinline__ bool full_any_active(const uint32_t* __restrict__ tfl
 __global__ void __launch_bounds__(TPB) k_full_b4(dclaw_params P, Geom g, const double* __restrict__ q_in,
                                                  const double* __restrict__ b, WorkF W, dclaw_clock* clk,
                                                  uint32_t* __restrict__ tflag) {
+    pdl_wait();
     const long long n = (long long)g.PX * g.PY;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
@@ -354,6 +360,7 @@ __global__ void __launch_bounds__(TPB) k_full_b4(dclaw_params P, Geom g, const d
 }
 
 __global__ void __launch_bounds__(TPB) k_full_taudir(dclaw_params P, Geom g, WorkF W) {
+    pdl_wait();
     const long long n = (long long)g.PX * g.PY;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
@@ -365,6 +372,7 @@ template <int DIR>
 __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_full_riemann(dclaw_params P, Geom g, WorkF W, dclaw_clock* clk,
                                                       uint32_t* __restrict__ brlog,
                                                       const uint32_t* __restrict__ tflag) {
+    pdl_wait();
     const int nfast = DIR == 0 ? g.mx + 3 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 3;
     const long long n = (long long)nfast * nslow;
@@ -403,6 +411,7 @@ __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_full_riem
 template <int DIR>
 __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_full_flux(dclaw_params P, Geom g, WorkF W, const dclaw_clock* clk,
                                                    uint32_t* __restrict__ brlog, const uint32_t* __restrict__ tflag) {
+    pdl_wait();
     const int nfast = DIR == 0 ? g.mx + 1 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 1;
     const long long n = (long long)nfast * nslow;
@@ -446,6 +455,7 @@ __device__ __forceinline__ double clip_next_dt(const dclaw_clock* clk, double dt
 }
 
 __global__ void k_tick(dclaw_params P, dclaw_clock* clk) {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double cfl = __longlong_as_double((long long)clk->cfl_bits);
     double dt = clk->dt;
@@ -458,6 +468,7 @@ __global__ void k_tick(dclaw_params P, dclaw_clock* clk) {
 }
 
 __global__ void k_clock_init(dclaw_clock* clk, double t, double dt, double t_final, int fixed_dt) {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     clk->t = t;
     clk->t_final = t_final;
@@ -529,6 +540,7 @@ __device__ __forceinline__ void last_block_tick(const dclaw_params& P, dclaw_clo
 __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_full_final(dclaw_params P, Geom g, WorkF W, const double* __restrict__ he,
                                                     double* __restrict__ q_out, dclaw_clock* clk,
                                                     const uint32_t* __restrict__ tflag) {
+    pdl_wait();
     const long long n = (long long)g.mx * g.my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < n) {
@@ -764,6 +776,7 @@ __global__ void __launch_bounds__(TPB, DCLAW_SCAN_MINB) k_scan_patch(dclaw_param
                                                                     unsigned int* counters,
                                                                     uint32_t* __restrict__ tflag, size_t s0,
                                                                     size_t s1, size_t z0, size_t z1) {
+    pdl_wait();
     // tile queue, list lengths, src2method 2's cell counter
     if (blockIdx.x == 0 && threadIdx.x < 6) counters[threadIdx.x] = 0u;
     const size_t n = (size_t)mx * my;
@@ -785,6 +798,7 @@ __global__ void __launch_bounds__(TPB) k_list_patch(int ntx, int nty, const dcla
                                                     const uint32_t* __restrict__ tflag, unsigned int* counters,
                                                     uint32_t* __restrict__ list_act, uint32_t* __restrict__ list_rec,
                                                     int ty0, int ty1) {
+    pdl_wait();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t ntiles = (uint32_t)ntx * (uint32_t)nty;
     const uint32_t epoch = clk->nsteps + 1u;
@@ -814,6 +828,7 @@ __global__ void __launch_bounds__(RECORDS_TPB, RECORDS_MINB) k_records_list(dcla
                                                                             const double* __restrict__ b, Rec R,
                                                                             const unsigned int* counters,
                                                                             const uint32_t* __restrict__ list_rec) {
+    pdl_wait();
     const uint32_t n = counters[2];
     const int ntx = (g.mx + TILE_X - 1) / TILE_X, nty = (g.my + TILE_Y - 1) / TILE_Y;
     for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
@@ -832,6 +847,7 @@ __global__ void __launch_bounds__(TILE_TPB, DCLAW_TILE_MINBLOCKS) k_tile_list(dc
                                                                              double* __restrict__ q_out,
                                                                              dclaw_clock* clk, unsigned int* counters,
                                                                              const uint32_t* __restrict__ list_act) {
+    pdl_wait();
     extern __shared__ double smem[];
     // the tile of this pass and the next one's, claimed at the start of this
     // pass: the barrier that ends a pass also publishes the next index
@@ -874,6 +890,7 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_list(dclaw_params 
                                                                   const unsigned int* counters,
                                                                   const uint32_t* __restrict__ list_act,
                                                                   int tick = 1) {
+    pdl_wait();
     const uint32_t nact = counters[1];
     const uint32_t ntx = (uint32_t)((g.mx + TILE_X - 1) / TILE_X);
     const double dt = clk->dt;
@@ -921,6 +938,7 @@ constexpr double QUAD_SHALLOW = DCLAW_QUAD_SHALLOW;  // in dry tolerances
 __global__ void __launch_bounds__(DCLAW_QUAD_TPB, DCLAW_QUAD_MINB) k_src2_quad_list(
     dclaw_params P, Geom g, const double* __restrict__ q_star, double* __restrict__ q_out, dclaw_clock* clk,
     unsigned int* counters, const uint32_t* __restrict__ list_act, int tick) {
+    pdl_wait();
     constexpr unsigned CELLS = TILE_X * TILE_Y;
     const unsigned long long ncell = (unsigned long long)counters[1] * CELLS;
     const uint32_t ntx = (uint32_t)((g.mx + TILE_X - 1) / TILE_X);
@@ -1038,6 +1056,7 @@ __global__ void __launch_bounds__(TPB) k_list_batch(int nmem, uint32_t ntiles, c
                                                     const dclaw_clock* clocks, const uint32_t* __restrict__ tflag,
                                                     unsigned int* counters, uint32_t* __restrict__ list_act,
                                                     uint32_t* __restrict__ list_rec) {
+    pdl_wait();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     bool act = false, rec = false;
     if (t < ntiles) {
@@ -1072,6 +1091,7 @@ __global__ void __launch_bounds__(BATCH_CELL_TPB, BATCH_CELL_MINB) k_records_til
                                                                               double* __restrict__ work,
                                                                               const unsigned int* counters,
                                                                               const uint32_t* __restrict__ list_rec) {
+    pdl_wait();
     const uint32_t n = counters[2];
     int m = -1;
     for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
@@ -1094,6 +1114,7 @@ __global__ void __launch_bounds__(TPB, DCLAW_SCAN_MINB) k_scan_batch(int nmem, u
                                                     const double* __restrict__ q_in, double* __restrict__ q_out,
                                                     unsigned int* counters, uint32_t* __restrict__ tflag, int TX,
                                                     int TY) {
+    pdl_wait();
     // tile queue, list lengths, src2method 2's cell counter
     if (blockIdx.x == 0 && threadIdx.x < 6) counters[threadIdx.x] = 0u;
     int m = -1;
@@ -1118,6 +1139,7 @@ __global__ void __launch_bounds__(TPB, 2) k_tile_batch(int nmem, uint32_t ntiles
                                                        const double* __restrict__ b, double* __restrict__ work,
                                                        unsigned int* counters, const uint32_t* __restrict__ list_act,
                                                        double* __restrict__ q_out) {
+    pdl_wait();
     extern __shared__ double smem[];
     __shared__ dclaw_member sM;
     __shared__ dclaw_params sP;
@@ -1178,6 +1200,7 @@ __global__ void __launch_bounds__(BATCH_CELL_TPB, BATCH_CELL_MINB) k_src2_batch(
                                                     double* __restrict__ q_out, const double* __restrict__ work,
                                                     const unsigned int* counters,
                                                     const uint32_t* __restrict__ list_act) {
+    pdl_wait();
     const uint32_t nact = counters[1];
     int m = -1;
     for (uint32_t k = blockIdx.x; k < nact; k += gridDim.x) {
@@ -1199,6 +1222,7 @@ __global__ void __launch_bounds__(BATCH_CELL_TPB, BATCH_CELL_MINB) k_src2_batch(
 // every member's tick, after its src2
 __global__ void __launch_bounds__(TPB) k_tick_batch(int nmem, const dclaw_params* __restrict__ prm,
                                                     dclaw_clock* clocks) {
+    pdl_wait();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m < nmem) tick_device(prm[m], clocks + m);
 }
@@ -1227,7 +1251,7 @@ inline int launch_tile_batch(const dclaw_batch* B, const dclaw_member* mem, cons
     if (batch_tile_attr<TX, TY>() != DCLAW_OK) return DCLAW_ERR_CUDA;
     unsigned grid = (unsigned)(nsm * (B->tile_ctas_per_sm > 0 ? B->tile_ctas_per_sm : 2));
     if (grid > B->ntiles) grid = B->ntiles > 0 ? B->ntiles : 1;
-    k_tile_batch<TX, TY><<<grid, TPB, TileGeom<TX, TY>::SMEM_BYTES, s>>>(B->nmembers, B->ntiles, mem, prm, clocks, b,
+    launch_pdl(k_tile_batch<TX, TY>, dim3(grid), dim3(TPB), TileGeom<TX, TY>::SMEM_BYTES, s, B->nmembers, B->ntiles, mem, prm, clocks, b,
                                                                         work, counters, list_act, q_out);
     return DCLAW_OK;
 }
@@ -1241,14 +1265,14 @@ inline int launch_batch_tiles(const dclaw_batch* B, const dclaw_member* mem, con
                               const uint32_t* list_rec, int nsm, int cpsm, cudaStream_t s) {
     unsigned g1 = (unsigned)(nsm * cpsm);
     if (g1 > B->ntiles) g1 = B->ntiles > 0 ? B->ntiles : 1;
-    k_records_tiles_batch<TX, TY><<<g1, BATCH_CELL_TPB, 0, s>>>(B->nmembers, B->ntiles, mem, prm, q_in, b, w, counters,
+    launch_pdl(k_records_tiles_batch<TX, TY>, dim3(g1), dim3(BATCH_CELL_TPB), 0, s, B->nmembers, B->ntiles, mem, prm, q_in, b, w, counters,
                                                                  list_rec);
     int rc = launch_tile_batch<TX, TY>(B, mem, prm, clocks, b, w, counters, list_act, nsm, s, q_out);
     if (rc != DCLAW_OK) return rc;
     if (!DCLAW_BATCH_SRC2_KERNEL) return DCLAW_OK;
     unsigned g3 = (unsigned)(nsm * cpsm);
     if (g3 > B->ntiles) g3 = B->ntiles > 0 ? B->ntiles : 1;
-    k_src2_batch<TX, TY><<<g3, BATCH_CELL_TPB, 0, s>>>(B->nmembers, B->ntiles, mem, prm, clocks, q_out, w, counters,
+    launch_pdl(k_src2_batch<TX, TY>, dim3(g3), dim3(BATCH_CELL_TPB), 0, s, B->nmembers, B->ntiles, mem, prm, clocks, q_out, w, counters,
                                                         list_act);
     return DCLAW_OK;
 }
@@ -1267,6 +1291,7 @@ inline int sm_count() {
 
 // ---- patch calls (padded layout) ------------------------------------------
 __global__ void __launch_bounds__(TPB) k_bc2amr(dclaw_params P, int mx, int my, double* q) {
+    pdl_wait();
     // one thread per padded cell; ghost cells read their source interior cell
     const int PX = mx + 4, PY = my + 4;
     const size_t npad = (size_t)PX * PY;
@@ -1290,6 +1315,7 @@ __global__ void __launch_bounds__(TPB) k_bc2amr(dclaw_params P, int mx, int my, 
 }
 
 __global__ void __launch_bounds__(TPB) k_setaux(dclaw_params P, int mx, int my, double* aux) {
+    pdl_wait();
     const int PX = mx + 4, PY = my + 4;
     const size_t npad = (size_t)PX * PY;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1306,6 +1332,7 @@ __global__ void __launch_bounds__(TPB) k_setaux(dclaw_params P, int mx, int my, 
 }
 
 __global__ void __launch_bounds__(TPB) k_b4_padded(dclaw_params P, int mx, int my, double* q, dclaw_clock* clk) {
+    pdl_wait();
     const int PX = mx + 4, PY = my + 4;
     const size_t npad = (size_t)PX * PY;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1327,6 +1354,7 @@ __global__ void __launch_bounds__(TPB) k_b4_padded(dclaw_params P, int mx, int m
 
 __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_update_padded(Geom g, Work W, double dt, double* q, double* fluxes,
                                                        dclaw_clock* clk) {
+    pdl_wait();
     const long long n = (long long)g.mx * g.my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
@@ -1348,6 +1376,7 @@ __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_update_pa
 }
 
 __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_src2_padded(dclaw_params P, int mx, int my, double dt, double* q) {
+    pdl_wait();
     const long long n = (long long)mx * my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
@@ -1440,6 +1469,7 @@ __global__ void __launch_bounds__(TPB) k_wave_speed(dclaw_params P, int mx, int 
 }
 
 __global__ void k_cfl_from_bits(dclaw_clock* clk) {
+    pdl_wait();
     if (threadIdx.x == 0 && blockIdx.x == 0) clk->cfl = __longlong_as_double((long long)clk->cfl_bits);
 }
 
@@ -1509,11 +1539,11 @@ inline void launch_src2_list(const dclaw_params& P, const Geom& g, const double*
         const unsigned long long all =
             ((unsigned long long)ntiles * (TILE_X * TILE_Y) + DCLAW_QUAD_TPB - 1) / DCLAW_QUAD_TPB;
         const unsigned most = (unsigned)(nsm * DCLAW_QUAD_MINB);
-        k_src2_quad_list<<<all < most ? (unsigned)all : most, DCLAW_QUAD_TPB, 0, s>>>(P, g, qstar, q_out, clock, counters,
+        launch_pdl(k_src2_quad_list, dim3(all < most ? (unsigned)all : most), dim3(DCLAW_QUAD_TPB), 0, s, P, g, qstar, q_out, clock, counters,
                                                                            list_act, tick);
         return;
     }
-    k_src2_list<<<g3, SRC2_TPB, 0, s>>>(P, g, qstar, q_out, clock, counters, list_act, tick);
+    launch_pdl(k_src2_list, dim3(g3), dim3(SRC2_TPB), 0, s, P, g, qstar, q_out, clock, counters, list_act, tick);
 }
 
 inline bool sizes_ok(int mx, int my) {
@@ -1694,7 +1724,7 @@ size_t dclaw_workspace_bytes(int mx, int my) {
 
 int dclaw_clock_init(dclaw_clock* clock, double t, double dt, double t_final, int fixed_dt, void* stream) {
     if (!clock) return DCLAW_ERR_ARG;
-    k_clock_init<<<1, 32, 0, (cudaStream_t)stream>>>(clock, t, dt, t_final, fixed_dt);
+    launch_pdl(k_clock_init, dim3(1), dim3(32), 0, (cudaStream_t)stream, clock, t, dt, t_final, fixed_dt);
     return cuda_status();
 }
 
@@ -1738,20 +1768,20 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
         const unsigned ntiles = (unsigned)ntx * (unsigned)nty;
         unsigned g0 = (unsigned)(nsm * DCLAW_SCAN_MINB * 2);
         if ((long long)g0 * TPB > ncell) g0 = nblocks(ncell);
-        k_scan_patch<<<g0, TPB, 0, s>>>(P, mx, my, q_in, q_out, clock, counters, tflag, 0, (size_t)ncell, 0,
+        launch_pdl(k_scan_patch, dim3(g0), dim3(TPB), 0, s, P, mx, my, q_in, q_out, clock, counters, tflag, 0, (size_t)ncell, 0,
                                         (size_t)ncell);
-        k_list_patch<<<(ntiles + TPB - 1) / TPB, TPB, 0, s>>>(ntx, nty, clock, tflag, counters, list_act, list_rec, 0,
+        launch_pdl(k_list_patch, dim3((ntiles + TPB - 1) / TPB), dim3(TPB), 0, s, ntx, nty, clock, tflag, counters, list_act, list_rec, 0,
                                                              nty - 1);
         unsigned g1 = (unsigned)(nsm * RECORDS_MINB);
         if (g1 > ntiles) g1 = ntiles;
-        k_records_list<<<g1, RECORDS_TPB, 0, s>>>(P, g, q_in, b, R, counters, list_rec);
+        launch_pdl(k_records_list, dim3(g1), dim3(RECORDS_TPB), 0, s, P, g, q_in, b, R, counters, list_rec);
         unsigned g2 = (unsigned)(nsm * DCLAW_TILE_MINBLOCKS);
         if (g2 > ntiles) g2 = ntiles;
         if (!DCLAW_LIST_SRC2_KERNEL) {
-            k_tile_list<true><<<g2, TILE_TPB, TG::SMEM_BYTES, s>>>(P, g, R, b, q_out, clock, counters, list_act);
+            launch_pdl(k_tile_list<true>, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, q_out, clock, counters, list_act);
             return cuda_status();
         }
-        k_tile_list<false><<<g2, TILE_TPB, TG::SMEM_BYTES, s>>>(P, g, R, b, qstar, clock, counters, list_act);
+        launch_pdl(k_tile_list<false>, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock, counters, list_act);
         unsigned g3 = (unsigned)(nsm * SRC2_MINB);
         if (g3 > ntiles) g3 = ntiles;
         launch_src2_list(P, g, qstar, q_out, clock, counters, list_act, g3, nsm, ntiles, 1, s);
@@ -1847,7 +1877,7 @@ int dclaw_step_host(const double* q_in, double* q_out, const double* b, int mx, 
             k_src2_cells<<<src2_blocks(nc), SRC2_TPB, 0, s>>>(P, g, qstar, dq_out, clock, tflag, (long long)(r0 - 1) * mx, nc,
                                                      0);
         }
-        if (k == nb - 1) k_tick<<<1, 32, 0, s>>>(P, clock);
+        if (k == nb - 1) launch_pdl(k_tick, dim3(1), dim3(32), 0, s, P, clock);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaEventRecord(hp->ev_cmp[k], s);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->down, hp->ev_cmp[k], 0);
@@ -1901,16 +1931,16 @@ int dclaw_step_rows(const double* q_in, double* q_out, const double* b, int mx, 
     const long long nscan = (long long)(sb - sa + 1) * mx;
     unsigned g0 = (unsigned)(sm * DCLAW_SCAN_MINB * 2);
     if ((long long)g0 * TPB > nscan) g0 = nblocks(nscan);
-    k_scan_patch<<<g0, TPB, 0, s>>>(P, mx, my, q_in, q_out, clock, counters, tflag, (size_t)(sa - 1) * mx,
+    launch_pdl(k_scan_patch, dim3(g0), dim3(TPB), 0, s, P, mx, my, q_in, q_out, clock, counters, tflag, (size_t)(sa - 1) * mx,
                                     (size_t)sb * mx, (size_t)(row_first - 1) * mx, (size_t)last * mx);
-    k_list_patch<<<(ntiles + TPB - 1) / TPB, TPB, 0, s>>>(ntx, ntyp, clock, tflag, counters, list_act, list_rec, ty0,
+    launch_pdl(k_list_patch, dim3((ntiles + TPB - 1) / TPB), dim3(TPB), 0, s, ntx, ntyp, clock, tflag, counters, list_act, list_rec, ty0,
                                                          ty1);
     unsigned g1 = (unsigned)(sm * RECORDS_MINB);
     if (g1 > ntiles) g1 = ntiles;
-    k_records_list<<<g1, RECORDS_TPB, 0, s>>>(P, g, q_in, b, R, counters, list_rec);
+    launch_pdl(k_records_list, dim3(g1), dim3(RECORDS_TPB), 0, s, P, g, q_in, b, R, counters, list_rec);
     unsigned g2 = (unsigned)(sm * DCLAW_TILE_MINBLOCKS);
     if (g2 > ntiles) g2 = ntiles;
-    k_tile_list<false><<<g2, TILE_TPB, TG::SMEM_BYTES, s>>>(P, g, R, b, qstar, clock, counters, list_act);
+    launch_pdl(k_tile_list<false>, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock, counters, list_act);
     unsigned g3 = (unsigned)(sm * SRC2_MINB);
     if (g3 > ntiles) g3 = ntiles;
     launch_src2_list(P, g, qstar, q_out, clock, counters, list_act, g3, sm, ntiles, 0, s);
@@ -1921,7 +1951,7 @@ int dclaw_clock_tick(dclaw_clock* clock, const dclaw_params* p, void* stream) {
     if (!clock || !p) return DCLAW_ERR_ARG;
     int rc = dclaw_params_check_5(p);
     if (rc) return rc;
-    k_tick<<<1, 32, 0, (cudaStream_t)stream>>>(*p, clock);
+    launch_pdl(k_tick, dim3(1), dim3(32), 0, (cudaStream_t)stream, *p, clock);
     return cuda_status();
 }
 
@@ -1929,13 +1959,13 @@ int dclaw_bc2amr(double* q, int mx, int my, int mbc, const dclaw_params* p, void
     if (!q || !p || mbc != 2 || !sizes_ok(mx, my)) return DCLAW_ERR_ARG;
     int rc = dclaw_params_check_5(p);
     if (rc) return rc;
-    k_bc2amr<<<nblocks((long long)(mx + 4) * (my + 4)), TPB, 0, (cudaStream_t)stream>>>(*p, mx, my, q);
+    launch_pdl(k_bc2amr, dim3(nblocks((long long)(mx + 4) * (my + 4))), dim3(TPB), 0, (cudaStream_t)stream, *p, mx, my, q);
     return cuda_status();
 }
 
 int dclaw_setaux(double* aux, int mx, int my, int mbc, const dclaw_params* p, void* stream) {
     if (!aux || !p || mbc != 2 || !sizes_ok(mx, my)) return DCLAW_ERR_ARG;
-    k_setaux<<<nblocks((long long)(mx + 4) * (my + 4)), TPB, 0, (cudaStream_t)stream>>>(*p, mx, my, aux);
+    launch_pdl(k_setaux, dim3(nblocks((long long)(mx + 4) * (my + 4))), dim3(TPB), 0, (cudaStream_t)stream, *p, mx, my, aux);
     return cuda_status();
 }
 
@@ -1947,14 +1977,14 @@ int dclaw_b4step2(double* q, double* aux, int mx, int my, int mbc, double dx, do
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t npad = (size_t)(mx + 4) * (my + 4);
-    k_b4_padded<<<nblocks((long long)npad), TPB, 0, s>>>(*p, mx, my, q, clock);
+    launch_pdl(k_b4_padded, dim3(nblocks((long long)npad)), dim3(TPB), 0, s, *p, mx, my, q, clock);
     Geom g{mx, my, mx + 4, my + 4, dx, dy};
     Work W{};
     W.qB = q;
     W.bP = aux;
     W.td = aux + 3 * npad;
     W.npad = npad;
-    k_taudir<<<nblocks((long long)npad), TPB, 0, s>>>(*p, g, W, 1);
+    launch_pdl(k_taudir, dim3(nblocks((long long)npad)), dim3(TPB), 0, s, *p, g, W, 1);
     return cuda_status();
 }
 
@@ -1974,17 +2004,17 @@ int dclaw_step2(double* q, const double* aux, int mx, int my, int mbc, double dx
     W.bP = const_cast<double*>(aux);
     W.td = const_cast<double*>(aux) + 3 * L.npad;
     // the caller reads cflgrid from the clock: a clock set to this dt
-    k_clock_init<<<1, 32, 0, s>>>(clock, 0.0, dt, 0.0, 1);
+    launch_pdl(k_clock_init, dim3(1), dim3(32), 0, s, clock, 0.0, dt, 0.0, 1);
     const dclaw_params P = *p;
     // the tau planes lie where the x-fluxes go after the solves have read them
     double* tau = W.fx;
-    k_taus<<<stage_blocks((long long)L.npad), STAGE_TPB, 0, s>>>(P, W, tau);
-    k_riemann<0><<<stage_blocks((long long)L.nxi), STAGE_TPB, 0, s>>>(P, g, W, tau, dt, clock);
-    k_riemann<1><<<stage_blocks((long long)L.nyi), STAGE_TPB, 0, s>>>(P, g, W, tau, dt, clock);
-    k_flux<0><<<stage_blocks((long long)(mx + 1) * (my + 2)), STAGE_TPB, 0, s>>>(P, g, W, dt);
-    k_flux<1><<<stage_blocks((long long)(mx + 2) * (my + 1)), STAGE_TPB, 0, s>>>(P, g, W, dt);
-    k_update_padded<<<stage_blocks((long long)mx * my), STAGE_TPB, 0, s>>>(g, W, dt, q, fluxes, clock);
-    k_cfl_from_bits<<<1, 32, 0, s>>>(clock);
+    launch_pdl(k_taus, dim3(stage_blocks((long long)L.npad)), dim3(STAGE_TPB), 0, s, P, W, tau);
+    launch_pdl(k_riemann<0>, dim3(stage_blocks((long long)L.nxi)), dim3(STAGE_TPB), 0, s, P, g, W, tau, dt, clock);
+    launch_pdl(k_riemann<1>, dim3(stage_blocks((long long)L.nyi)), dim3(STAGE_TPB), 0, s, P, g, W, tau, dt, clock);
+    launch_pdl(k_flux<0>, dim3(stage_blocks((long long)(mx + 1) * (my + 2))), dim3(STAGE_TPB), 0, s, P, g, W, dt);
+    launch_pdl(k_flux<1>, dim3(stage_blocks((long long)(mx + 2) * (my + 1))), dim3(STAGE_TPB), 0, s, P, g, W, dt);
+    launch_pdl(k_update_padded, dim3(stage_blocks((long long)mx * my)), dim3(STAGE_TPB), 0, s, g, W, dt, q, fluxes, clock);
+    launch_pdl(k_cfl_from_bits, dim3(1), dim3(32), 0, s, clock);
     return cuda_status();
 }
 
@@ -1994,7 +2024,7 @@ int dclaw_src2(double* q, const double* aux, int mx, int my, int mbc, double dx,
     if (!q || !p || mbc != 2 || !sizes_ok(mx, my)) return DCLAW_ERR_ARG;
     int rc = dclaw_params_check_5(p);
     if (rc) return rc;
-    k_src2_padded<<<stage_blocks((long long)mx * my), STAGE_TPB, 0, (cudaStream_t)stream>>>(*p, mx, my, dt, q);
+    launch_pdl(k_src2_padded, dim3(stage_blocks((long long)mx * my)), dim3(STAGE_TPB), 0, (cudaStream_t)stream, *p, mx, my, dt, q);
     return cuda_status();
 }
 
@@ -2092,14 +2122,14 @@ int dclaw_step_full(const double* q_in, double* q_out, const double* b, const do
         cudaMemsetAsync(branch_log, 0, nlog * sizeof(uint32_t), s);
     }
     const long long npad = (long long)g.PX * g.PY;
-    k_full_b4<<<nblocks(npad), TPB, 0, s>>>(P, g, q_in, b, W, clock, tflag);
-    k_full_taudir<<<nblocks(npad), TPB, 0, s>>>(P, g, W);
-    k_full_riemann<0><<<stage_blocks((long long)(mx + 3) * (my + 2)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_riemann<1><<<stage_blocks((long long)(mx + 2) * (my + 3)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_flux<0><<<stage_blocks((long long)(mx + 1) * (my + 2)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_flux<1><<<stage_blocks((long long)(mx + 2) * (my + 1)), STAGE_TPB, 0, s>>>(P, g, W, clock, branch_log, tflag);
-    k_full_final<<<stage_blocks((long long)mx * my), STAGE_TPB, 0, s>>>(P, g, W, h_e, q_out, clock, tflag);
-    k_tick<<<1, 32, 0, s>>>(P, clock);
+    launch_pdl(k_full_b4, dim3(nblocks(npad)), dim3(TPB), 0, s, P, g, q_in, b, W, clock, tflag);
+    launch_pdl(k_full_taudir, dim3(nblocks(npad)), dim3(TPB), 0, s, P, g, W);
+    launch_pdl(k_full_riemann<0>, dim3(stage_blocks((long long)(mx + 3) * (my + 2))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
+    launch_pdl(k_full_riemann<1>, dim3(stage_blocks((long long)(mx + 2) * (my + 3))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
+    launch_pdl(k_full_flux<0>, dim3(stage_blocks((long long)(mx + 1) * (my + 2))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
+    launch_pdl(k_full_flux<1>, dim3(stage_blocks((long long)(mx + 2) * (my + 1))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
+    launch_pdl(k_full_final, dim3(stage_blocks((long long)mx * my)), dim3(STAGE_TPB), 0, s, P, g, W, h_e, q_out, clock, tflag);
+    launch_pdl(k_tick, dim3(1), dim3(32), 0, s, P, clock);
     return cuda_status();
 }
 
@@ -2252,9 +2282,9 @@ int dclaw_step_batched(const dclaw_batch* batch, const dclaw_member* members, co
     const int TX = batch_tx(batch->tile_shape), TY = batch_ty(batch->tile_shape);
     unsigned g0 = (unsigned)(nsm * cpsm);
     if (g0 > batch->nschunks) g0 = batch->nschunks;
-    k_scan_batch<<<g0, TPB, 0, s>>>(batch->nmembers, batch->nschunks, members, params, clocks, q_in, q_out, counters,
+    launch_pdl(k_scan_batch, dim3(g0), dim3(TPB), 0, s, batch->nmembers, batch->nschunks, members, params, clocks, q_in, q_out, counters,
                                     tflag, TX, TY);
-    k_list_batch<<<(unsigned)((batch->ntiles + TPB - 1) / TPB), TPB, 0, s>>>(batch->nmembers, batch->ntiles, members,
+    launch_pdl(k_list_batch, dim3((unsigned)((batch->ntiles + TPB - 1) / TPB)), dim3(TPB), 0, s, batch->nmembers, batch->ntiles, members,
                                                                             clocks, tflag, counters, list_act, list_rec);
     int rc = DCLAW_OK;
     switch (batch->tile_shape) {
@@ -2263,7 +2293,7 @@ int dclaw_step_batched(const dclaw_batch* batch, const dclaw_member* members, co
         default: rc = launch_batch_tiles<batch_tx(2), batch_ty(2)>(batch, members, params, clocks, q_in, q_out, b, w, counters, tflag, list_act, list_rec, nsm, cpsm, s); break;
     }
     if (rc != DCLAW_OK) return rc;
-    k_tick_batch<<<(unsigned)((batch->nmembers + TPB - 1) / TPB), TPB, 0, s>>>(batch->nmembers, params, clocks);
+    launch_pdl(k_tick_batch, dim3((unsigned)((batch->nmembers + TPB - 1) / TPB)), dim3(TPB), 0, s, batch->nmembers, params, clocks);
     return cuda_status();
 }
 
