@@ -593,19 +593,17 @@ class EnsembleStepAdjoint:
             _lib.check(int(st), f"ensemble adjoint, member {k}")
 
 
-def _ensemble(members, theta, fixed_dt: bool, bed: torch.Tensor | None = None):
+def _ensemble(members, theta, fixed_dt: bool, q: torch.Tensor, bed: torch.Tensor | None = None):
+    """A stepper over the members at theta, its state and (when given) its
+    bed from device arenas."""
     from .ensemble import EnsembleStepper, Member
 
     th = theta.detach().cpu().tolist()
     mem = [Member(m.q, m.b, with_theta(m.params, th[k]), m.dx, m.dy, m.dt_initial, m.t_final,
                   getattr(m, "t_obs", 0.0))
            for k, m in enumerate(members)]
-    st = EnsembleStepper(mem, theta.device, fixed_dt=fixed_dt)
-    if bed is not None:
-        if bed.shape != st.bed.shape:
-            raise ValueError(f"bed must be the ensemble's bed arena, shape {tuple(st.bed.shape)}")
-        st.bed.copy_(bed.detach())
-    return st
+    return EnsembleStepper(mem, theta.device, fixed_dt=fixed_dt, q=q.detach(),
+                           bed=None if bed is None else bed.detach())
 
 
 def _clock_field(st, k: int) -> torch.Tensor:
@@ -618,8 +616,7 @@ class _EnsembleRollout(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q0, theta, members, n_steps, out_steps, checkpoint_block, fixed_dt, dt_schedule, select,
                 n_obs, bed):
-        st = _ensemble(members, theta, fixed_dt or dt_schedule is not None, bed)
-        st.qa.copy_(q0.detach())
+        st = _ensemble(members, theta, fixed_dt or dt_schedule is not None, q0, bed)
         lib = _lib.load()
         reserve = 2 * sum(lib.dclaw_adjoint_workspace_bytes(m.q.shape[2], m.q.shape[1]) for m in members)
         k = _block(n_steps, checkpoint_block, st.qa.numel() * 8, reserve, q0.device)
@@ -671,10 +668,12 @@ class _EnsembleRollout(torch.autograd.Function):
                                                 _lib.ptr(obs_step), _lib.stream_ptr()), "observation record")
         for kk, s in enumerate(st.status()):
             _lib.check(s, f"ensemble rollout, member {kk}")
-        # the bed goes through save_for_backward (None when absent) so that an
-        # in-place change between forward and backward raises autograd's
-        # version error instead of silently changing the recompute
-        ctx.save_for_backward(dts, store, bed)
+        # the bed goes through save_for_backward so that an in-place change
+        # between forward and backward raises autograd's version error
+        # instead of silently changing the recompute; without one, the arena
+        # of the members' beds the forward pass uploaded
+        ctx.own_bed = bed is None
+        ctx.save_for_backward(dts, store, st.bed if bed is None else bed)
         ctx.select = select
         ctx.meta = (members, theta.detach(), int(n_steps), tuple(out_steps), k)
         ctx.obs_steps = None
@@ -694,17 +693,17 @@ class _EnsembleRollout(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_out):
         dts, store, bed = ctx.saved_tensors
-        bed = None if bed is None else bed.detach()
+        bed = bed.detach()
         ckpt = list(store.unbind(0))
         members, theta, n_steps, out_steps, k = ctx.meta
         dev = dts.device
         where = {}
         for idx, n in enumerate(out_steps):
             where.setdefault(n, []).append(idx)
-        fw = _ensemble(members, theta, True, bed)
+        fw = _ensemble(members, theta, True, ckpt[0], bed)
         adjs = [EnsembleStepAdjoint(fw), EnsembleStepAdjoint(fw)]
         # the bed arena's gradient, when the run was given one that requires grad
-        bbar = torch.zeros_like(fw.bed) if bed is not None and ctx.needs_input_grad[10] else None
+        bbar = torch.zeros_like(fw.bed) if not ctx.own_bed and ctx.needs_input_grad[10] else None
         lam = torch.zeros_like(fw.qa)
         lam2 = torch.zeros_like(lam)   # arena gaps between members stay zero
         pbar = torch.zeros((fw.n, 4), dtype=torch.float64, device=dev)

@@ -56,9 +56,17 @@ def clock_array(dts, t_finals, fixed_dt: bool = False, t_obs=None) -> np.ndarray
 
 
 class EnsembleStepper:
-    """All members on one device, advanced together."""
+    """All members on one device, advanced together.
 
-    def __init__(self, members: list[Member], device="cuda", tile_shape: int = 0, fixed_dt: bool = False):
+    q, bed (device arenas in this layout, optional): copied instead of the
+    members' arrays, whose q and b then only set the layout. A gradient
+    builds its steppers from arenas already on the device: uploading eight
+    members of 1024 x 190 cells again, in the forward and in the backward
+    pass, took 12 of its 28 ms.
+    """
+
+    def __init__(self, members: list[Member], device="cuda", tile_shape: int = 0, fixed_dt: bool = False, *,
+                 q: torch.Tensor | None = None, bed: torch.Tensor | None = None):
         self.lib = _lib.load()
         self.members = members
         self.n = len(members)
@@ -76,11 +84,19 @@ class EnsembleStepper:
         self.qa = torch.zeros(self.batch.q_doubles, dtype=torch.float64, device=self.device)
         self.qb = torch.zeros_like(self.qa)
         self.bed = torch.zeros(self.batch.b_doubles, dtype=torch.float64, device=self.device)
+        if bed is not None and bed.shape != self.bed.shape:
+            raise ValueError(f"bed must be the ensemble's bed arena, shape {tuple(self.bed.shape)}")
         for k, m in enumerate(members):
             o, c = self.cm[k].q_off, int(self.mx[k]) * int(self.my[k])
-            self.qa[o:o + 5 * c].copy_(torch.from_numpy(np.ascontiguousarray(m.q, dtype=np.float64).ravel()))
+            if q is None:
+                self.qa[o:o + 5 * c].copy_(torch.from_numpy(np.ascontiguousarray(m.q, dtype=np.float64).ravel()))
             ob = self.cm[k].b_off
-            self.bed[ob:ob + c].copy_(torch.from_numpy(np.ascontiguousarray(m.b, dtype=np.float64).ravel()))
+            if bed is None:
+                self.bed[ob:ob + c].copy_(torch.from_numpy(np.ascontiguousarray(m.b, dtype=np.float64).ravel()))
+        if q is not None:
+            self.qa.copy_(q)
+        if bed is not None:
+            self.bed.copy_(bed)
         params = (CParams * self.n)(*[m.params.to_c() for m in members])
         self.params = torch.frombuffer(bytearray(bytes(params)), dtype=torch.uint8).to(self.device)
         self.clocks = torch.tensor(clock_array([m.dt_initial for m in members], [m.t_final for m in members],
