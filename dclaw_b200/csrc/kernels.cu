@@ -566,7 +566,7 @@ template <int TX, int TY, bool WITH_SRC2, int NT>
 __device__ __forceinline__ double tile_body(const dclaw_params& P, const Geom& g, const Rec& R,
                                             const double* __restrict__ b, double* __restrict__ q_out, double dt,
                                             int i0, int j0, double* smem, uint32_t* __restrict__ brlog, bool& nan,
-                                            bool active = true) {
+                                            double crit, bool active = true) {
     using TG = TileGeom<TX, TY>;
     TileMem M;
     M.A = smem;
@@ -636,7 +636,7 @@ __device__ __forceinline__ double tile_body(const dclaw_params& P, const Geom& g
                 bool need = it < nsolve && tile_needs_solve(P, g, M, dir, it, i0, j0, TX);
                 if (it < nsolve && !need) {
                     bool ok;
-                    tile_riemann(P, g, R, M, dir, it, i0, j0, TX, TY, ok);
+                    tile_riemann(P, g, R, M, dir, it, i0, j0, TX, TY, ok, crit);
                 }
                 const unsigned bal = __ballot_sync(0xffffffffu, need);
                 int base = 0;
@@ -654,7 +654,7 @@ __device__ __forceinline__ double tile_body(const dclaw_params& P, const Geom& g
             const int nneed = *M.nlist;
             for (int w = tid; w < nneed; w += NT) {
                 bool ok;
-                double s = tile_riemann(P, g, R, M, dir, M.list[w], i0, j0, TX, TY, ok);
+                double s = tile_riemann(P, g, R, M, dir, M.list[w], i0, j0, TX, TY, ok, crit);
                 if (ok) cfl = fmax2(cfl, dtd * s);
             }
             __syncthreads();
@@ -709,7 +709,7 @@ __device__ __forceinline__ double tile_body(const dclaw_params& P, const Geom& g
             }
         }
         for (int it = tid; it < TX * TY; it += NT)
-            if (tile_final<TX, TY, WITH_SRC2>(P, g, R, M, it, i0, j0, dt, q_out)) nan = true;
+            if (tile_final<TX, TY, WITH_SRC2>(P, g, R, M, it, i0, j0, dt, dtdx, dtdy, q_out)) nan = true;
     }
     if (!(cfl == cfl)) cfl = 0.0;
     return cfl;
@@ -726,7 +726,8 @@ __global__ void __launch_bounds__(TILE_TPB, DCLAW_TILE_MINBLOCKS) k_tile(dclaw_p
     const int i0 = 1 + blockIdx.x * TX, j0 = 1 + ty * TY;
     const bool active = !tflag || brlog || tflag[ty * gridDim.x + blockIdx.x] == clk->nsteps + 1u;
     bool nan;
-    double cfl = tile_body<TX, TY, WITH_SRC2, TILE_TPB>(P, g, R, b, q_out, clk->dt, i0, j0, smem, brlog, nan, active);
+    double cfl = tile_body<TX, TY, WITH_SRC2, TILE_TPB>(P, g, R, b, q_out, clk->dt, i0, j0, smem, brlog, nan,
+                                                         critical_root(P), active);
     if (nan) flag_status(clk, DCLAW_ERR_NAN);
     block_max_to(cfl, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
     if (WITH_SRC2) last_block_tick(P, clk);
@@ -854,7 +855,7 @@ __global__ void __launch_bounds__(TILE_TPB, DCLAW_TILE_MINBLOCKS) k_tile_list(dc
     __shared__ uint32_t s_t[2];
     const unsigned int nact = counters[1];
     const uint32_t ntx = (uint32_t)((g.mx + TILE_X - 1) / TILE_X);
-    const double dt = clk->dt;
+    const double dt = clk->dt, crit = critical_root(P);
     double cfl = 0.0;
     bool nan_any = false;
     if (threadIdx.x == 0) {
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(TILE_TPB, DCLAW_TILE_MINBLOCKS) k_tile_list(dc
         const int i0 = 1 + (int)(t % ntx) * TILE_X, j0 = 1 + (int)(t / ntx) * TILE_Y;
         bool nan;
         const double c =
-            tile_body<TILE_X, TILE_Y, WITH_SRC2, TILE_TPB>(P, g, R, b, q_out, dt, i0, j0, smem, nullptr, nan);
+            tile_body<TILE_X, TILE_Y, WITH_SRC2, TILE_TPB>(P, g, R, b, q_out, dt, i0, j0, smem, nullptr, nan, crit);
         cfl = fmax2(cfl, c);
         nan_any = nan_any || nan;
         // the next tile's staging overwrites shared memory
@@ -1174,7 +1175,7 @@ __global__ void __launch_bounds__(TPB, 2) k_tile_batch(int nmem, uint32_t ntiles
         // otherwise its pre-src2 state (k_src2_batch follows)
         double* dst = DCLAW_BATCH_SRC2_KERNEL ? work + sM.qs_off : q_out + sM.q_off;
         double cfl = tile_body<TX, TY, !DCLAW_BATCH_SRC2_KERNEL, TPB>(sP, g, R, b + sM.b_off, dst, clocks[m].dt, i0, j0,
-                                                                     smem, nullptr, nan);
+                                                                     smem, nullptr, nan, critical_root(sP));
         if (nan) flag_status(clocks + m, DCLAW_ERR_NAN);
         // block max of this tile's Courant number into member m's clock
         cfl = warp_max(cfl);

@@ -159,27 +159,33 @@ struct RType {
     bool rare1, rare2;
 };
 
-// riemanntype with maxiter = 1
-DC_HD RType riemanntype(double hL, double hR, double uL, double uR, double drytol, double g) {
+// riemanntype with maxiter = 1. cL = sqrt(g hL), cR = sqrt(g hR), rL =
+// sqrt(hL), rR = sqrt(hR): the solver has them, and a root (or a division)
+// is 130 cycles of a chain nothing overlaps, so none is taken twice.
+DC_HD RType riemanntype(double hL, double hR, double uL, double uR, double cL, double cR, double rL, double rR,
+                        double drytol, double g) {
     RType o;
-    double h_min = fmin2(hR, hL);
-    double h_max = fmax2(hR, hL);
+    // the deeper and the shallower side
+    const bool Rmin = hR < hL, Rmax = hR > hL;
+    double h_min = Rmin ? hR : hL;
+    double h_max = Rmax ? hR : hL;
     double delu = uR - uL;
     if (h_min <= drytol) {
         o.hm = 0.0;
-        o.s1m = uR + uL - 2.0 * sqrt(g * hR) + 2.0 * sqrt(g * hL);
+        o.s1m = uR + uL - 2.0 * cR + 2.0 * cL;
         o.s2m = o.s1m;
         if (hL <= 0.0) { o.rare2 = true; o.rare1 = false; }
         else { o.rare1 = true; o.rare2 = false; }
     } else {
-        double F_min = delu + 2.0 * (sqrt(g * h_min) - sqrt(g * h_max));
+        const double c_min = Rmin ? cR : cL, c_max = Rmax ? cR : cL;
+        double F_min = delu + 2.0 * (c_min - c_max);
         double F_max = delu + (h_max - h_min) * (sqrt(.5 * g * (h_max + h_min) / (h_max * h_min)));
         if (F_min > 0.0) {
-            double hm = (1.0 / (16.0 * g)) * sq(fmax2(0.0, -delu + 2.0 * (sqrt(g * hL) + sqrt(g * hR))));
+            double hm = (1.0 / (16.0 * g)) * sq(fmax2(0.0, -delu + 2.0 * (cL + cR)));
             o.hm = hm;
             double sghm = sqrt(g * hm);
-            o.s1m = uL + 2.0 * sqrt(g * hL) - 3.0 * sghm;
-            o.s2m = uR - 2.0 * sqrt(g * hR) + 3.0 * sghm;
+            o.s1m = uL + 2.0 * cL - 3.0 * sghm;
+            o.s2m = uR - 2.0 * cR + 3.0 * sghm;
             o.rare1 = true;
             o.rare2 = true;
         } else if (F_max <= 0.0) {
@@ -188,8 +194,9 @@ DC_HD RType riemanntype(double hL, double hR, double uL, double uR, double dryto
             double gR = sqrt(.5 * g * (1.0 / h0 + 1.0 / hR));
             double F0 = delu + (h0 - hL) * gL + (h0 - hR) * gR;
             double dfdh = gL - g * (h0 - hL) / (4.0 * (sq(h0)) * gL) + gR - g * (h0 - hR) / (4.0 * (sq(h0)) * gR);
-            double slope = 2.0 * sqrt(h0) * dfdh;
-            h0 = sq(sqrt(h0) - F0 / slope);
+            const double r0 = Rmax ? rR : rL;
+            double slope = 2.0 * r0 * dfdh;
+            h0 = sq(r0 - F0 / slope);
             double hm = h0;
             o.hm = hm;
             double u1m = uL - (hm - hL) * sqrt((.5 * g) * (1.0 / hm + 1.0 / hL));
@@ -201,21 +208,22 @@ DC_HD RType riemanntype(double hL, double hR, double uL, double uR, double dryto
             o.rare2 = false;
         } else {
             double h0 = h_min;
-            double F0 = delu + 2.0 * (sqrt(g * h0) - sqrt(g * h_max))
-                        + (h0 - h_min) * sqrt(.5 * g * (1.0 / h0 + 1.0 / h_min));
+            // the reference's last term, (h0 - h_min) sqrt(.5 g (1/h0 +
+            // 1/h_min)), is 0 times a finite root at h0 = h_min
+            double F0 = delu + 2.0 * (c_min - c_max) + 0.0;
             double slope = (F_max - F0) / (h_max - h_min);
             h0 = h0 - F0 / slope;
             double hm = h0;
             o.hm = hm;
             double sghm = sqrt(g * hm);
             if (hL > hR) {
-                double a = uL + 2.0 * sqrt(g * hL);
+                double a = uL + 2.0 * cL;
                 o.s1m = a - 3.0 * sghm;
                 o.s2m = a - sghm;
                 o.rare1 = true;
                 o.rare2 = false;
             } else {
-                double a = uR - 2.0 * sqrt(g * hR);
+                double a = uR - 2.0 * cR;
                 o.s2m = a + 3.0 * sghm;
                 o.s1m = a + sghm;
                 o.rare2 = true;
@@ -224,6 +232,10 @@ DC_HD RType riemanntype(double hL, double hR, double uL, double uR, double dryto
         }
     }
     return o;
+}
+
+DC_HD RType riemanntype(double hL, double hR, double uL, double uR, double drytol, double g) {
+    return riemanntype(hL, hR, uL, uR, sqrt(g * hL), sqrt(g * hR), sqrt(hL), sqrt(hR), drytol, g);
 }
 
 // Result of one interface solve in compact form. In the reference's five
@@ -268,7 +280,11 @@ struct ChiWaves {
 // on the velocity only through u^2 + v^2. With cw, the species waves are
 // computed too from L.chi, R.chi (riemannsolvers_dclaw.f:463-468, merged at
 // :495-510; the dry side takes the wet side's chi, rpn2_dclaw.f:197,226).
-DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, ChiWaves* cw = nullptr) {
+// criticaltol_2: critical_root(P), which a kernel takes once.
+DC_HD double critical_tol(const dclaw_params& P) { return fmax2(P.dry_tolerance * P.grav, 1e-6); }
+DC_HD double critical_root(const dclaw_params& P) { return sqrt(critical_tol(P)); }
+DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, ChiWaves* cw,
+                           const double criticaltol_2) {
     const double grav = P.grav;
     const double drytol = P.dry_tolerance;
     double wall1 = 1.0, wall2 = 1.0, wall3 = 1.0;
@@ -282,12 +298,16 @@ DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, 
         chiL = L.chi;
         chiR = R.chi;
     }
+    // sqrt(g h) and sqrt(h) of the two sides (0 on a dry one)
+    double cL = 0.0, cR = 0.0, sqhL = 0.0, sqhR = 0.0;
     if (hR <= drytol) {
         hR = 0.0;
         pR = 0.0;
         mR = mL;
         chiR = chiL;
-        RType t = riemanntype(hL, hL, uL, -uL, drytol, grav);
+        cL = sqrt(grav * hL);
+        sqhL = sqrt(hL);
+        RType t = riemanntype(hL, hL, uL, -uL, cL, cL, sqhL, sqhL, drytol, grav);
         double hstartest = fmax2(hL, t.hm);
         if (hstartest + bL < bR) {
             wall2 = 0.0; wall3 = 0.0;
@@ -295,13 +315,16 @@ DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, 
             hR = hL; huR = -huL; hvR = hvL; hmR = hmL; bR = bL;
             uR = -uL; vR = vL; mR = mL; pR = pL;
             rhoR_sv = rhoL_sv; tauR_sv = tauL_sv;
+            cR = cL; sqhR = sqhL;
         }
     } else if (hL <= drytol) {
         hL = 0.0;
         pL = 0.0;
         mL = mR;
         chiL = chiR;
-        RType t = riemanntype(hR, hR, -uR, uR, drytol, grav);
+        cR = sqrt(grav * hR);
+        sqhR = sqrt(hR);
+        RType t = riemanntype(hR, hR, -uR, uR, cR, cR, sqhR, sqhR, drytol, grav);
         double hstartest = fmax2(hR, t.hm);
         if (hstartest + bR < bL) {
             wall1 = 0.0; wall2 = 0.0;
@@ -309,13 +332,18 @@ DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, 
             hL = hR; huL = -huR; hvL = hvR; hmL = hmR; mL = mR; bL = bR;
             uL = -uR; vL = vR; pL = pR;
             rhoL_sv = rhoR_sv; tauL_sv = tauR_sv;
+            cL = cR; sqhL = sqhR;
         }
+    } else {
+        cL = sqrt(grav * hL);
+        cR = sqrt(grav * hR);
+        sqhL = sqrt(hL);
+        sqhR = sqrt(hR);
     }
     if (wallprob && br) *br |= BR_WALL;
 
     // ---- riemann_dig2_aug_sswave_ez ----
-    const double criticaltol = fmax2(drytol * grav, 1e-6);
-    const double criticaltol_2 = sqrt(criticaltol);
+    const double criticaltol = critical_tol(P);
     const double gz = grav;  // cos(0) = 1
     double rhoL, rhoR, tauL, tauR;
     if (hL >= drytol && hR >= drytol) {
@@ -346,8 +374,6 @@ DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, 
     // kappa = 1: eps = 1 + 0*gamma = 1, geps = gz
     const double geps = gz;
 
-    double sqhL = sqrt(hL), sqhR = sqrt(hR);
-    double cL = sqrt(geps * hL), cR = sqrt(geps * hR);
     double sL = uL - cL;
     double sR = uR + cR;
     double uhat = (sqhL * uL + sqhR * uR) / (sqhR + sqhL);
@@ -359,7 +385,7 @@ DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, 
     double sw1 = sE1, sw3 = sE2;
     double u = uhat;
 
-    RType rt = riemanntype(hL, hR, uL, uR, drytol, geps);
+    RType rt = riemanntype(hL, hR, uL, uR, cL, cR, sqhL, sqhR, drytol, geps);
     sw1 = fmin2(sw1, rt.s2m);
     sw3 = fmax2(sw3, rt.s1m);
     double sw2 = 0.5 * (sw3 + sw1);
@@ -429,10 +455,11 @@ DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, 
     double grg = gamma * rho * gz;
     double del4 = -gamma * rho * gz * u * (hR - hL) + grg * del1 + u * (pR - pL);
 
-    double vnorm = sqrt(sq(uR) + sq(uL) + sq(vR) + sq(vL));
+    // the reference tests the root of this sum, positive with it
+    double vnorm2 = sq(uR) + sq(uL) + sq(vR) + sq(vL);
     bool is_static = false;
     double tausource;
-    if (vnorm > 0.0) {
+    if (vnorm2 > 0.0) {
         tausource = 0.0;
     } else {
         double tdR = R.taudir;
@@ -521,6 +548,10 @@ DC_BIG Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, 
     return w;
 }
 
+DC_HD Waves riemann_solve(const dclaw_params& P, Side L, Side R, uint32_t* br, ChiWaves* cw = nullptr) {
+    return riemann_solve(P, L, R, br, cw, critical_root(P));
+}
+
 // ---------------------------------------------------------------------------
 // rpt2 for one fluctuation. cell = the imp cell (A2 state: h, hn, ht, hm),
 // b = its bed, topo1/topo3 = bed of the neighbours below/above in the
@@ -538,15 +569,15 @@ struct Rpt2Cell {
     double u, m, chi, eta, r5, s1, s2, s3, s31;
 };
 
-DC_HD Rpt2Cell rpt2_cell(const dclaw_params& P, double h, double hn, double ht, double hm, double b, double topo1,
+// u, v: the quotients hn / h and ht / h of a wet cell
+DC_HD Rpt2Cell rpt2_cell(const dclaw_params& P, double h, double u, double v, double hm, double b, double topo1,
                          double topo3, double hchi = 0.0, bool with_chi = false) {
     Rpt2Cell c;
     c.ok = false;
     c.u = c.m = c.chi = c.eta = c.r5 = c.s1 = c.s2 = c.s3 = c.s31 = 0.0;
     if (h <= P.dry_tolerance) return c;
     const double g = P.grav;
-    c.u = hn / h;
-    double v = ht / h;
+    c.u = u;
     c.m = hm / h;
     if (with_chi) c.chi = hchi / h;
     c.eta = h + b;
@@ -616,7 +647,12 @@ DC_BIG bool rpt2_split(const dclaw_params& P, double h, double hn, double ht, do
                                           double b, double topo1, double topo3, const double asdq[5],
                                           double bm[5], double bp[5], double hchi = 0.0,
                                           double* bmp6 = nullptr) {
-    const Rpt2Cell c = rpt2_cell(P, h, hn, ht, hm, b, topo1, topo3, hchi, bmp6 != nullptr);
+    double u = 0.0, v = 0.0;
+    if (!(h <= P.dry_tolerance)) {
+        u = hn / h;
+        v = ht / h;
+    }
+    const Rpt2Cell c = rpt2_cell(P, h, u, v, hm, b, topo1, topo3, hchi, bmp6 != nullptr);
     return rpt2_apply(c, topo1, topo3, asdq, bm, bp, bmp6);
 }
 

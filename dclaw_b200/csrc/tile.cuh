@@ -86,16 +86,24 @@ DC_HD bool cell_record(const dclaw_params& P, const Geom& g, const double* __res
     double hu = q_in[plane + c], hv = q_in[2 * plane + c], hm = q_in[3 * plane + c], p = q_in[4 * plane + c];
     bool nan = (h != h) || (hu != hu) || (hv != hv) || (hm != hm) || (p != p);
     bool wet = h > P.dry_tolerance;
+    double uq = 0.0, vq = 0.0;
     if (wet) {
         if (flip_u) hu = -hu;
         if (flip_v) hv = -hv;
-        double u, v, m;
-        qfix(P, h, hu, hv, hm, p, u, v, m, P.grav);   // b4step2
-        double s = sqrt((sq(hu) + sq(hv))) / h;      // speed limit (h > 0)
-        if (s > P.speed_limit) {
-            double sratio = P.speed_limit / s;
-            hu = hu * sratio;
-            hv = hv * sratio;
+        double m;
+        qfix(P, h, hu, hv, hm, p, uq, vq, m, P.grav);   // b4step2
+        // speed limit (h > 0): the speed's root and quotient are taken only
+        // where the speed may reach half the limit
+        const double q2 = sq(hu) + sq(hv), far = 0.5 * P.speed_limit * h;
+        if (!(P.speed_limit > 0.0 && q2 < far * far)) {
+            double s = sqrt(q2) / h;
+            if (s > P.speed_limit) {
+                double sratio = P.speed_limit / s;
+                hu = hu * sratio;
+                hv = hv * sratio;
+                uq = hu / h;
+                vq = hv / h;
+            }
         }
     } else {
         h = 0.0;
@@ -106,7 +114,6 @@ DC_HD bool cell_record(const dclaw_params& P, const Geom& g, const double* __res
     double fs = 0.0, tdx = 0.0, tdy = 0.0;
     double tau1 = 0.0, rho1 = 0.0;
     if (wet) {
-        const double uq = hu / h, vq = hv / h;
         double m1 = fmin2(fmax2(hm / h, 0.0), 1.0);
         double hm1 = h * m1;
         double p1 = clip_p(P, h, m1, p);
@@ -315,9 +322,9 @@ DC_HD bool tile_needs_solve(const dclaw_params& P, const Geom& g, const TileMem&
 // Riemann solve of sweep `dir` for tile-local item (slice s, interface k).
 // dir 0: s = row r, k = x-interface; dir 1: s = column c, k = y-interface.
 // Returns max |s| (0 for skipped items); cfl_ok tells whether the item
-// counts for the Courant number.
+// counts for the Courant number. crit: critical_root(P).
 DC_HD double tile_riemann(const dclaw_params& P, const Geom& g, const Rec& R, const TileMem& M, int dir,
-                          int item, int i0, int j0, int TX, int TY, bool& cfl_ok) {
+                          int item, int i0, int j0, int TX, int TY, bool& cfl_ok, double crit) {
     int sl, k;
     if (dir == 0) { sl = j0 - 1 + item / (TX + 3); k = i0 - 1 + item % (TX + 3); }
     else { sl = i0 - 1 + item % (TX + 2); k = j0 - 1 + item / (TX + 2); }
@@ -337,7 +344,7 @@ DC_HD double tile_riemann(const dclaw_params& P, const Geom& g, const Rec& R, co
         } else {
             Side Rs = rec_side(P, R, g, M, iR, jR, dir, false);
             Side Ls = rec_side(P, R, g, M, iL, jL, dir, k - 1 >= 0);
-            w = riemann_solve(P, Ls, Rs, &bits);
+            w = riemann_solve(P, Ls, Rs, &bits, nullptr, crit);
         }
         cfl_ok = k >= 1 && k <= nlen + 1;
     }
@@ -349,15 +356,21 @@ DC_HD double tile_riemann(const dclaw_params& P, const Geom& g, const Rec& R, co
     return fmax2(fmax2(fabs(w.s1), fabs(w.s2)), fabs(w.s5));
 }
 
-// A2 state (h, hn, ht, hm) of a record cell
+DC_HD double tile_riemann(const dclaw_params& P, const Geom& g, const Rec& R, const TileMem& M, int dir,
+                          int item, int i0, int j0, int TX, int TY, bool& cfl_ok) {
+    return tile_riemann(P, g, R, M, dir, item, i0, j0, TX, TY, cfl_ok, critical_root(P));
+}
+
+// A2 state of a record cell: h, the normal and tangential velocities (the
+// record's quotients, so rpt2 divides no momentum by h again) and hm
 DC_HD void rec_a2(const dclaw_params& P, const Rec& R, const Geom& g, const TileMem& M, int i, int j, int dir,
-                  double& h, double& hn, double& ht, double& hm) {
+                  double& h, double& un, double& ut, double& hm) {
     const size_t pi = pidx(g, i, j);
     h = M.h(i, j);
-    if (h <= P.dry_tolerance) { h = 0.0; hn = 0.0; ht = 0.0; hm = 0.0; return; }
-    double hu = R.get(R_HU, pi), hv = R.get(R_HV, pi);
-    hn = dir == 0 ? hu : hv;
-    ht = dir == 0 ? hv : hu;
+    if (h <= P.dry_tolerance) { h = 0.0; un = 0.0; ut = 0.0; hm = 0.0; return; }
+    double u = R.get(R_UQ, pi), v = R.get(R_VQ, pi);
+    un = dir == 0 ? u : v;
+    ut = dir == 0 ? v : u;
     hm = h * R.get(R_M2, pi);
 }
 
@@ -409,13 +422,13 @@ DC_HD bool iface_limited(const dclaw_params& P, const TileMem& M, int dir, int i
 DC_HD bool split_cell(const dclaw_params& P, const Rec& R, const Geom& g, const TileMem& M, int dir, int ci,
                       int cj, const double src[5], double half, double Um[5], double Up[5]) {
     const bool y = dir != 0;
-    double h, hn, ht, hm;
-    rec_a2(P, R, g, M, ci, cj, dir, h, hn, ht, hm);
+    double h, un, ut, hm;
+    rec_a2(P, R, g, M, ci, cj, dir, h, un, ut, hm);
     double topo1, topo3;
     if (!y) { topo1 = M.bed(ci, cj - 1); topo3 = M.bed(ci, cj + 1); }
     else { topo1 = M.bed(ci - 1, cj); topo3 = M.bed(ci + 1, cj); }
     double asdq[5] = {src[0], y ? src[2] : src[1], y ? src[1] : src[2], src[3], src[4]}, bm[5], bp[5];
-    bool done = rpt2_split(P, h, hn, ht, hm, M.bed(ci, cj), topo1, topo3, asdq, bm, bp);
+    bool done = rpt2_apply(rpt2_cell(P, h, un, ut, hm, M.bed(ci, cj), topo1, topo3), topo1, topo3, asdq, bm, bp);
     double bmq[5] = {bm[0], y ? bm[2] : bm[1], y ? bm[1] : bm[2], bm[3], bm[4]};
     double bpq[5] = {bp[0], y ? bp[2] : bp[1], y ? bp[1] : bp[2], bp[3], bp[4]};
     for (int m = 0; m < 5; ++m) {
@@ -432,12 +445,12 @@ DC_HD void split_cell2(const dclaw_params& P, const Rec& R, const Geom& g, const
                        int cj, const double src1[5], const double src2[5], double half, double U1m[5],
                        double U1p[5], double U2m[5], double U2p[5], bool& d1, bool& d2) {
     const bool y = dir != 0;
-    double h, hn, ht, hm;
-    rec_a2(P, R, g, M, ci, cj, dir, h, hn, ht, hm);
+    double h, un, ut, hm;
+    rec_a2(P, R, g, M, ci, cj, dir, h, un, ut, hm);
     double topo1, topo3;
     if (!y) { topo1 = M.bed(ci, cj - 1); topo3 = M.bed(ci, cj + 1); }
     else { topo1 = M.bed(ci - 1, cj); topo3 = M.bed(ci + 1, cj); }
-    const Rpt2Cell cell = rpt2_cell(P, h, hn, ht, hm, M.bed(ci, cj), topo1, topo3);
+    const Rpt2Cell cell = rpt2_cell(P, h, un, ut, hm, M.bed(ci, cj), topo1, topo3);
     auto one = [&](const double* src, double* Um, double* Up) -> bool {
         double asdq[5] = {src[0], y ? src[2] : src[1], y ? src[1] : src[2], src[3], src[4]}, bm[5], bp[5];
         bool done = rpt2_apply(cell, topo1, topo3, asdq, bm, bp);
@@ -652,10 +665,9 @@ DC_HD void tile_T_store(const TileMem& M, int item, const double T[5]) {
 // otherwise q_out holds the updated state before src2. Returns true on NaN.
 template <int TX, int TY, bool WITH_SRC2>
 DC_HD bool tile_final(const dclaw_params& P, const Geom& g, const Rec& R, const TileMem& M, int item, int i0,
-                      int j0, double dt, double* __restrict__ q_out) {
+                      int j0, double dt, double dtdx, double dtdy, double* __restrict__ q_out) {
     int i = i0 + item % TX, j = j0 + item / TX;
     if (i > g.mx || j > g.my) return false;
-    const double dtdx = dt / g.dx, dtdy = dt / g.dy;
     const size_t pc = pidx(g, i, j);
     double qb[5];
     qb[0] = M.h(i, j);
@@ -685,6 +697,12 @@ DC_HD bool tile_final(const dclaw_params& P, const Geom& g, const Rec& R, const 
     const size_t c = (size_t)(j - 1) * g.mx + (size_t)(i - 1);
     for (int m = 0; m < 5; ++m) q_out[(size_t)m * plane + c] = qn[m];
     return nan;
+}
+
+template <int TX, int TY, bool WITH_SRC2>
+DC_HD bool tile_final(const dclaw_params& P, const Geom& g, const Rec& R, const TileMem& M, int item, int i0,
+                      int j0, double dt, double* __restrict__ q_out) {
+    return tile_final<TX, TY, WITH_SRC2>(P, g, R, M, item, i0, j0, dt, dt / g.dx, dt / g.dy, q_out);
 }
 
 // src2 of interior cell c (0-based linear index) from the updated state
