@@ -493,9 +493,11 @@ __global__ void k_clock_set_obs(dclaw_clock* clk, double t_obs) {
 // Records of every padded cell, and the marks. prow0 / nprow: the padded
 // rows (0 .. my+3 for j = -1 .. my+2) this launch covers, all of them by
 // default.
-__global__ void __launch_bounds__(TPB, DCLAW_PLAIN_CELL_MINB) k_records(dclaw_params P, Geom g, const double* __restrict__ q_in,
+template <int MINB>
+__global__ void __launch_bounds__(TPB, MINB) k_records(dclaw_params P, Geom g, const double* __restrict__ q_in,
                                                  const double* __restrict__ b, Rec R, dclaw_clock* clk,
                                                  uint32_t* __restrict__ tflag, int prow0 = 0, int nprow = -1) {
+    pdl_wait();
     const long long n = (long long)g.PX * (nprow < 0 ? g.PY : nprow);
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
@@ -715,12 +717,140 @@ __device__ __forceinline__ double tile_body(const dclaw_params& P, const Geom& g
     return cfl;
 }
 
+// One tile with its two sweeps side by side: threads 0..255 take the x-sweep,
+// 256..511 the y-sweep, which read the same state and meet only in the
+// update. One CTA per SM (139 KB, 512 threads at 128 registers), so a tile
+// takes one solve and one flux phase instead of two of each, and half as
+// many tiles run at once: for patches whose active tiles leave SMs idle
+// anyway, where a step lasts as long as its longest chain.
+template <int TX, int TY, bool WITH_SRC2>
+__device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const Geom& g, const Rec& R,
+                                                  const double* __restrict__ b, double* __restrict__ q_out, double dt,
+                                                  int i0, int j0, double* smem, bool& nan, double crit) {
+    using TG = TileGeom<TX, TY>;
+    static_assert(TX + 1 <= 16 && TY + 1 <= 16 && (TX + 2) * 16 <= 256 && (TY + 2) * 16 <= 256, "half-warp per slice");
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int dir = tid >> 8, gt = tid & 255;
+    TileMem M;
+    M.A = smem + (size_t)dir * NW * TG::NA;
+    M.B = smem + (size_t)2 * NW * TG::NA;
+    M.C = M.B + (size_t)10 * TG::NB;
+    M.D = M.C + (size_t)10 * TG::NC;
+    M.H = M.D + (size_t)10 * TG::ND;
+    M.Bd = M.H + TG::NHB;
+    M.T5 = nullptr;
+    M.Fy = M.Bd + TG::NHB;
+    char* per = reinterpret_cast<char*>(M.Fy + (size_t)10 * TG::NTS) + (size_t)dir * (8 * TG::NA + 16);
+    M.bits = reinterpret_cast<uint32_t*>(per);
+    M.list = reinterpret_cast<int*>(M.bits + TG::NA);
+    M.nlist = M.list + TG::NA;
+    M.NA = TG::NA;
+    M.hi0 = i0 - 3;
+    M.hj0 = j0 - 3;
+    M.hw = TG::HW;
+    M.hv = TX + 6;
+    bool any = false;
+    if (gt == 0) *M.nlist = 0;
+    for (int it = tid; it < TG::NHB; it += 512)
+        if (tile_stage_hb(g, R, b, M, it)) any = true;
+    any = __syncthreads_or(any) != 0;
+    nan = false;
+    if (!any) {
+        const size_t plane = (size_t)g.mx * g.my;
+        for (int it = tid; it < TX * TY; it += 512) {
+            int i = i0 + it % TX, j = j0 + it / TX;
+            if (i > g.mx || j > g.my) continue;
+            size_t c = (size_t)(j - 1) * g.mx + (size_t)(i - 1);
+            for (int m = 0; m < 5; ++m) q_out[(size_t)m * plane + c] = 0.0;
+        }
+        return 0.0;
+    }
+    const double dtdx = dt / g.dx, dtdy = dt / g.dy, dtd = dir == 0 ? dtdx : dtdy;
+    // the items that need a solve, as a dense list (tile_body)
+    const int nsolve = dir == 0 ? TG::NXW : TG::NYW;
+    for (int it0 = 0; it0 < nsolve; it0 += 256) {
+        const int it = it0 + gt;
+        bool need = it < nsolve && tile_needs_solve(P, g, M, dir, it, i0, j0, TX);
+        if (it < nsolve && !need) {
+            bool ok;
+            tile_riemann(P, g, R, M, dir, it, i0, j0, TX, TY, ok, crit);
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, need);
+        int base = 0;
+        if (lane == 0 && bal) base = atomicAdd(M.nlist, __popc(bal));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (need) M.list[base + __popc(bal & ((1u << lane) - 1u))] = it;
+    }
+    __syncthreads();
+    double cfl = 0.0;
+    const int nneed = *M.nlist;
+    for (int w = gt; w < nneed; w += 256) {
+        bool ok;
+        double s = tile_riemann(P, g, R, M, dir, M.list[w], i0, j0, TX, TY, ok, crit);
+        if (ok) cfl = fmax2(cfl, dtd * s);
+    }
+    __syncthreads();
+    {
+        const int sl = gt >> 4, k = gt & 15;
+        const int nsl = dir == 0 ? TY + 2 : TX + 2, span = dir == 0 ? TX : TY;
+        const int s = (dir == 0 ? j0 : i0) - 1 + sl, a = (dir == 0 ? i0 : j0) + k;
+        const int smax = dir == 0 ? g.my + 1 : g.mx + 1, amax = dir == 0 ? g.mx : g.my;
+        const bool sl_ok = sl < nsl && s >= 0 && s <= smax;
+        double v[15];
+        if (sl_ok && k <= span && a <= amax + 1) {
+            if (dir == 0) tile_x_iface<TX, TY>(P, M, s, a, i0, j0, dtd, v, nullptr);
+            else tile_y_iface<TX, TY>(P, M, s, a, i0, j0, dtd, v, nullptr);
+        } else {
+            for (int m = 0; m < 15; ++m) v[m] = 0.0;
+        }
+        double vn[15];
+        for (int m = 0; m < 15; ++m) vn[m] = __shfl_down_sync(0xffffffffu, v[m], 1);
+        if (sl_ok && k < span && a <= amax) {
+            if (dir == 0) tile_flux_cell<TX, TY, true>(P, g, R, M, 0, a, s, i0, j0, dtd, v, vn, 0, 0, nullptr);
+            else tile_flux_cell<TX, TY, true>(P, g, R, M, 1, s, a, i0, j0, dtd, v, vn, 0, 0, nullptr);
+        }
+    }
+    __syncthreads();
+    for (int it = tid; it < TX * TY; it += 512)
+        if (tile_final<TX, TY, WITH_SRC2, true>(P, g, R, M, it, i0, j0, dt, dtdx, dtdy, q_out)) nan = true;
+    if (!(cfl == cfl)) cfl = 0.0;
+    return cfl;
+}
+
+// the tiles of a small patch, one CTA each, with src2; the last CTA applies
+// the tick. A tile not flagged active writes its zeros.
+template <int TX, int TY>
+__global__ void __launch_bounds__(512, 1) k_tile_apart(dclaw_params P, Geom g, Rec R, const double* __restrict__ b,
+                                                       double* __restrict__ q_out, dclaw_clock* clk,
+                                                       const uint32_t* __restrict__ tflag) {
+    pdl_wait();
+    extern __shared__ double smem[];
+    const int i0 = 1 + blockIdx.x * TX, j0 = 1 + blockIdx.y * TY;
+    bool nan = false;
+    double cfl = 0.0;
+    if (tflag[blockIdx.y * gridDim.x + blockIdx.x] == clk->nsteps + 1u) {
+        cfl = tile_body_apart<TX, TY, true>(P, g, R, b, q_out, clk->dt, i0, j0, smem, nan, critical_root(P));
+    } else {
+        const size_t plane = (size_t)g.mx * g.my;
+        for (int it = threadIdx.x; it < TX * TY; it += 512) {
+            int i = i0 + it % TX, j = j0 + it / TX;
+            if (i > g.mx || j > g.my) continue;
+            size_t c = (size_t)(j - 1) * g.mx + (size_t)(i - 1);
+            for (int m = 0; m < 5; ++m) q_out[(size_t)m * plane + c] = 0.0;
+        }
+    }
+    if (nan) flag_status(clk, DCLAW_ERR_NAN);
+    warp_max_to(cfl, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
+    last_block_tick(P, clk);
+}
+
 // ty0: the first tile row of the launch (grid.y tile rows from there)
 template <int TX, int TY, bool WITH_SRC2>
 __global__ void __launch_bounds__(TILE_TPB, DCLAW_TILE_MINBLOCKS) k_tile(dclaw_params P, Geom g, Rec R, const double* __restrict__ b,
                                                  double* __restrict__ q_out, dclaw_clock* clk,
                                                  uint32_t* __restrict__ brlog, const uint32_t* __restrict__ tflag,
                                                  int ty0 = 0) {
+    pdl_wait();
     extern __shared__ double smem[];
     const int ty = (int)blockIdx.y + ty0;
     const int i0 = 1 + blockIdx.x * TX, j0 = 1 + ty * TY;
@@ -739,6 +869,7 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_cells(dclaw_params
                                                     double* __restrict__ q_out, dclaw_clock* clk,
                                                     const uint32_t* __restrict__ tflag, long long c0 = 0,
                                                     long long ncell = -1, int tick = 1) {
+    pdl_wait();
     const long long n = ncell < 0 ? (long long)g.mx * g.my : ncell;
     long long idx = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < c0 + n) {
@@ -1524,6 +1655,8 @@ inline int ensure_tile_smem_attr() {
                                      bytes) != cudaSuccess ||
                 cudaFuncSetAttribute(k_tile_list<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
                     cudaSuccess ||
+                cudaFuncSetAttribute(k_tile_apart<TILE_X, TILE_Y>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)TileGeom<TILE_X, TILE_Y>::SMEM2_BYTES) != cudaSuccess ||
                 cudaFuncSetAttribute(k_tile_list<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
                 return DCLAW_ERR_CUDA;
             done[dev].store(true, std::memory_order_release);
@@ -1531,6 +1664,23 @@ inline int ensure_tile_smem_attr() {
     }
     return DCLAW_OK;
 }
+
+// Patches up to this many cells step in two launches, k_records over every
+// padded cell and k_tile_apart over every tile (src2method 2 keeps the lists:
+// its lanes take cells from them). Their active tiles do not fill the SMs, so
+// a step lasts as long as its longest chain, which the lists' three more
+// launches and the tile's two sweeps in turn lengthen. A step over the lists
+// against this, in us (share of the patch that is wet): 64^2 (0.2) 55.8 and
+// 34.0, 200^2 (0.5) 61.5 and 37.0, 333 x 200 (0.3) 63.5 and 47.2, 316^2 (0.9)
+// 91.0 and 80.9, 350^2 (0.3) 64.3 and 65.3, 350^2 (0.9) 95 and 102,
+// 512^2 (0.1) 61 and 73. The records take 84 registers there, without the
+// spills that pay where occupancy counts.
+#ifndef DCLAW_SMALL_CELLS
+#define DCLAW_SMALL_CELLS 100000
+#endif
+constexpr long long SMALL_CELLS = DCLAW_SMALL_CELLS;
+constexpr int SMALL_RECORDS_MINB = 2, SMALL_RECORDS_TPB = 128;
+inline unsigned small_blocks(long long n) { return (unsigned)((n + SMALL_RECORDS_TPB - 1) / SMALL_RECORDS_TPB); }
 
 // src2 over the active list (g3: k_src2_list's grid)
 inline void launch_src2_list(const dclaw_params& P, const Geom& g, const double* qstar, double* q_out,
@@ -1756,9 +1906,10 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
     }
     uint32_t* tflag = (uint32_t*)((char*)work + L.off_tflag);
     const int ntx = (mx + TILE_X - 1) / TILE_X, nty = (my + TILE_Y - 1) / TILE_Y;
-    if (!branch_log) {
+    const bool small = (long long)mx * my <= SMALL_CELLS && p->src2method != 2;
+    if (!branch_log && !small) {
         // over the tile lists (the branch log needs every interface's bits,
-        // so it keeps the full-grid kernels below)
+        // so it keeps the full-grid kernels at the end)
         const int nsm = sm_count();
         if (nsm <= 0) return DCLAW_ERR_CUDA;
         unsigned int* counters = (unsigned int*)((char*)work + L.off_counters);
@@ -1788,16 +1939,23 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
         launch_src2_list(P, g, qstar, q_out, clock, counters, list_act, g3, nsm, ntiles, 1, s);
         return cuda_status();
     }
-    k_records<<<nblocks((long long)L.npad), TPB, 0, s>>>(P, g, q_in, b, R, clock, tflag);
     dim3 grid(ntx, nty);
+    if (!branch_log) {
+        launch_pdl(k_records<SMALL_RECORDS_MINB>, dim3(small_blocks((long long)L.npad)), dim3(SMALL_RECORDS_TPB), 0, s, P, g,
+                   q_in, b, R, clock, tflag, 0, -1);
+        launch_pdl(k_tile_apart<TILE_X, TILE_Y>, grid, dim3(512), TG::SMEM2_BYTES, s, P, g, R, b, q_out, clock, tflag);
+        return cuda_status();
+    }
+    k_records<DCLAW_PLAIN_CELL_MINB><<<nblocks((long long)L.npad), TPB, 0, s>>>(P, g, q_in, b, R, clock, tflag);
     if (DCLAW_SRC2_KERNEL) {
         double* qstar = (double*)((char*)work + L.off_qstar);
-        k_tile<TILE_X, TILE_Y, false><<<grid, TILE_TPB, TG::SMEM_BYTES, s>>>(P, g, R, b, qstar, clock, branch_log,
-                                                                             tflag);
-        k_src2_cells<<<src2_blocks((long long)mx * my), SRC2_TPB, 0, s>>>(P, g, qstar, q_out, clock, tflag);
+        launch_pdl(k_tile<TILE_X, TILE_Y, false>, grid, dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock,
+                   branch_log, tflag, 0);
+        launch_pdl(k_src2_cells, dim3(src2_blocks((long long)mx * my)), dim3(SRC2_TPB), 0, s, P, g, qstar, q_out, clock,
+                   tflag, 0ll, -1ll, 1);
     } else {
-        k_tile<TILE_X, TILE_Y, true><<<grid, TILE_TPB, TG::SMEM_BYTES, s>>>(P, g, R, b, q_out, clock, branch_log,
-                                                                            tflag);
+        launch_pdl(k_tile<TILE_X, TILE_Y, true>, grid, dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, q_out, clock,
+                   branch_log, tflag, 0);
     }
     return cuda_status();
 }
@@ -1865,7 +2023,7 @@ int dclaw_step_host(const double* q_in, double* q_out, const double* b, int mx, 
         const int jb = k == nb - 1 ? my + 2 : (first[k + 1] * TILE_Y + 2 < my + 2 ? first[k + 1] * TILE_Y + 2 : my + 2);
         if (jb >= ja) {
             const int nrow = jb - ja + 1;
-            k_records<<<nblocks((long long)g.PX * nrow), TPB, 0, s>>>(P, g, dq_in, b, R, clock, tflag, ja + 1, nrow);
+            k_records<DCLAW_PLAIN_CELL_MINB><<<nblocks((long long)g.PX * nrow), TPB, 0, s>>>(P, g, dq_in, b, R, clock, tflag, ja + 1, nrow);
             ja = jb + 1;
         }
         const int nty = first[k + 1] - first[k];
@@ -2184,7 +2342,7 @@ int dclaw_step_noalloc(const double* q_in, double* q_out, const double* b, int m
     const size_t npad = (size_t)(mx + 4) * (my + 4);
     Rec R{scratch, npad};
     const dclaw_params P = *p;
-    k_records<<<nblocks((long long)npad), TPB, 0, s>>>(P, g, q_in, b, R, clock, nullptr);
+    k_records<DCLAW_PLAIN_CELL_MINB><<<nblocks((long long)npad), TPB, 0, s>>>(P, g, q_in, b, R, clock, nullptr);
     dim3 grid((mx + TILE_X - 1) / TILE_X, (my + TILE_Y - 1) / TILE_Y);
     k_tile<TILE_X, TILE_Y, true><<<grid, TILE_TPB, TileGeom<TILE_X, TILE_Y>::SMEM_BYTES, s>>>(P, g, R, b, q_out, clock,
                                                                                      nullptr, nullptr);

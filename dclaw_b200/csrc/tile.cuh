@@ -213,6 +213,10 @@ struct TileGeom {
     // + branch bits of the sweep's items, the list of items that need a
     // solve, and its length
     static constexpr size_t SMEM_BYTES = SMEM_DOUBLES * 8 + 4 * (size_t)NA + 4 * (size_t)NA + 16;
+    // both sweeps side by side: waves, bits and list of each, the y-fluxes
+    // in place of T
+    static constexpr size_t SMEM2_DOUBLES = 2 * (size_t)NW * NA + 10 * NB + 10 * NC + 10 * ND + 2 * NHB + 10 * NTS;
+    static constexpr size_t SMEM2_BYTES = SMEM2_DOUBLES * 8 + 2 * (8 * (size_t)NA + 16);
 };
 
 struct TileMem {
@@ -223,6 +227,7 @@ struct TileMem {
     double* H;   // record h of cells (i0-3..i0+TX+2) x (j0-3..j0+TY+2), row pitch hw
     double* Bd;  // bed of the same cells
     double* T5;  // [NTS][5]: T(k, c) of the x-sweep, read by the y-sweep's flux phase
+    double* Fy;  // [NTS][10]: y-fluxes faddm/faddp, where the sweeps run side by side (APART)
     uint32_t* bits;  // NA Riemann branch bits of the current sweep
     int* list;       // NA: items of the current sweep that need a solve
     int* nlist;      // length of the list
@@ -500,7 +505,7 @@ DC_HD void tile_y_iface(const dclaw_params& P, const TileMem& M, int c, int a, i
     iface_limited(P, M, 1, witem(a - 1), witem(a), witem(a + 1), h0, dtdy, v, v + 5, v + 10, bits);
 }
 
-template <int TX, int TY>
+template <int TX, int TY, bool APART = false>
 DC_HD void tile_flux_cell(const dclaw_params& P, const Geom& g, const Rec& R, const TileMem& M, int dir, int c,
                           int r, int i0, int j0, double dtdx, const double* v0, const double* v1, uint32_t lb0,
                           uint32_t lb1, uint32_t* log);
@@ -538,7 +543,9 @@ DC_HD void tile_flux(const dclaw_params& P, const Geom& g, const Rec& R, const T
 
 // The rest of tile_flux for cell (c, r), given the limited fluctuations of
 // its own interface (v0, limiter bits lb0) and of the next one (v1, lb1).
-template <int TX, int TY>
+// APART: the sweeps run side by side, so the y-fluxes are stored by
+// themselves and tile_final adds T to them.
+template <int TX, int TY, bool APART>
 DC_HD void tile_flux_cell(const dclaw_params& P, const Geom& g, const Rec& R, const TileMem& M, int dir, int c,
                           int r, int i0, int j0, double dtdx, const double* v0, const double* v1, uint32_t lb0,
                           uint32_t lb1, uint32_t* log) {
@@ -573,6 +580,15 @@ DC_HD void tile_flux_cell(const dclaw_params& P, const Geom& g, const Rec& R, co
             if (last) {
                 fadd(am1, ap1, cq1, fm, fp);
                 dst = M.B + (size_t)((r - j0) * (TX + 1) + (c + 1 - i0)) * 10;
+                for (int m = 0; m < 5; ++m) { dst[m] = fm[m]; dst[5 + m] = fp[m]; }
+            }
+        } else if (APART) {
+            fadd(am0, ap0, cq0, fm, fp);
+            double* dst = M.Fy + (size_t)((r - j0) * TX + (c - i0)) * 10;
+            for (int m = 0; m < 5; ++m) { dst[m] = fm[m]; dst[5 + m] = fp[m]; }
+            if (last) {
+                fadd(am1, ap1, cq1, fm, fp);
+                dst = M.Fy + (size_t)((r + 1 - j0) * TX + (c - i0)) * 10;
                 for (int m = 0; m < 5; ++m) { dst[m] = fm[m]; dst[5 + m] = fp[m]; }
             }
         } else {
@@ -663,7 +679,8 @@ DC_HD void tile_T_store(const TileMem& M, int item, const double T[5]) {
 // flux-differencing update of tile cell (i, j), written to q_out (interior
 // layout); with WITH_SRC2 the cell's src2 follows in the same thread,
 // otherwise q_out holds the updated state before src2. Returns true on NaN.
-template <int TX, int TY, bool WITH_SRC2>
+// APART: gm/gp = T + faddm_y/faddp_y are summed here (tile_flux_cell).
+template <int TX, int TY, bool WITH_SRC2, bool APART = false>
 DC_HD bool tile_final(const dclaw_params& P, const Geom& g, const Rec& R, const TileMem& M, int item, int i0,
                       int j0, double dt, double dtdx, double dtdy, double* __restrict__ q_out) {
     int i = i0 + item % TX, j = j0 + item / TX;
@@ -681,14 +698,21 @@ DC_HD bool tile_final(const dclaw_params& P, const Geom& g, const Rec& R, const 
     const double* Gy_im = M.D + (size_t)((i - 1 - (i0 - 1)) * TY + (j - j0)) * 10;  // column i-1
     const double* Gy_i = Gy_im + (size_t)10 * TY;
     const double* Gy_ip = Gy_im + (size_t)20 * TY;
-    const double* C0 = M.C + (size_t)((j - j0) * TX + (i - i0)) * 10;       // y-iface j
-    const double* C1 = M.C + (size_t)((j + 1 - j0) * TX + (i - i0)) * 10;   // y-iface j+1
+    const double* Y = APART ? M.Fy : M.C;
+    const double* C0 = Y + (size_t)((j - j0) * TX + (i - i0)) * 10;       // y-iface j
+    const double* C1 = Y + (size_t)((j + 1 - j0) * TX + (i - i0)) * 10;   // y-iface j+1
+    // APART: the x-sweep's G1x/G2x of rows j-1, j, j+1 (T of interfaces j, j+1)
+    const double* G = M.C + (size_t)((j - j0) * TX + (i - i0)) * 10;
     double qn[5];
     for (int m = 0; m < 5; ++m) {
         double fm = ((0.0 + Fx1[m]) + Gy_i[5 + m]) + Gy_ip[m];
         double fp = ((0.0 + Fx0[5 + m]) + Gy_im[5 + m]) + Gy_i[m];
         double gm = C1[m];
         double gp = C0[5 + m];
+        if (APART) {
+            gm = ((0.0 + G[10 * TX + 5 + m]) + G[20 * TX + m]) + gm;
+            gp = ((0.0 + G[5 + m]) + G[10 * TX + m]) + gp;
+        }
         qn[m] = qb[m] - dtdx * (fm - fp) - dtdy * (gm - gp);
     }
     bool nan = (qn[0] != qn[0]) || (qn[1] != qn[1]) || (qn[2] != qn[2]) || (qn[3] != qn[3]) || (qn[4] != qn[4]);
