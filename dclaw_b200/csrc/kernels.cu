@@ -1712,14 +1712,16 @@ constexpr int MAX_HOST_BANDS = 64;
 
 inline int host_auto_bands(int mx, int my) {
     const int nty = (my + TILE_Y - 1) / TILE_Y;
-    // about 28 MB of state per band: enough work per band to fill the GPU
-    // and few enough launches and copies, fine enough that the first upload
-    // and the last download (the parts that do not overlap) stay short. On
-    // the 4096^2 state (24 bands) the step then takes 15.2 ms, 1.03x the
-    // bare copies both ways at once (14.7 ms); 12, 17, 20, 28 and 32 bands
-    // took 15.7, 15.5, 15.2, 15.5 and 15.6 ms, 4 bands 1.25x, 64 bands 1.22x.
+    // About 4 MB of state per band up to 10 bands, then about 28 MB: enough
+    // work per band to pay for its launches and copies, fine enough that the
+    // first upload and the last download (the parts that do not overlap)
+    // stay short. 512^2 in 1, 3, 6 bands takes 0.55, 0.40, 0.47 ms; 1024^2
+    // in 2, 6, 10, 16 bands 1.43, 1.31, 1.09, 1.22 ms (bare copies both ways
+    // at once: 0.89); 2048^2 in 6, 10, 16 bands 4.24, 4.19, 4.24 ms (3.45);
+    // 4096^2 in 12, 20, 24, 32 bands 15.9, 15.1, 15.3, 15.2 ms (14.5).
     const double state = 40.0 * mx * (double)my;
-    int nb = (int)(state / 28.0e6) + 1;
+    const int fine = (int)(state / 4.0e6) + 1, coarse = (int)(state / 28.0e6) + 1;
+    int nb = fine < 10 ? fine : (coarse > 10 ? coarse : 10);
     if (nb > MAX_HOST_BANDS) nb = MAX_HOST_BANDS;
     if (nb > nty) nb = nty;
     return nb < 1 ? 1 : nb;
@@ -1763,11 +1765,15 @@ inline HostPipe* host_pipe() {
 
 inline size_t host_state_bytes(int mx, int my) { return align256((size_t)5 * mx * my * 8); }
 
-// rows lo .. hi (1-based, inclusive) of the five planes of a state
+// rows lo .. hi (1-based, inclusive) of the five planes of a state: in one
+// copy of five rows for patches up to 16 MB a plane, where the copies' own
+// cost shows (1024^2 in 10 bands 1.09 ms, 1.64 ms with a copy per plane); above,
+// a copy per plane (4096^2 in 20 bands 15.07 ms against 15.43)
 inline cudaError_t copy_rows(double* dst, const double* src, int mx, int my, int lo, int hi, cudaMemcpyKind kind,
                              cudaStream_t s) {
     if (lo > hi) return cudaSuccess;
     const size_t plane = (size_t)mx * my, off = (size_t)(lo - 1) * mx, n = (size_t)(hi - lo + 1) * mx;
+    if (plane * 8 <= (16u << 20)) return cudaMemcpy2DAsync(dst + off, plane * 8, src + off, plane * 8, n * 8, 5, kind, s);
     for (int m = 0; m < 5; ++m) {
         cudaError_t e = cudaMemcpyAsync(dst + m * plane + off, src + m * plane + off, n * 8, kind, s);
         if (e != cudaSuccess) return e;
@@ -2014,6 +2020,16 @@ int dclaw_step_host(const double* q_in, double* q_out, const double* b, int mx, 
         e = copy_rows(dq_in, q_in, mx, my, lo, hi, cudaMemcpyHostToDevice, hp->up);
         if (e == cudaSuccess) e = cudaEventRecord(hp->ev_up[k], hp->up);
         lo = hi + 1 > lo ? hi + 1 : lo;
+    }
+    if (nb == 1 && e == cudaSuccess) {
+        // one band: the device step between the two copies
+        e = cudaStreamWaitEvent(s, hp->ev_up[0], 0);
+        if (e == cudaSuccess) {
+            rc = dclaw_step(dq_in, dq_out, b, mx, my, dx, dy, p, clock, work, L.total_fused, nullptr, stream);
+            if (rc) return rc;
+            e = copy_rows(q_out, dq_out, mx, my, 1, my, cudaMemcpyDeviceToHost, s);
+        }
+        return e == cudaSuccess ? cuda_status() : DCLAW_ERR_CUDA;
     }
     // compute on the caller's stream, downloads behind it
     int ja = -1;
