@@ -1152,89 +1152,116 @@ DC_HD void load_a2_b(const dclaw_params& P, const Work& W, size_t pi, int cn, in
     qb[4] += pb;
 }
 
-// Adjoints produced by the reverse of one interface's flux stage: its own
-// 15 stored values, the wave components (12, no speeds; W1, W2 h/n, W5) of
-// the interfaces on its left and right (limiter), and the A2 states of
-// cells i-1 and i (transverse splits).
-struct FluxB {
-    double self[NW];
-    double left[12], right[12];
-    double a2l[4], a2r[4];
-};
-
-DC_HD void waves_to_compact(int cn, int ct, const double W1[5], const double W2[5], const double W5[5],
-                            double* o /*12*/) {
-    o[0] = W1[0]; o[1] = W1[cn]; o[2] = W1[ct]; o[3] = W1[3]; o[4] = W1[4];
-    o[5] = W2[0]; o[6] = W2[cn];
-    o[7] = W5[0]; o[8] = W5[cn]; o[9] = W5[ct]; o[10] = W5[3]; o[11] = W5[4];
+// One wave family's components of interface oi as a 5-vector in q order
+// (f 0: wave 1, 1: wave 2, 2: wave 5; expand_waves for one family)
+template <int DIR>
+DC_HD void family_wave(const double* __restrict__ wv, size_t nplane, size_t oi, int f, double Wf[5]) {
+    const int cn = DIR == 0 ? 1 : 2, ct = DIR == 0 ? 2 : 1;
+    const double* v = wv + (size_t)(f == 0 ? W_1H : f == 1 ? W_2H : W_5H) * nplane + oi;
+    const bool all = f != 1;   // wave 2 has its h and normal components only
+    Wf[0] = v[0];
+    Wf[cn] = v[nplane];
+    Wf[ct] = all ? v[2 * nplane] : 0.0;
+    Wf[3] = all ? v[3 * nplane] : 0.0;
+    Wf[4] = all ? v[4 * nplane] : 0.0;
 }
 
-// Stage D reverse. fb[30]: adjoints of the interface's faddm, faddp, U1m,
-// U1p, U2m, U2p (5 each, q order).
+// the limiter's factor of a family (limit_family, which leaves a wave of
+// zero norm as it is: 1)
+DC_HD double limit_factor(int mth, double s, const double Wm[5], const double Wi[5], const double Wp[5]) {
+    double wnorm2 = 0.0, dotl = 0.0, dotr = 0.0;
+    for (int m = 0; m < 5; ++m) {
+        wnorm2 = wnorm2 + sq(Wi[m]);
+        dotl = dotl + Wm[m] * Wi[m];
+        dotr = dotr + Wi[m] * Wp[m];
+    }
+    if (wnorm2 == 0.0) return 1.0;
+    uint32_t code;
+    return limiter_phi(mth, (s > 0.0 ? dotl : dotr) / wnorm2, code);
+}
+
+// Stage D reverse at interface i of slice r, from the adjoints lam of the
+// updated interior states (5 planes mx*my, before src2; stage_update's
+// accumulation) to the interface's NFB slots of dst (npl apart): its own 15
+// stored values, the wave components (12, no speeds) of the interfaces on
+// its left and right (limiter), and the A2 states (4 each) of cells i-1 and i
+// (transverse splits). The values of an interface, 45 waves, 30 flux
+// adjoints and 47 results, are three times the registers a thread has when
+// two CTAs share an SM: kept whole they spilled 1.4 KB a thread, more than
+// the L1 holds, and the kernel waited on that. So the waves are read by
+// family, in both passes, each result is stored when it is known, and what
+// lives across the passes is the fluctuations' and corrections' adjoints.
+// The families and the two splits are loops, not copies, for the
+// instruction cache.
 template <int DIR>
-DC_HD void stage_flux_b(const dclaw_params& P, const Geom& g, const Work& W, int r, int i, double dtdx,
-                        const double* fb, FluxB& o) {
+DC_HD void stage_flux_b(const dclaw_params& P, const Geom& g, const Work& W, const double* __restrict__ lam, int r,
+                        int i, double dt, double* __restrict__ dst, size_t npl) {
     const double* wv = DIR == 0 ? W.wx : W.wy;
     const size_t nplane = DIR == 0 ? W.nxi : W.nyi;
     auto oidx = [&](int ii) -> size_t { return DIR == 0 ? xidx(g, r, ii) : yidx(g, ii, r); };
     auto cidx = [&](int ii) -> size_t { return DIR == 0 ? pidx(g, ii, r) : pidx(g, r, ii); };
     const int cn = DIR == 0 ? 1 : 2, ct = DIR == 0 ? 2 : 1;
-    for (int k = 0; k < NW; ++k) o.self[k] = 0.0;
-    for (int k = 0; k < 12; ++k) { o.left[k] = 0.0; o.right[k] = 0.0; }
-    for (int k = 0; k < 4; ++k) { o.a2l[k] = 0.0; o.a2r[k] = 0.0; }
-
-    double s[3], W1[5], W2[5], W5[5];
-    expand_waves<DIR>(wv, nplane, oidx(i), s, W1, W2, W5);
-    double amdq[5], apdq[5];
-    for (int m = 0; m < 5; ++m) {
-        double am = 0.0, ap = 0.0;
-        if (s[0] < 0.0) am = am + W1[m]; else if (s[0] > 0.0) ap = ap + W1[m];
-        if (s[1] < 0.0) am = am + W2[m]; else if (s[1] > 0.0) ap = ap + W2[m];
-        if (s[2] < 0.0) am = am + W5[m]; else if (s[2] > 0.0) ap = ap + W5[m];
-        amdq[m] = am;
-        apdq[m] = ap;
-    }
-    double L1[5], L2[5], L5[5];  // limited waves
-    for (int m = 0; m < 5; ++m) { L1[m] = W1[m]; L2[m] = W2[m]; L5[m] = W5[m]; }
-    double sm[3], Wm1[5], Wm2[5], Wm5[5], sp[3], Wp1[5], Wp2[5], Wp5[5];
-    bool lim = P.order != 1 && P.limiter != 0;
+    const double dtdn = DIR == 0 ? dt / g.dx : dt / g.dy, dtdt = DIR == 0 ? dt / g.dy : dt / g.dx;
+    const size_t oi = oidx(i), plane = (size_t)g.mx * g.my;
+    const bool second = P.order != 1, lim = second && P.limiter != 0;
+    const bool fold = P.order > 1 && P.transverse_waves == 2;
+    // adjoint of component m of cell c along the slice, d slices across
+    auto L = [&](int c, int d, int m) -> double {
+        const int ci = DIR == 0 ? c : r + d, cj = DIR == 0 ? r + d : c;
+        if (ci < 1 || ci > g.mx || cj < 1 || cj > g.my) return 0.0;
+        return lam[(size_t)m * plane + (size_t)(cj - 1) * g.mx + (size_t)(ci - 1)];
+    };
     bool wet4 = false;
-    double cqxx[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    double c1 = 0.0, c2 = 0.0, c5 = 0.0;
-    if (P.order != 1) {
-        if (lim) {
-            expand_waves<DIR>(wv, nplane, oidx(i - 1), sm, Wm1, Wm2, Wm5);
-            expand_waves<DIR>(wv, nplane, oidx(i + 1), sp, Wp1, Wp2, Wp5);
-            limit_family(P.limiter, 1, s[0], Wm1, L1, Wp1, nullptr);
-            limit_family(P.limiter, 2, s[1], Wm2, L2, Wp2, nullptr);
-            limit_family(P.limiter, 5, s[2], Wm5, L5, Wp5, nullptr);
-        }
+    if (second) {
         double hl2 = W.qB[cidx(i - 2)], hl = W.qB[cidx(i - 1)], hr = W.qB[cidx(i)], hr2 = W.qB[cidx(i + 1)];
         wet4 = hl * hr * hl2 * hr2 > 0.0;
-        if (wet4) {
-            c1 = fsign(1.0, s[0]) * (1.0 - fabs(s[0]) * dtdx);
-            c2 = fsign(1.0, s[1]) * (1.0 - fabs(s[1]) * dtdx);
-            c5 = fsign(1.0, s[2]) * (1.0 - fabs(s[2]) * dtdx);
+    }
+    // ---- forward: limiter factors, the splits' fluctuations ----
+    double wl[3] = {1.0, 1.0, 1.0};
+    double as1[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, as2[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    {
+        double cq[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int f = 0; f < 3; ++f) {
+            double Wf[5];
+            const double s = wv[(size_t)f * nplane + oi];
+            family_wave<DIR>(wv, nplane, oi, f, Wf);
+            double w = 1.0;
+            if (lim) {
+                double Wm[5], Wp[5];
+                family_wave<DIR>(wv, nplane, oidx(i - 1), f, Wm);
+                family_wave<DIR>(wv, nplane, oidx(i + 1), f, Wp);
+                w = limit_factor(P.limiter, s, Wm, Wf, Wp);
+            }
+            wl[0] = f == 0 ? w : wl[0];
+            wl[1] = f == 1 ? w : wl[1];
+            wl[2] = f == 2 ? w : wl[2];
+            const double c = fsign(1.0, s) * (1.0 - fabs(s) * dtdn);
             for (int m = 0; m < 5; ++m) {
-                double cq = 0.0;
-                cq = cq + c1 * L1[m];
-                cq = cq + c2 * L2[m];
-                cq = cq + c5 * L5[m];
-                cqxx[m] = cq;
+                if (s < 0.0) as1[m] = as1[m] + Wf[m];
+                else if (s > 0.0) as2[m] = as2[m] + Wf[m];
+                if (wet4) cq[m] = cq[m] + c * (w * Wf[m]);
             }
         }
+        if (fold)
+            for (int m = 0; m < 5; ++m) {
+                as1[m] = as1[m] + cq[m];
+                as2[m] = as2[m] - cq[m];
+            }
     }
     // ---- reverse ----
     double amdqb[5], apdqb[5], cqxxb[5];
     for (int m = 0; m < 5; ++m) {
-        amdqb[m] = fb[m];
-        apdqb[m] = -fb[5 + m];
-        cqxxb[m] = P.order != 1 ? 0.5 * fb[m] + 0.5 * fb[5 + m] : 0.0;
+        const double fm = -dtdn * L(i - 1, 0, m), fp = dtdn * L(i, 0, m);
+        amdqb[m] = fm;
+        apdqb[m] = -fp;
+        cqxxb[m] = second ? 0.5 * fm + 0.5 * fp : 0.0;
     }
-    if (P.transverse_waves != 0) {
-        const bool fold = P.order > 1 && P.transverse_waves == 2;
-        const double half = 0.5 * dtdx;
-        for (int imp = 1; imp <= 2; ++imp) {
+#pragma unroll 1
+    for (int imp = 1; imp <= 2; ++imp) {
+        double xb[4] = {0.0, 0.0, 0.0, 0.0};
+        if (P.transverse_waves != 0) {
+            const double half = 0.5 * dtdn;
             const int cc = imp == 1 ? i - 1 : i;
             const size_t pc = cidx(cc);
             double h, hn, ht, hm;
@@ -1242,101 +1269,73 @@ DC_HD void stage_flux_b(const dclaw_params& P, const Geom& g, const Work& W, int
             double topo1, topo3;
             if (DIR == 0) { topo1 = W.bP[pidx(g, cc, r - 1)]; topo3 = W.bP[pidx(g, cc, r + 1)]; }
             else { topo1 = W.bP[pidx(g, r - 1, cc)]; topo3 = W.bP[pidx(g, r + 1, cc)]; }
-            const double* src = imp == 1 ? amdq : apdq;
-            double asdq[5];
+            double as[5], bm[5], bp[5];
             for (int m = 0; m < 5; ++m) {
-                double v = src[m];
-                if (fold) v = imp == 1 ? v + cqxx[m] : v - cqxx[m];
-                asdq[m] = v;
+                as[m] = imp == 1 ? as1[m] : as2[m];
+                const double l0 = L(cc, 0, m);
+                bm[m] = half * (dtdt * (L(cc, -1, m) - l0));
+                bp[m] = half * (dtdt * (l0 - L(cc, 1, m)));
             }
-            double asdq_s[5] = {asdq[0], asdq[cn], asdq[ct], asdq[3], asdq[4]};
-            const int ob = imp == 1 ? 10 : 20;
-            double bmb_q[5], bpb_q[5];
-            for (int m = 0; m < 5; ++m) {
-                bmb_q[m] = half * fb[ob + m];
-                bpb_q[m] = half * fb[ob + 5 + m];
-            }
-            double bmb[5] = {bmb_q[0], bmb_q[cn], bmb_q[ct], bmb_q[3], bmb_q[4]};
-            double bpb[5] = {bpb_q[0], bpb_q[cn], bpb_q[ct], bpb_q[3], bpb_q[4]};
+            const double asdq_s[5] = {as[0], as[cn], as[ct], as[3], as[4]};
+            const double bmb[5] = {bm[0], bm[cn], bm[ct], bm[3], bm[4]};
+            const double bpb[5] = {bp[0], bp[cn], bp[ct], bp[3], bp[4]};
             double asb_s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-            double* xb = imp == 1 ? o.a2l : o.a2r;
             rpt2_split_b(P, h, hn, ht, hm, W.bP[pc], topo1, topo3, asdq_s, bmb, bpb, xb, asb_s);
             double asb[5];
             asb[0] = asb_s[0]; asb[cn] = asb_s[1]; asb[ct] = asb_s[2]; asb[3] = asb_s[3]; asb[4] = asb_s[4];
             for (int m = 0; m < 5; ++m) {
-                if (imp == 1) { amdqb[m] += asb[m]; if (fold) cqxxb[m] += asb[m]; }
-                else { apdqb[m] += asb[m]; if (fold) cqxxb[m] -= asb[m]; }
+                if (imp == 1) amdqb[m] += asb[m];
+                else apdqb[m] += asb[m];
+                if (fold) cqxxb[m] += imp == 1 ? asb[m] : -asb[m];
             }
         }
+        for (int k = 0; k < 4; ++k) dst[(size_t)(35 + 4 * imp + k) * npl + oi] = xb[k];
     }
-    double L1b[5] = {0, 0, 0, 0, 0}, L2b[5] = {0, 0, 0, 0, 0}, L5b[5] = {0, 0, 0, 0, 0};
-    double sb[3] = {0.0, 0.0, 0.0};
-    if (wet4) {
-        double c1b = 0.0, c2b = 0.0, c5b = 0.0;
+#pragma unroll 1
+    for (int f = 0; f < 3; ++f) {
+        double Wf[5], Wb[5];
+        const double s = wv[(size_t)f * nplane + oi];
+        family_wave<DIR>(wv, nplane, oi, f, Wf);
+        const double w = f == 0 ? wl[0] : f == 1 ? wl[1] : wl[2];
+        double sb = 0.0;
+        for (int m = 0; m < 5; ++m) Wb[m] = 0.0;
+        if (wet4) {
+            const double c = fsign(1.0, s) * (1.0 - fabs(s) * dtdn);
+            double cb = 0.0;
+            for (int m = 0; m < 5; ++m) {
+                Wb[m] += c * cqxxb[m];
+                cb += cqxxb[m] * (w * Wf[m]);
+            }
+            // c = sign(1, s) (1 - |s| dtdx): dc/ds = -dtdx for s != 0
+            if (s != 0.0) sb -= cb * dtdn;
+        }
+        double Wmb[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, Wpb[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (lim) {
+            double Wm[5], Wp[5];
+            family_wave<DIR>(wv, nplane, oidx(i - 1), f, Wm);
+            family_wave<DIR>(wv, nplane, oidx(i + 1), f, Wp);
+            limit_family_b(P.limiter, s, Wm, Wf, Wp, Wb, Wmb, Wpb);
+        }
         for (int m = 0; m < 5; ++m) {
-            L1b[m] += c1 * cqxxb[m];
-            L2b[m] += c2 * cqxxb[m];
-            L5b[m] += c5 * cqxxb[m];
-            c1b += cqxxb[m] * L1[m];
-            c2b += cqxxb[m] * L2[m];
-            c5b += cqxxb[m] * L5[m];
+            if (s < 0.0) Wb[m] += amdqb[m];
+            else if (s > 0.0) Wb[m] += apdqb[m];
         }
-        // c = sign(1, s) (1 - |s| dtdx): dc/ds = -dtdx for s != 0
-        if (s[0] != 0.0) sb[0] -= c1b * dtdx;
-        if (s[1] != 0.0) sb[1] -= c2b * dtdx;
-        if (s[2] != 0.0) sb[2] -= c5b * dtdx;
-    }
-    double W1b[5], W2b[5], W5b[5];
-    for (int m = 0; m < 5; ++m) { W1b[m] = L1b[m]; W2b[m] = L2b[m]; W5b[m] = L5b[m]; }
-    if (lim) {
-        double Wm1b[5] = {0, 0, 0, 0, 0}, Wm2b[5] = {0, 0, 0, 0, 0}, Wm5b[5] = {0, 0, 0, 0, 0};
-        double Wp1b[5] = {0, 0, 0, 0, 0}, Wp2b[5] = {0, 0, 0, 0, 0}, Wp5b[5] = {0, 0, 0, 0, 0};
-        limit_family_b(P.limiter, s[0], Wm1, W1, Wp1, W1b, Wm1b, Wp1b);
-        limit_family_b(P.limiter, s[1], Wm2, W2, Wp2, W2b, Wm2b, Wp2b);
-        limit_family_b(P.limiter, s[2], Wm5, W5, Wp5, W5b, Wm5b, Wp5b);
-        waves_to_compact(cn, ct, Wm1b, Wm2b, Wm5b, o.left);
-        waves_to_compact(cn, ct, Wp1b, Wp2b, Wp5b, o.right);
-    }
-    for (int m = 0; m < 5; ++m) {
-        if (s[0] < 0.0) W1b[m] += amdqb[m]; else if (s[0] > 0.0) W1b[m] += apdqb[m];
-        if (s[1] < 0.0) W2b[m] += amdqb[m]; else if (s[1] > 0.0) W2b[m] += apdqb[m];
-        if (s[2] < 0.0) W5b[m] += amdqb[m]; else if (s[2] > 0.0) W5b[m] += apdqb[m];
-    }
-    o.self[W_S1] = sb[0]; o.self[W_S2] = sb[1]; o.self[W_S5] = sb[2];
-    o.self[W_1H] = W1b[0]; o.self[W_1N] = W1b[cn]; o.self[W_1T] = W1b[ct]; o.self[W_1M] = W1b[3];
-    o.self[W_1P] = W1b[4];
-    o.self[W_2H] = W2b[0]; o.self[W_2N] = W2b[cn];
-    o.self[W_5H] = W5b[0]; o.self[W_5N] = W5b[cn]; o.self[W_5T] = W5b[ct]; o.self[W_5M] = W5b[3];
-    o.self[W_5P] = W5b[4];
-}
-
-// Adjoint of the 30 stored flux values of interface i of slice r from the
-// adjoints lam of the updated interior states (5 planes mx*my, before src2),
-// following stage_update's accumulation.
-template <int DIR>
-DC_HD void flux_bar(const Geom& g, const double* __restrict__ lam, int r, int i, double dt, double* fb) {
-    const double dtdx = dt / g.dx, dtdy = dt / g.dy;
-    const size_t plane = (size_t)g.mx * g.my;
-    auto L = [&](int ci, int cj, int m) -> double {
-        if (ci < 1 || ci > g.mx || cj < 1 || cj > g.my) return 0.0;
-        return lam[(size_t)m * plane + (size_t)(cj - 1) * g.mx + (size_t)(ci - 1)];
-    };
-    for (int m = 0; m < 5; ++m) {
-        if (DIR == 0) {
-            fb[m] = -dtdx * L(i - 1, r, m);
-            fb[5 + m] = dtdx * L(i, r, m);
-            fb[10 + m] = dtdy * (L(i - 1, r - 1, m) - L(i - 1, r, m));
-            fb[15 + m] = dtdy * (L(i - 1, r, m) - L(i - 1, r + 1, m));
-            fb[20 + m] = dtdy * (L(i, r - 1, m) - L(i, r, m));
-            fb[25 + m] = dtdy * (L(i, r, m) - L(i, r + 1, m));
-        } else {
-            fb[m] = -dtdy * L(r, i - 1, m);
-            fb[5 + m] = dtdy * L(r, i, m);
-            fb[10 + m] = dtdx * (L(r - 1, i - 1, m) - L(r, i - 1, m));
-            fb[15 + m] = dtdx * (L(r, i - 1, m) - L(r + 1, i - 1, m));
-            fb[20 + m] = dtdx * (L(r - 1, i, m) - L(r, i, m));
-            fb[25 + m] = dtdx * (L(r, i, m) - L(r + 1, i, m));
-        }
+        // wave slots of the three interfaces: own from 3, left from 15, right from 27
+        const int o = f == 0 ? 0 : f == 1 ? 5 : 7;
+        auto put = [&](int base, const double* v) {
+            double* d = dst + (size_t)(base + o) * npl + oi;
+            d[0] = v[0];
+            d[npl] = v[cn];
+            if (f != 1) {
+                d[2 * npl] = v[ct];
+                d[3 * npl] = v[3];
+                d[4 * npl] = v[4];
+            }
+        };
+        dst[(size_t)f * npl + oi] = sb;
+        put(3, Wb);
+        put(15, Wmb);
+        put(27, Wpb);
     }
 }
 
@@ -1852,7 +1851,7 @@ DC_HD void stage_b4_b(const dclaw_params& P, const Geom& g, const double* __rest
 // stages' slots (gathers, no atomics), so each is one data-parallel launch.
 namespace dclaw {
 
-constexpr int NFB = 47;  // FluxB: self 15, left 12, right 12, a2l 4, a2r 4
+constexpr int NFB = 47;  // stage_flux_b: self 15, left 12, right 12, a2l 4, a2r 4
 constexpr int NCB = 16;  // CellB of both sides: q[5], fs, taudir; then the beds of L and R
 constexpr int NTD = 14;  // taudir reverse: qb[5], neighbour depths[4], beds of the cell and L, R, B, T
 constexpr int NQSB = 6;  // per padded cell: its source cell's q adjoint (5), its bed's adjoint
@@ -1915,19 +1914,7 @@ DC_HD void adj_item_src2(const dclaw_params& P, const Geom& g, const Work& W, co
 template <int DIR>
 DC_HD void adj_item_flux(const dclaw_params& P, const Geom& g, const Work& W, const AdjWork& A, int r, int i,
                          double dt) {
-    double fb[30];
-    flux_bar<DIR>(g, A.lamq, r, i, dt, fb);
-    FluxB o;
-    const double dtdx = DIR == 0 ? dt / g.dx : dt / g.dy;
-    stage_flux_b<DIR>(P, g, W, r, i, dtdx, fb, o);
-    double* dst = DIR == 0 ? A.xfb : A.yfb;
-    const size_t np = DIR == 0 ? W.nxi : W.nyi;
-    const size_t oi = DIR == 0 ? xidx(g, r, i) : yidx(g, i, r);
-    for (int k = 0; k < NW; ++k) dst[(size_t)k * np + oi] = o.self[k];
-    for (int k = 0; k < 12; ++k) dst[(size_t)(15 + k) * np + oi] = o.left[k];
-    for (int k = 0; k < 12; ++k) dst[(size_t)(27 + k) * np + oi] = o.right[k];
-    for (int k = 0; k < 4; ++k) dst[(size_t)(39 + k) * np + oi] = o.a2l[k];
-    for (int k = 0; k < 4; ++k) dst[(size_t)(43 + k) * np + oi] = o.a2r[k];
+    stage_flux_b<DIR>(P, g, W, A.lamq, r, i, dt, DIR == 0 ? A.xfb : A.yfb, DIR == 0 ? W.nxi : W.nyi);
 }
 
 template <int DIR>
