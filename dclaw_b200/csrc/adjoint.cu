@@ -206,7 +206,7 @@ __device__ __forceinline__ void block_item(const BatchArgs& a, int m, const dcla
         if (OP == OP_FW_B4) {
             if (stage_b4(P, g, q_in, a.b + M.b_off, W, ci, cj) && a.status) atomicCAS(a.status + m, 0, DCLAW_ERR_NAN);
         } else if (OP == OP_FW_TAUDIR) {
-            stage_taudir(P, g, W, ci, cj);
+            adj_item_taudir_fw(P, g, W, ci, cj);
         } else if (OP == OP_FW_SVREC) {
             adj_item_svrec(P, g, W, A, ci, cj);
         } else if (OP == OP_RV_TAUDIR) {

@@ -920,13 +920,17 @@ DC_HD void load_side_b_sv(const dclaw_params& P, const Work& W, const double* __
     const size_t np = W.npad;
     const double tb = sb.tau_sv;
     const int kn = comp_n == 1 ? SV_DU : SV_DV, kt = comp_n == 1 ? SV_DV : SV_DU;
-    double hb = sb.h + tb * r[SV_DH * np];
-    double unb = sb.un + tb * r[(size_t)kn * np];
-    double utb = sb.ut + tb * r[(size_t)kt * np];
-    double mb = sb.m + (tb * r[SV_DM * np] + sb.rho_sv * (P.rho_s - P.rho_f));
-    double pb = sb.p + tb * r[SV_DP * np];
-    pbar[PB_PHI] += tb * r[SV_DPHI * np];
-    pbar[PB_MU] += tb * r[SV_DMU * np];
+    // (a moving side has no record and no tau adjoint)
+    double hb = sb.h, unb = sb.un, utb = sb.ut, mb = sb.m + sb.rho_sv * (P.rho_s - P.rho_f), pb = sb.p;
+    if (tb != 0.0) {
+        hb += tb * r[SV_DH * np];
+        unb += tb * r[(size_t)kn * np];
+        utb += tb * r[(size_t)kt * np];
+        mb += tb * r[SV_DM * np];
+        pb += tb * r[SV_DP * np];
+        pbar[PB_PHI] += tb * r[SV_DPHI * np];
+        pbar[PB_MU] += tb * r[SV_DMU * np];
+    }
     double hnb = sb.hn + unb / h, htb = sb.ht + utb / h;
     hb -= unb * un / h + utb * ut / h;
     double hmb = sb.hm;
@@ -949,6 +953,7 @@ DC_HD void svrec_cell(const dclaw_params& P, const Work& W, double* __restrict__
     const double h = W.qB[pi];
     if (h <= P.dry_tolerance) return;  // dry sides never read their record
     const double u = W.qB[np + pi] / h, v = W.qB[2 * np + pi] / h;
+    if (moves(u, v)) return;           // nor moving ones
     double hm = W.qB[3 * np + pi], p = W.qB[4 * np + pi], m;
     for (int a = 0; a < 2; ++a) {
         qfix_mp(P, h, hm, p, m, P.grav);
@@ -1634,6 +1639,8 @@ DC_HD bool src2_cell_b(const dclaw_params& P, double phi, double dt, const doubl
 DC_HD void stage_taudir_b(const dclaw_params& P, const Geom& g, const Work& W, int i, int j, const double tdb[3],
                           double qb[5], double nb[4], double* pbar, double bedb[5]) {
     if (i < 0 || j < 0 || i > g.mx + 1 || j > g.my + 1) return;
+    // every adjoint below is a multiple of these: zeros at all but cells at rest
+    if (tdb[0] == 0.0 && tdb[1] == 0.0 && tdb[2] == 0.0) return;
     const size_t pi = pidx(g, i, j);
     const double dry = P.dry_tolerance;
     const double gz = P.grav;
@@ -1890,6 +1897,17 @@ constexpr int ACT_TILE = 16, ACT_REACH = 4;
 DC_HD bool adj_active(const AdjWork& A, int i, int j) {
     if (!A.act) return true;
     return A.act[((j + 1) / ACT_TILE) * A.act_nx + (i + 1) / ACT_TILE] != 0u;
+}
+
+// padded cell (i, j), i in -1..mx+2, j in -1..my+2: calc_taudir for the
+// solver (a moving cell's outputs are not read)
+DC_HD void adj_item_taudir_fw(const dclaw_params& P, const Geom& g, const Work& W, int i, int j) {
+    const size_t pi = pidx(g, i, j);
+    if (cell_moves(P, W.qB, W.npad, pi)) {
+        for (int k = 0; k < 3; ++k) W.td[(size_t)k * W.npad + pi] = 0.0;
+        return;
+    }
+    stage_taudir(P, g, W, i, j);
 }
 
 // padded cell (i, j), i in -1..mx+2, j in -1..my+2: setvars records

@@ -201,7 +201,7 @@ DC_HD Side full_load_side(const dclaw_params& P, const WorkF& W, size_t pi, int 
     s.un = hn / h;
     s.ut = ht / h;
     s.rho_sv = m * (P.rho_s - P.rho_f) + P.rho_f;
-    s.tau_sv = full_tau(W)[(twice ? W.npad : 0) + pi];
+    s.tau_sv = moves(s.un, s.ut) ? 0.0 : full_tau(W)[(twice ? W.npad : 0) + pi];
     return s;
 }
 

@@ -257,6 +257,13 @@ DC_HD void zero_waves(Waves& w) {
     w.w5h = w.w5n = w.w5t = w.w5m = w.w5p = 0.0;
 }
 
+// Whether a cell of velocity (u, v) moves. The solver reads tau, the static-
+// friction direction and the factor of safety of its sides only where
+// neither does (vnorm2 in riemann_solve, at least this sum): the step's own
+// stages leave them out, setvars and calc_taudir with them, for every cell
+// that moves.
+DC_HD bool moves(double u, double v) { return sq(u) + sq(v) > 0.0; }
+
 // Side state handed to the solver (after the two rpn2 qfix passes).
 struct Side {
     double h, hn, ht, hm, p;  // conserved, normal/tangential momentum

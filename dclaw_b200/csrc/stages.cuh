@@ -104,9 +104,9 @@ DC_HD bool stage_b4(const dclaw_params& P, const Geom& g, const double* __restri
 }
 
 // ---------------------------------------------------------------------------
-// tau of a wet cell's two rpn2 states, once per cell instead of once per
-// interface side (setvars, with its atan, tan and tanh, is over half of an
-// interface's work when both sides evaluate it): plane 0 after one qfix pass
+// tau of a wet cell's two rpn2 states, where the solver reads it (moves), once
+// per cell instead of once per interface side (setvars, with its atan, tan and
+// tanh, is over half of an interface's work when both sides evaluate it): plane 0 after one qfix pass
 // (A1), plane 1 after two (A2). setvars reads the velocity only through
 // u^2 + v^2, so one value serves both sweep directions.
 // put_taus: from the state after the first pass and its tau1.
@@ -118,14 +118,22 @@ DC_HD void put_taus(const dclaw_params& P, double h, double u, double v, double 
     tau[npad + pi] = m == m1 && p == p1 ? tau1 : setvars<false>(P, P.phi, h, u, v, m, p, P.grav).tau;
 }
 
-// cell_taus: from the b4step2 state's padded planes; a dry cell has none
+// cell_taus: from the b4step2 state's padded planes; a dry cell has none, and
+// a moving one's are not read
 DC_HD void cell_taus(const dclaw_params& P, const double* __restrict__ qB, size_t npad, size_t pi, double* tau) {
     const double h = qB[pi];
     if (h <= P.dry_tolerance) return;
     double hm = qB[3 * npad + pi], p = qB[4 * npad + pi], m;
     qfix_mp(P, h, hm, p, m, P.grav);
     const double u = qB[npad + pi] / h, v = qB[2 * npad + pi] / h;
+    if (moves(u, v)) return;
     put_taus(P, h, u, v, hm, p, m, setvars<false>(P, P.phi, h, u, v, m, p, P.grav).tau, npad, pi, tau);
+}
+
+// a cell of the b4step2 state that is wet and moves
+DC_HD bool cell_moves(const dclaw_params& P, const double* __restrict__ qB, size_t npad, size_t pi) {
+    const double h = qB[pi];
+    return h > P.dry_tolerance && moves(qB[npad + pi] / h, qB[2 * npad + pi] / h);
 }
 
 // ---------------------------------------------------------------------------
@@ -136,7 +144,8 @@ DC_HD void cell_taus(const dclaw_params& P, const double* __restrict__ qB, size_
 // three output planes, bed(pi) the bed of padded cell pi (the bed less the
 // bed change on the full state: digclaw_module.f90:555-613). tau (nullable):
 // two planes that receive tau of the cell's rpn2 states where it is wet
-// (cell_taus).
+// (cell_taus); the outputs are then for the solver alone, and a moving cell's
+// are zeros.
 template <typename Bed>
 DC_HD void taudir_cell(const dclaw_params& P, const Geom& g, const double* __restrict__ qB, size_t npad,
                        double* td, Bed bed, int i, int j, double* tau = nullptr) {
@@ -147,6 +156,10 @@ DC_HD void taudir_cell(const dclaw_params& P, const Geom& g, const double* __res
     if (i < 0 || j < 0 || i > g.mx + 1 || j > g.my + 1) {
         fs[pi] = 0.0; tx[pi] = 0.0; ty[pi] = 0.0;
         if (tau) cell_taus(P, qB, npad, pi, tau);
+        return;
+    }
+    if (tau && cell_moves(P, qB, npad, pi)) {
+        fs[pi] = 0.0; tx[pi] = 0.0; ty[pi] = 0.0;
         return;
     }
     const double dry = P.dry_tolerance;
@@ -256,7 +269,8 @@ DC_HD Side load_side(const dclaw_params& P, const Work& W, size_t pi, int comp_n
 // twice) of a wet padded cell, SV_N planes per state (padded layout): tau and
 // its partial derivatives in (h, u, v, m, p, phi, mu), u = hu/h, v = hv/h.
 // setvars reads the velocity only through u^2 + v^2, so the record serves
-// both sweep directions. Written by the adjoint's record stage.
+// both sweep directions. Written by the adjoint's record stage, for cells that
+// do not move (moves).
 constexpr int SV_N = 8;
 constexpr int NSV = 2 * SV_N;
 enum { SV_TAU = 0, SV_DH, SV_DU, SV_DV, SV_DM, SV_DP, SV_DPHI, SV_DMU };
@@ -288,7 +302,7 @@ DC_HD Side load_side_sv(const dclaw_params& P, const Work& W, const double* __re
     s.un = hn / h;
     s.ut = ht / h;
     s.rho_sv = m * (P.rho_s - P.rho_f) + P.rho_f;
-    s.tau_sv = sv[(size_t)(twice ? second : 0) * W.npad + pi];
+    s.tau_sv = moves(s.un, s.ut) ? 0.0 : sv[(size_t)(twice ? second : 0) * W.npad + pi];
     return s;
 }
 

@@ -113,17 +113,13 @@ DC_HD bool cell_record(const dclaw_params& P, const Geom& g, const double* __res
     R.put(R_H, pi, h);
     double fs = 0.0, tdx = 0.0, tdy = 0.0;
     double tau1 = 0.0, rho1 = 0.0;
+    const bool moving = wet && moves(uq, vq);
     if (wet) {
         double m1 = fmin2(fmax2(hm / h, 0.0), 1.0);
         double hm1 = h * m1;
         double p1 = clip_p(P, h, m1, p);
         double m2 = fmin2(fmax2(hm1 / h, 0.0), 1.0);
         double p2 = clip_p(P, h, m2, p1);
-        SetVars s1 = setvars<false>(P, P.phi, h, uq, vq, m1, p1, P.grav);
-        tau1 = s1.tau;
-        rho1 = s1.rho;
-        double tau2 = s1.tau;
-        if (!(m2 == m1 && p2 == p1)) tau2 = setvars<false>(P, P.phi, h, uq, vq, m2, p2, P.grav).tau;
         R.put(R_HU, pi, hu);
         R.put(R_HV, pi, hv);
         R.put(R_HM, pi, hm);
@@ -132,6 +128,12 @@ DC_HD bool cell_record(const dclaw_params& P, const Geom& g, const double* __res
         R.put(R_VQ, pi, vq);
         R.put(R_M1, pi, m1);
         R.put(R_M2, pi, m2);
+        if (moving) return nan;  // rec_side reads no more of it
+        SetVars s1 = setvars<false>(P, P.phi, h, uq, vq, m1, p1, P.grav);
+        tau1 = s1.tau;
+        rho1 = s1.rho;
+        double tau2 = s1.tau;
+        if (!(m2 == m1 && p2 == p1)) tau2 = setvars<false>(P, P.phi, h, uq, vq, m2, p2, P.grav).tau;
         R.put(R_TAU1, pi, tau1);
         R.put(R_TAU2, pi, tau2);
     }
@@ -262,27 +264,25 @@ DC_HD Side rec_side(const dclaw_params& P, const Rec& R, const Geom& g, const Ti
     const size_t pi = pidx(g, i, j);
     Side s;
     s.b = M.bed(i, j);
-    s.fs = R.get(R_FS, pi);
-    s.taudir = R.get(dir == 0 ? R_TDX : R_TDY, pi);
     double h = M.h(i, j);
     if (h <= P.dry_tolerance) {
         s.h = 0.0; s.hn = 0.0; s.ht = 0.0; s.hm = 0.0; s.p = 0.0;
         s.un = 0.0; s.ut = 0.0; s.m = 0.0; s.rho_sv = 0.0; s.tau_sv = 0.0;
+        s.fs = R.get(R_FS, pi);
+        s.taudir = R.get(dir == 0 ? R_TDX : R_TDY, pi);
         return s;
     }
     double hu = R.get(R_HU, pi), hv = R.get(R_HV, pi);
     double uq = R.get(R_UQ, pi), vq = R.get(R_VQ, pi);
     double m1 = R.get(R_M1, pi);
     double p1 = clip_p(P, h, m1, R.get(R_P, pi));
-    double m, p, tau;
+    double m, p;
     if (twice) {
         m = R.get(R_M2, pi);
         p = clip_p(P, h, m, p1);
-        tau = R.get(R_TAU2, pi);
     } else {
         m = m1;
         p = p1;
-        tau = R.get(R_TAU1, pi);
     }
     s.h = h;
     s.hn = dir == 0 ? hu : hv;
@@ -293,7 +293,13 @@ DC_HD Side rec_side(const dclaw_params& P, const Rec& R, const Geom& g, const Ti
     s.hm = h * m;
     s.p = p;
     s.rho_sv = m * (P.rho_s - P.rho_f) + P.rho_f;
-    s.tau_sv = tau;
+    if (moves(uq, vq)) {
+        s.fs = s.taudir = s.tau_sv = 0.0;
+    } else {
+        s.fs = R.get(R_FS, pi);
+        s.taudir = R.get(dir == 0 ? R_TDX : R_TDY, pi);
+        s.tau_sv = R.get(twice ? R_TAU2 : R_TAU1, pi);
+    }
     return s;
 }
 
