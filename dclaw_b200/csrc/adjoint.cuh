@@ -49,13 +49,12 @@ DC_HD void qfix_b(const dclaw_params& P, double h, double hu, double hv, double 
     m_b += hmb * h;
     double m1b = (m1 < 1.0) ? m_b : 0.0;
     double m0b = (m0 > 0.0) ? m1b : 0.0;
-    double hm_b = m0b / h;
-    h_b -= m0b * m0 / h;
-    double hu_b = hub + ub / h;
-    h_b -= ub * u / h;
-    double hv_b = hvb + vb / h;
-    h_b -= vb * v / h;
-    hb = h_b; hub = hu_b; hvb = hv_b; hmb = hm_b; pb = pin_b;
+    // x / h: its adjoint over h serves numerator and denominator
+    const double mh = m0b / h, uh = ub / h, vh = vb / h;
+    h_b -= mh * m0;
+    h_b -= uh * u;
+    h_b -= vh * v;
+    hb = h_b; hub = hub + uh; hvb = hvb + vh; hmb = mh; pb = pin_b;
 }
 
 // qfix_mp on a wet cell: inputs (h, hm, p); hmb, pb hold adjoints of the
@@ -78,9 +77,8 @@ DC_HD void qfix_mp_b(const dclaw_params& P, double h, double hm, double p, doubl
     m_b += hmb * h;
     double m1b = (m1 < 1.0) ? m_b : 0.0;
     double m0b = (m0 > 0.0) ? m1b : 0.0;
-    double hm_b = m0b / h;
-    hb -= m0b * m0 / h;
-    hmb = hm_b;
+    hmb = m0b / h;
+    hb -= hmb * m0;
     pb = pin_b;
 }
 
@@ -111,8 +109,9 @@ DC_HD void qfix_cmass_b(const dclaw_params& P, double m, double p_exc, double u,
     rhohb += pe_maxb * gz;
     h_b += -pe_maxb * P.rho_f * gz - pe_minb * P.rho_f * gz;
     // h = rhoh / rho
-    rhohb += h_b / rho;
-    double rho_b = rhob - h_b * h / rho;
+    const double hr = h_b / rho;
+    rhohb += hr;
+    double rho_b = rhob - hr * h;
     m2b += rho_b * (P.rho_s - P.rho_f);
     double m1b = (m1 < 1.0) ? m2b : 0.0;
     mb = (m > 0.0) ? m1b : 0.0;
@@ -149,26 +148,29 @@ DC_HD void setvars_b(const dclaw_params& P, double phi, double h, double u, doub
         m_eq = P.m_crit * (sNd / (sNd + sNn));
     }
     double x = P.c1 * (m - m_eq);
-    double t = em::d_tan(phi + em::d_atan(x));
-    double tau0 = sig_eff * t;
-    double th = em::d_tanh(100.0 * (m - 0.1));
     // reverse
     double rho_b = ob.rho;
-    double m_b = 0.0, h_b = 0.0;
-    double tau0b = ob.tau * 0.5 * (1.0 + th);
-    double thb = ob.tau * tau0 * 0.5;
-    m_b += thb * (1.0 - th * th) * 100.0;
-    double sig_effb = tau0b * t;
-    double argb = tau0b * sig_eff * (1.0 + t * t);
-    phib += argb;
-    double xb = ob.tanpsi + argb / (1.0 + x * x);
+    double m_b = 0.0, h_b = 0.0, sig_effb = 0.0, xb = ob.tanpsi;
+    if (ob.tau != 0.0) {
+        double t = em::d_tan(phi + em::d_atan(x));
+        double tau0 = sig_eff * t;
+        double th = em::d_tanh(100.0 * (m - 0.1));
+        double tau0b = ob.tau * 0.5 * (1.0 + th);
+        double thb = ob.tau * tau0 * 0.5;
+        m_b += thb * (1.0 - th * th) * 100.0;
+        sig_effb += tau0b * t;
+        double argb = tau0b * sig_eff * (1.0 + t * t);
+        phib += argb;
+        xb += argb / (1.0 + x * x);
+    }
     m_b += xb * P.c1;
     double m_eqb = ob.m_eq - xb * P.c1;
     double shearb = 0.0;
     if (Nnum > 0.0) {
         double D = sNd + sNn;
-        double sNdb = m_eqb * P.m_crit * sNn / (D * D);
-        double sNnb = -m_eqb * P.m_crit * sNd / (D * D);
+        const double w = m_eqb * P.m_crit / (D * D);
+        double sNdb = w * sNn;
+        double sNnb = -w * sNd;
         double Ndenb = dsqrt_b(sNd, sNdb);
         double Nnumb = dsqrt_b(sNn, sNnb);
         pbar[PB_MU] += Nnumb * shear;
@@ -177,11 +179,12 @@ DC_HD void setvars_b(const dclaw_params& P, double phi, double h, double u, doub
         sig_effb += Ndenb;
     }
     if (h > P.dry_tolerance) {
-        double vnormb = shearb * 2.0 / h;
-        h_b -= shearb * shear / h;
+        const double sh = shearb / h;
+        h_b -= sh * shear;
         if (vnorm > 0.0) {
-            ub += vnormb * u / vnorm;
-            vb += vnormb * v / vnorm;
+            const double w = sh * 2.0 / vnorm;
+            ub += w * u;
+            vb += w * v;
         }
     }
     double alphainvb = ob.alphainv;
@@ -211,8 +214,9 @@ DC_HD void setvars_b(const dclaw_params& P, double phi, double h, double u, doub
 
 // ---------------------------------------------------------------------------
 // riemanntype: adjoints of (hm, s1m, s2m) to (hL, hR, uL, uR), accumulated.
-DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double drytol, double g, double hmb,
-                         double s1mb, double s2mb, double& hLb, double& hRb, double& uLb, double& uRb) {
+// cL = sqrt(g hL), cR = sqrt(g hR).
+DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double cL, double cR, double drytol, double g,
+                         double hmb, double s1mb, double s2mb, double& hLb, double& hRb, double& uLb, double& uRb) {
     double h_min = fmin2(hR, hL);
     double h_max = fmax2(hR, hL);
     double delu = uR - uL;
@@ -221,14 +225,13 @@ DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double dryt
         double sb = s1mb + s2mb;
         uRb += sb;
         uLb += sb;
-        double cR = sqrt(g * hR), cL = sqrt(g * hL);
         hRb += -2.0 * g * dsqrt_b(cR, sb);
         hLb += 2.0 * g * dsqrt_b(cL, sb);
         return;
     }
-    double F_min = delu + 2.0 * (sqrt(g * h_min) - sqrt(g * h_max));
+    const double c_min = hR < hL ? cR : cL, c_max = hR > hL ? cR : cL;
+    double F_min = delu + 2.0 * (c_min - c_max);
     double F_max = delu + (h_max - h_min) * (sqrt(.5 * g * (h_max + h_min) / (h_max * h_min)));
-    double cL = sqrt(g * hL), cR = sqrt(g * hR);
     if (F_min > 0.0) {
         double X = -delu + 2.0 * (cL + cR);
         double Y = fmax2(0.0, X);
@@ -290,11 +293,12 @@ DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double dryt
         double gLb = dfdhb, gRb = dfdhb;
         double T1b = -dfdhb, T2b = -dfdhb;
         // T = g (H - hX) / (4 H^2 gX)
-        Hb += T1b * (g / (4.0 * H * H * gL)) * (1.0 - 2.0 * (H - hL) / H);
-        hLb += T1b * (-g / (4.0 * H * H * gL));
+        const double eL = g / (4.0 * H * H * gL), eR = g / (4.0 * H * H * gR);
+        Hb += T1b * eL * (1.0 - 2.0 * (H - hL) / H);
+        hLb -= T1b * eL;
         gLb += T1b * (-T1 / gL);
-        Hb += T2b * (g / (4.0 * H * H * gR)) * (1.0 - 2.0 * (H - hR) / H);
-        hRb += T2b * (-g / (4.0 * H * H * gR));
+        Hb += T2b * eR * (1.0 - 2.0 * (H - hR) / H);
+        hRb -= T2b * eR;
         gRb += T2b * (-T2 / gR);
         // F0
         delub += F0b;
@@ -310,7 +314,7 @@ DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double dryt
         if (hR > hL) hRb += Hb; else hLb += Hb;
     } else {
         // one secant step from h_min: F0 = delu + 2 (sqrt(g h_min) - sqrt(g h_max)) + 0
-        double sgmin = sqrt(g * h_min), sgmax = sqrt(g * h_max);
+        const double sgmin = c_min, sgmax = c_max;
         double F0 = delu + 2.0 * (sgmin - sgmax);
         double dh = h_max - h_min;
         double Q = sqrt(.5 * g * (h_max + h_min) / (h_max * h_min));
@@ -332,10 +336,10 @@ DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double dryt
         double hmt = hmb + g * dsqrt_b(sghm, sghmb);
         double hminb = hmt;
         double F0b = -hmt / slope;
-        double slopeb = hmt * F0 / (slope * slope);
+        double slopeb = -F0b * F0 / slope;
         double Fmaxb = slopeb / dh;
-        F0b -= slopeb / dh;
-        double dhb = -slopeb * slope / dh;
+        F0b -= Fmaxb;
+        double dhb = -Fmaxb * slope;
         // F_max = delu + dh * Q,  Q = sqrt(.5 g (hmax + hmin) / (hmax hmin))
         delub += Fmaxb;
         dhb += Fmaxb * Q;
@@ -343,8 +347,9 @@ DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double dryt
         double Xq = .5 * g * (h_max + h_min) / (h_max * h_min);
         double Xqb = dsqrt_b(Q, Qb);
         // Xq = .5 g (hmax + hmin) / (hmax hmin) = .5 g (1/hmin + 1/hmax)
-        double hmaxb = Xqb * (.5 * g / (h_max * h_min) - Xq / h_max);
-        hminb += Xqb * (.5 * g / (h_max * h_min) - Xq / h_min);
+        const double e = .5 * g / (h_max * h_min);
+        double hmaxb = Xqb * (e - Xq / h_max);
+        hminb += Xqb * (e - Xq / h_min);
         hmaxb += dhb;
         hminb -= dhb;
         delub += F0b;
@@ -355,6 +360,11 @@ DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double dryt
     }
     uRb += delub;
     uLb -= delub;
+}
+
+DC_HD void riemanntype_b(double hL, double hR, double uL, double uR, double drytol, double g, double hmb,
+                         double s1mb, double s2mb, double& hLb, double& hRb, double& uLb, double& uRb) {
+    riemanntype_b(hL, hR, uL, uR, sqrt(g * hL), sqrt(g * hR), drytol, g, hmb, s1mb, s2mb, hLb, hRb, uLb, uRb);
 }
 
 // ---------------------------------------------------------------------------
@@ -381,10 +391,13 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
     double hmL = L.hm, hmR = R.hm, pL = L.p, pR = R.p, bL = L.b, bR = R.b;
     double uL = L.un, uR = R.un, vL = L.ut, vR = R.ut, mL = L.m, mR = R.m;
     double rhoL_sv = L.rho_sv, tauL_sv = L.tau_sv, rhoR_sv = R.rho_sv, tauR_sv = R.tau_sv;
+    double cL = 0.0, cR = 0.0, sqhL = 0.0, sqhR = 0.0;
     if (hR <= drytol) {
         pre = 1;
         hR = 0.0; pR = 0.0; mR = mL;
-        RType t = riemanntype(hL, hL, uL, -uL, drytol, grav);
+        cL = sqrt(grav * hL);
+        sqhL = sqrt(hL);
+        RType t = riemanntype(hL, hL, uL, -uL, cL, cL, sqhL, sqhL, drytol, grav);
         double hstartest = fmax2(hL, t.hm);
         if (hstartest + bL < bR) {
             wall2 = 0.0; wall3 = 0.0;
@@ -392,11 +405,14 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
             hR = hL; huR = -huL; hvR = hvL; hmR = hmL; bR = bL;
             uR = -uL; vR = vL; mR = mL; pR = pL;
             rhoR_sv = rhoL_sv; tauR_sv = tauL_sv;
+            cR = cL; sqhR = sqhL;
         }
     } else if (hL <= drytol) {
         pre = 2;
         hL = 0.0; pL = 0.0; mL = mR;
-        RType t = riemanntype(hR, hR, -uR, uR, drytol, grav);
+        cR = sqrt(grav * hR);
+        sqhR = sqrt(hR);
+        RType t = riemanntype(hR, hR, -uR, uR, cR, cR, sqhR, sqhR, drytol, grav);
         double hstartest = fmax2(hR, t.hm);
         if (hstartest + bR < bL) {
             wall1 = 0.0; wall2 = 0.0;
@@ -404,7 +420,13 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
             hL = hR; huL = -huR; hvL = hvR; hmL = hmR; mL = mR; bL = bR;
             uL = -uR; vL = vR; pL = pR;
             rhoL_sv = rhoR_sv; tauL_sv = tauR_sv;
+            cL = cR; sqhL = sqhR;
         }
+    } else {
+        cL = sqrt(grav * hL);
+        cR = sqrt(grav * hR);
+        sqhL = sqrt(hL);
+        sqhR = sqrt(hR);
     }
     const double criticaltol = fmax2(drytol * grav, 1e-6);
     const double criticaltol_2 = sqrt(criticaltol);
@@ -433,8 +455,6 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
         gammaR = 0.25 * (P.rho_f + 3.0 * rhoR) / rhoR;
     }
     const double geps = gz;
-    double sqhL = sqrt(hL), sqhR = sqrt(hR);
-    double cL = sqrt(geps * hL), cR = sqrt(geps * hR);
     double sL = uL - cL, sR = uR + cR;
     double Du = sqhR + sqhL;
     double uhat = (sqhL * uL + sqhR * uR) / Du;
@@ -443,7 +463,7 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
     double sE1 = fmin2(sL, sRoe1);
     double sE2 = fmax2(sR, sRoe2);
     double u = uhat;
-    RType rt = riemanntype(hL, hR, uL, uR, drytol, geps);
+    RType rt = riemanntype(hL, hR, uL, uR, cL, cR, sqhL, sqhR, drytol, geps);
     double sw1 = fmin2(sE1, rt.s2m);
     double sw3 = fmax2(sE2, rt.s1m);
     double Dd = sE2 - sE1;
@@ -520,13 +540,13 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
     double del1 = huR - huL;
     double del2a = hR * sq(uR) + 0.5 * 1.0 * gz * sq(hR) - (hL * sq(uL) + 0.5 * 1.0 * gz * sq(hL));
     double grg = gamma * rho * gz;
-    double vnorm = sqrt(sq(uR) + sq(uL) + sq(vR) + sq(vL));
+    double vnorm2 = sq(uR) + sq(uL) + sq(vR) + sq(vL);
     bool is_static = false;
     int tcase = 0;  // 0: moving (tausource 0), 1: static, 2: sign-matched friction
     double tdR = R.taudir;
     double tA = 0.0, tB = 0.0, ts0 = 0.0;
     double xs = del2a - source2dx;
-    if (vnorm > 0.0) {
+    if (vnorm2 > 0.0) {
         tcase = 0;
     } else {
         tA = tdR * tauR / rhoR;
@@ -600,8 +620,9 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
         del1b += del4b * grg;
         pRb += del4b * ui;
         pLb -= del4b * ui;
-        hustarb += uib / hstarHLL;
-        hstarb -= uib * ui / hstarHLL;
+        const double w = uib / hstarHLL;
+        hustarb += w;
+        hstarb -= w * ui;
     }
     huLb += hustarb;
     fw11b += hustarb;
@@ -636,14 +657,15 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
     double ab_ = 0.0, cb_ = 0.0, bbb_ = 0.0, del2b = 0.0;
     if (!rc) {
         // beta1 = (c del0 - del1)/D, beta3 = (del1 - a del0)/D, beta2 = a c del0 - (a+c) del1 + del2
-        cb_ += beta1b * (del0 - beta1) / D;
-        ab_ += beta1b * beta1 / D;
-        del0b += beta1b * c / D;
-        del1b -= beta1b / D;
-        ab_ += beta3b * (beta3 - del0) / D;
-        cb_ -= beta3b * beta3 / D;
-        del1b += beta3b / D;
-        del0b -= beta3b * a / D;
+        const double w1 = beta1b / D, w3 = beta3b / D;
+        cb_ += w1 * (del0 - beta1);
+        ab_ += w1 * beta1;
+        del0b += w1 * c;
+        del1b -= w1;
+        ab_ += w3 * (beta3 - del0);
+        cb_ -= w3 * beta3;
+        del1b += w3;
+        del0b -= w3 * a;
         ab_ += beta2b * (c * del0 - del1);
         cb_ += beta2b * (a * del0 - del1);
         del0b += beta2b * a * c;
@@ -726,30 +748,43 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
         const double dS = sE2 - sE1;
         if (dcase == 1) {
             // X1 = hstar dS / sE2, X2 = hstar dS / sE1
-            hstarb += X1b * dS / sE2;
-            sE2b += X1b * hstarHLL / sE2 - X1b * X1 / sE2;
-            sE1b -= X1b * hstarHLL / sE2;
-            hstarb += X2b * dS / sE1;
-            sE2b += X2b * hstarHLL / sE1;
-            sE1b += -X2b * hstarHLL / sE1 - X2b * X2 / sE1;
+            if (X1b != 0.0) {
+                const double w = X1b / sE2;
+                hstarb += w * dS;
+                sE2b += w * hstarHLL - w * X1;
+                sE1b -= w * hstarHLL;
+            }
+            if (X2b != 0.0) {
+                const double w = X2b / sE1;
+                hstarb += w * dS;
+                sE2b += w * hstarHLL;
+                sE1b += -w * hstarHLL - w * X2;
+            }
         } else if (dcase == 2) {
-            hstarb += X1b * dS / sE1;
-            sE2b += X1b * hstarHLL / sE1;
-            sE1b += -X1b * hstarHLL / sE1 - X1b * X1 / sE1;
+            if (X1b != 0.0) {
+                const double w = X1b / sE1;
+                hstarb += w * dS;
+                sE2b += w * hstarHLL;
+                sE1b += -w * hstarHLL - w * X1;
+            }
             hLb -= X2b;
         } else {
             hRb += X1b;
-            hstarb += X2b * dS / sE2;
-            sE2b += X2b * hstarHLL / sE2 - X2b * X2 / sE2;
-            sE1b -= X2b * hstarHLL / sE2;
+            if (X2b != 0.0) {
+                const double w = X2b / sE2;
+                hstarb += w * dS;
+                sE2b += w * hstarHLL - w * X2;
+                sE1b -= w * hstarHLL;
+            }
         }
     }
     if (sonic) {
         delbb -= d0b;
     } else {
-        delbb += d0b * gz * hbar / s1s2bar;
-        hbarb += d0b * delb * gz / s1s2bar;
-        s1s2barb -= d0b * d0 / s1s2bar;
+        const double w = d0b / s1s2bar;
+        delbb += w * gz * hbar;
+        hbarb += w * delb * gz;
+        s1s2barb -= w * d0;
     }
     // source2dx
     if (u0) {
@@ -768,10 +803,11 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
             hbarb += x0b * (-gz) * delb;
             delbb += x0b * (-gz) * hbar;
         } else {
-            hbarb += x0b * (-gz * delb * s1s2tilde) / s1s2bar;
-            delbb += x0b * (-gz * hbar * s1s2tilde) / s1s2bar;
-            s1s2tildeb += x0b * (-gz * hbar * delb) / s1s2bar;
-            s1s2barb -= x0b * x0 / s1s2bar;
+            const double w = x0b / s1s2bar;
+            hbarb += w * (-gz * delb * s1s2tilde);
+            delbb += w * (-gz * hbar * s1s2tilde);
+            s1s2tildeb += w * (-gz * hbar * delb);
+            s1s2barb -= w * x0;
         }
     }
     // s1s2tilde, s1s2bar, hbar, delb
@@ -789,13 +825,13 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
     bLb -= delbb;
     // hstarHLL = max(Qh, 0)
     if (Qh > 0.0) {
-        double Qb = hstarb;
-        huLb += Qb / Dd;
-        huRb -= Qb / Dd;
-        sE2b += Qb * hR / Dd - Qb * Qh / Dd;
-        hRb += Qb * sE2 / Dd;
-        sE1b += -Qb * hL / Dd + Qb * Qh / Dd;
-        hLb -= Qb * sE1 / Dd;
+        const double w = hstarb / Dd;
+        huLb += w;
+        huRb -= w;
+        sE2b += w * hR - w * Qh;
+        hRb += w * sE2;
+        sE1b += -w * hL + w * Qh;
+        hLb -= w * sE1;
     }
     // sw2, sw3, sw1
     double s1mb = 0.0, s2mb = 0.0;
@@ -812,7 +848,7 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
     }
     if (sE2 > rt.s1m) sE2b += sw3b; else s1mb += sw3b;
     if (sE1 < rt.s2m) sE1b += sw1b; else s2mb += sw1b;
-    riemanntype_b(hL, hR, uL, uR, drytol, geps, 0.0, s1mb, s2mb, hLb, hRb, uLb, uRb);
+    riemanntype_b(hL, hR, uL, uR, cL, cR, drytol, geps, 0.0, s1mb, s2mb, hLb, hRb, uLb, uRb);
     // sE1 = min(sL, sRoe1), sE2 = max(sR, sRoe2)
     double sLb = 0, sRb = 0, sRoe1b = 0, sRoe2b = 0;
     if (sL < sRoe1) sLb += sE1b; else sRoe1b += sE1b;
@@ -822,9 +858,10 @@ DC_HD bool riemann_solve_b(const dclaw_params& P, const Side& L, const Side& R, 
     double tch = dsqrt_b(chat, chatb);
     hRb += tch * geps * 0.5;
     hLb += tch * geps * 0.5;
-    double sqhLb = uhatb * (uL - uhat) / Du, sqhRb = uhatb * (uR - uhat) / Du;
-    uLb += uhatb * sqhL / Du;
-    uRb += uhatb * sqhR / Du;
+    const double uw = uhatb / Du;
+    double sqhLb = uw * (uL - uhat), sqhRb = uw * (uR - uhat);
+    uLb += uw * sqhL;
+    uRb += uw * sqhR;
     uLb += sLb;
     double cLb = -sLb;
     uRb += sRb;
@@ -931,8 +968,9 @@ DC_HD void load_side_b_sv(const dclaw_params& P, const Work& W, const double* __
         pbar[PB_PHI] += tb * r[SV_DPHI * np];
         pbar[PB_MU] += tb * r[SV_DMU * np];
     }
-    double hnb = sb.hn + unb / h, htb = sb.ht + utb / h;
-    hb -= unb * un / h + utb * ut / h;
+    const double unh = unb / h, uth = utb / h;
+    double hnb = sb.hn + unh, htb = sb.ht + uth;
+    hb -= unh * un + uth * ut;
     double hmb = sb.hm;
     if (twice) {
         qfix_mp_b(P, h, hm1, p1, P.grav, hb, hmb, pb, mb);
@@ -1112,17 +1150,18 @@ DC_HD void rpt2_split_b(const dclaw_params& P, double h, double hn, double ht, d
     }
     wave(s3, beta3, s3b, b3b);
     // betas
-    s3b += b1b * (d1 - beta1) / Dn;
-    s1b += b1b * beta1 / Dn;
-    asdqb[0] += b1b * s3 / Dn;
-    asdqb[2] -= b1b / Dn;
+    const double w1 = b1b / Dn, w3 = b3b / Dn;
+    s3b += w1 * (d1 - beta1);
+    s1b += w1 * beta1;
+    asdqb[0] += w1 * s3;
+    asdqb[2] -= w1;
     ub -= b2b * d1;
     asdqb[0] -= b2b * u;
     asdqb[1] += b2b;
-    s1b += b3b * (beta3 - d1) / Dn;
-    s3b -= b3b * beta3 / Dn;
-    asdqb[2] += b3b / Dn;
-    asdqb[0] -= b3b * s1 / Dn;
+    s1b += w3 * (beta3 - d1);
+    s3b -= w3 * beta3;
+    asdqb[2] += w3;
+    asdqb[0] -= w3 * s1;
     vb += s1b + s2b + s3b;
     double sghb = -s1b + s3b;
     double hb = g * dsqrt_b(sgh, sghb);
@@ -1131,10 +1170,11 @@ DC_HD void rpt2_split_b(const dclaw_params& P, double h, double hn, double ht, d
     if (P.src2method == -1) rhob -= gammab * gamma / rho;
     else rhob -= gammab * 0.25 * P.rho_f / (rho * rho);
     mb += rhob * (P.rho_s - P.rho_f);
-    xb[1] += ub / h;
-    xb[2] += vb / h;
-    xb[3] += mb / h;
-    hb -= (ub * u + vb * v + mb * m) / h;
+    const double uh = ub / h, vh = vb / h, mh = mb / h;
+    xb[1] += uh;
+    xb[2] += vh;
+    xb[3] += mh;
+    hb -= uh * u + vh * v + mh * m;
     xb[0] += hb;
 }
 
@@ -1414,9 +1454,10 @@ DC_HD void mp_update_relax_b(const dclaw_params& P, double phi, double dt, doubl
     double Db = argb * (-dt * rf / rhoh);
     rhohb -= argb * arg2 / rhoh;
     // krate2 = D (rho4 - rf) / rhoh
-    Db += krate2b * (rho4 - rf) / rhoh;
-    double rho4b = krate2b * D / rhoh;
-    rhohb -= krate2b * krate2 / rhoh;
+    const double kr = krate2b / rhoh;
+    Db += kr * (rho4 - rf);
+    double rho4b = kr * D;
+    rhohb -= kr * krate2;
     // D = -2 (kperm / (mu h4)) pex4
     double kpermb = Db * (-2.0 * pex4 / (P.mu * h4));
     double pex4b = Db * (-2.0 * (sv.kperm / (P.mu * h4)));
@@ -1457,16 +1498,17 @@ DC_HD void mp_update_relax_b(const dclaw_params& P, double phi, double dt, doubl
         double pAb = qpb;
         double T = dt * 3.0 * vnorm * sv.tanpsi * sv.alphainv;
         double Tb = -pAb / h;
-        double hbb = qhb + pAb * T / (h * h);
+        double hbb = qhb - Tb * T / h;
         double vnormb = Tb * dt * 3.0 * sv.tanpsi * sv.alphainv;
         double tanpsib = Tb * dt * 3.0 * vnorm * sv.alphainv;
         alphainvb += Tb * dt * 3.0 * vnorm * sv.tanpsi;
         // vnorm = nrm / h
         double nrmb = vnormb / h;
-        hbb -= vnormb * vnorm / h;
+        hbb -= nrmb * vnorm;
         if (nrm > 0.0) {
-            qhub += nrmb * hu / nrm;
-            qhvb += nrmb * hv / nrm;
+            const double w = nrmb / nrm;
+            qhub += w * hu;
+            qhvb += w * hv;
         }
         // hu = h u, hv = h v, hm = h m
         double u_b = qhub * h, v_b = qhvb * h, m_b = qhmb * h;
@@ -1583,11 +1625,12 @@ DC_HD bool src2_cell_b(const dclaw_params& P, double phi, double dt, const doubl
     if (moving) {
         // u2 = hu2 / h1, v2 = hv2 / h1
         double hu2b = u2b / h1, hv2b = v2b / h1;
-        h1b -= (u2b * u2 + v2b * v2) / h1;
+        h1b -= hu2b * u2 + hv2b * v2;
         // hu2 = hvnorm hu1 / hvnorm0, hv2 = hvnorm hv1 / hvnorm0
         double hvnormb = (hu2b * hu1 + hv2b * hv1) / hvnorm0;
-        hu1b += hu2b * hvnorm / hvnorm0;
-        hv1b += hv2b * hvnorm / hvnorm0;
+        const double slow = hvnorm / hvnorm0;
+        hu1b += hu2b * slow;
+        hv1b += hv2b * slow;
         double hvnorm0b = -(hu2b * hu2 + hv2b * hv2) / hvnorm0;
         // hvnorm = h1 vn2
         h1b += hvnormb * vn2;
@@ -1603,13 +1646,16 @@ DC_HD bool src2_cell_b(const dclaw_params& P, double phi, double dt, const doubl
         // vn1 = max(0, a), a = vnorm - dt tau / rhoh
         double ab = (0.0 > a) ? 0.0 : vn1b;
         double vnormb = ab;
-        taub -= ab * dt / rhoh;
-        rhohb += ab * dt * sv.tau / (rhoh * rhoh);
+        const double w0 = ab * dt / rhoh;
+        taub -= w0;
+        rhohb += w0 * sv.tau / rhoh;
         // vnorm = hvnorm0 / h1
-        hvnorm0b += vnormb / h1;
-        h1b -= vnormb * vnorm / h1;
-        hu1b += hvnorm0b * hu1 / hvnorm0;
-        hv1b += hvnorm0b * hv1 / hvnorm0;
+        const double vh = vnormb / h1;
+        hvnorm0b += vh;
+        h1b -= vh * vnorm;
+        const double w = hvnorm0b / hvnorm0;
+        hu1b += w * hu1;
+        hv1b += w * hv1;
     } else {
         u1b += u2b;
         v1b += v2b;
