@@ -284,23 +284,107 @@ struct BlkMinB {
     static constexpr int value = heavy ? DCLAW_ADJ_HEAVY_MINB : DCLAW_ADJ_MINB / 2;
 };
 
-// One stage over a list of (member, block) entries (grid-stride; every
-// thread of a CTA runs the same iterations, so the barriers are uniform).
-// A CTA has one thread per item of a 16 x 16 block; two CTAs per SM at up
-// to 128 registers a thread.
+// Stage OP on one listed block (all threads of the CTA): m its member, whose
+// table entry and parameters are sM and sP, blk the block. A CTA has one
+// thread per item of a 16 x 16 block; two CTAs per SM at up to 128 registers
+// a thread.
+struct BlockScratch {
+    int list[BTPB];
+    int wcnt[BTPB / 32];
+};
 template <int OP>
+__device__ __forceinline__ void block_stage(const BatchArgs& a, int m, const dclaw_adj_member& sM,
+                                            const dclaw_params& sP, int blk, BlockScratch& sh) {
+    const Geom g{sM.mx, sM.my, sM.mx + 4, sM.my + 4, sM.dx, sM.dy};
+    AdjLayout L;
+    Work W;
+    AdjWork A;
+    uint32_t* act;
+    batch_member_work(a, sM, L, W, A, act);
+    const int bx = blk % L.act_nx, by = blk / L.act_nx;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int ci = bx * ACT_TILE + tx - 1, cj = by * ACT_TILE + ty - 1;
+    double pb[NPB] = {0.0, 0.0, 0.0, 0.0};
+    if (OP == OP_RV_RX || OP == OP_RV_RY) {
+        // the reverse of a dry-dry solve writes zeros (the forward
+        // skipped it): those items store their zeros here, the others
+        // are gathered into a dense list so that the warps running the
+        // reverse solver are full of them
+        constexpr int DIR = OP == OP_RV_RX ? 0 : 1;
+        const int mx = g.mx, my = g.my;
+        const bool valid = DIR == 0 ? (ci >= 0 && cj >= 0 && ci <= mx + 2 && cj <= my + 1)
+                                    : (ci >= 0 && cj >= 0 && ci <= mx + 1 && cj <= my + 2);
+        bool need = false;
+        if (valid) {
+            // x: row r = cj, interface i = ci (cells i-1, i); y: column r = ci, interface i = cj
+            const size_t pL = DIR == 0 ? pidx(g, ci - 1, cj) : pidx(g, ci, cj - 1);
+            const size_t pR = pidx(g, ci, cj);
+            need = !(W.qB[pL] <= sP.dry_tolerance && W.qB[pR] <= sP.dry_tolerance);
+            if (!need) {
+                double* dst = DIR == 0 ? A.xcb : A.ycb;
+                const size_t np = DIR == 0 ? W.nxi : W.nyi;
+                const size_t oi = DIR == 0 ? xidx(g, cj, ci) : yidx(g, cj, ci);
+                const int nz = A.bed ? NCB : NCB_Q;
+                for (int k = 0; k < nz; ++k) dst[(size_t)k * np + oi] = 0.0;
+            }
+        }
+        // the list is in thread order (warp counts summed in warp
+        // order), so each item lands on the same thread every run and
+        // the block's parameter partial is bit-reproducible
+        const unsigned bal = __ballot_sync(0xffffffffu, need);
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        if (lane == 0) sh.wcnt[wid] = __popc(bal);
+        __syncthreads();
+        int base = 0, tot = 0;
+        for (int w = 0; w < BTPB / 32; ++w) {
+            base += w < wid ? sh.wcnt[w] : 0;
+            tot += sh.wcnt[w];
+        }
+        if (need) sh.list[base + __popc(bal & ((1u << lane) - 1u))] = threadIdx.x;
+        __syncthreads();
+        if ((int)threadIdx.x < tot) {
+            const int t = sh.list[threadIdx.x];
+            block_item<OP>(a, m, sM, sP, g, W, A, L, bx * ACT_TILE + (t & 15) - 1, by * ACT_TILE + (t >> 4) - 1,
+                           pb);
+        }
+    } else if (OpTraits<OP>::PBAR || OP >= OP_RV_SRC2 || act[blk] ||
+               near_active_block(act, L.act_nx, L.act_ny, bx, by, ci, cj, FwMargin<OP>::value)) {
+        // forward stages run over active blocks and their neighbours; in
+        // a neighbour, only near the active ones
+        block_item<OP>(a, m, sM, sP, g, W, A, L, ci, cj, pb);
+    }
+    if (OpTraits<OP>::PBAR) {
+        const int pidx = OP == OP_RV_SRC2 ? 0 : OP == OP_RV_RX ? 1 : OP == OP_RV_RY ? 2 : 3;
+        double* part = (double*)(a.work + sM.work_off + L.off_part);
+        block_pbar<BTPB / 32>(pb, part + ((size_t)pidx * L.act_nx * L.act_ny + blk) * NPB);
+    }
+}
+
+// Stage OP over a list of (member, block) entries, then, where OP2 is
+// another, OP2 over the same list (the y items after the x items). Grid-
+// stride; every thread of a CTA runs the same iterations, so the barriers are
+// uniform. On a 512^2 patch one direction's blocks fill the resident CTAs one
+// and a half times, and launched by itself each direction pays for two
+// rounds: with both directions in one launch the forward solves and fluxes of
+// a 512^2 step take 196 us with what else is prepared (215 in two), the
+// reverse chain 433 us with the fluxes so (442). The reverse solves spill
+// most, and two codes of theirs at once miss the instruction cache: they are
+// paired up to PAIR_SOLVES_BLOCKS blocks (128^2, 81: 128 us, 156 in two
+// launches; 333 x 200, 273: 220 and 223), not above (512^2, 1089: 442 and
+// 433; 1024^2: 1204 and 1168).
+constexpr uint32_t PAIR_SOLVES_BLOCKS = 600;
+template <int OP, int OP2 = OP>
 __global__ void __launch_bounds__(BTPB, BlkMinB<OP>::value) k_adj_blocks(BatchArgs a, const uint64_t* __restrict__ list,
-                                                                     const unsigned int* __restrict__ count) {
+                                                                         const unsigned int* __restrict__ count) {
     __shared__ dclaw_adj_member sM;
     __shared__ dclaw_params sP;
     __shared__ uint64_t s_e;
-    __shared__ int s_list[BTPB];
-    __shared__ int s_wcnt[BTPB / 32];
+    __shared__ BlockScratch sh;
     pdl_wait();
-    const unsigned int n = *count;
+    const unsigned int n = *count, total = OP == OP2 ? n : 2u * n;
     int cur = -1;
-    for (unsigned int k = blockIdx.x; k < n; k += gridDim.x) {
-        if (threadIdx.x == 0) s_e = list[k];
+    for (unsigned int k = blockIdx.x; k < total; k += gridDim.x) {
+        if (threadIdx.x == 0) s_e = list[k < n ? k : k - n];
         __syncthreads();
         const int m = (int)(s_e >> 32);
         const int blk = (int)(s_e & 0xffffffffu);
@@ -313,69 +397,8 @@ __global__ void __launch_bounds__(BTPB, BlkMinB<OP>::value) k_adj_blocks(BatchAr
             __syncthreads();
             cur = m;
         }
-        const Geom g{sM.mx, sM.my, sM.mx + 4, sM.my + 4, sM.dx, sM.dy};
-        AdjLayout L;
-        Work W;
-        AdjWork A;
-        uint32_t* act;
-        batch_member_work(a, sM, L, W, A, act);
-        const int bx = blk % L.act_nx, by = blk / L.act_nx;
-        const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-        const int ci = bx * ACT_TILE + tx - 1, cj = by * ACT_TILE + ty - 1;
-        double pb[NPB] = {0.0, 0.0, 0.0, 0.0};
-        if (OP == OP_RV_RX || OP == OP_RV_RY) {
-            // the reverse of a dry-dry solve writes zeros (the forward
-            // skipped it): those items store their zeros here, the others
-            // are gathered into a dense list so that the warps running the
-            // reverse solver are full of them
-            constexpr int DIR = OP == OP_RV_RX ? 0 : 1;
-            const int mx = g.mx, my = g.my;
-            const bool valid = DIR == 0 ? (ci >= 0 && cj >= 0 && ci <= mx + 2 && cj <= my + 1)
-                                        : (ci >= 0 && cj >= 0 && ci <= mx + 1 && cj <= my + 2);
-            bool need = false;
-            if (valid) {
-                // x: row r = cj, interface i = ci (cells i-1, i); y: column r = ci, interface i = cj
-                const size_t pL = DIR == 0 ? pidx(g, ci - 1, cj) : pidx(g, ci, cj - 1);
-                const size_t pR = pidx(g, ci, cj);
-                need = !(W.qB[pL] <= sP.dry_tolerance && W.qB[pR] <= sP.dry_tolerance);
-                if (!need) {
-                    double* dst = DIR == 0 ? A.xcb : A.ycb;
-                    const size_t np = DIR == 0 ? W.nxi : W.nyi;
-                    const size_t oi = DIR == 0 ? xidx(g, cj, ci) : yidx(g, cj, ci);
-                    const int nz = A.bed ? NCB : NCB_Q;
-                    for (int k = 0; k < nz; ++k) dst[(size_t)k * np + oi] = 0.0;
-                }
-            }
-            // the list is in thread order (warp counts summed in warp
-            // order), so each item lands on the same thread every run and
-            // the block's parameter partial is bit-reproducible
-            const unsigned bal = __ballot_sync(0xffffffffu, need);
-            const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-            if (lane == 0) s_wcnt[wid] = __popc(bal);
-            __syncthreads();
-            int base = 0, tot = 0;
-            for (int w = 0; w < BTPB / 32; ++w) {
-                base += w < wid ? s_wcnt[w] : 0;
-                tot += s_wcnt[w];
-            }
-            if (need) s_list[base + __popc(bal & ((1u << lane) - 1u))] = threadIdx.x;
-            __syncthreads();
-            if ((int)threadIdx.x < tot) {
-                const int t = s_list[threadIdx.x];
-                block_item<OP>(a, m, sM, sP, g, W, A, L, bx * ACT_TILE + (t & 15) - 1, by * ACT_TILE + (t >> 4) - 1,
-                               pb);
-            }
-        } else if (OpTraits<OP>::PBAR || OP >= OP_RV_SRC2 || act[blk] ||
-                   near_active_block(act, L.act_nx, L.act_ny, bx, by, ci, cj, FwMargin<OP>::value)) {
-            // forward stages run over active blocks and their neighbours; in
-            // a neighbour, only near the active ones
-            block_item<OP>(a, m, sM, sP, g, W, A, L, ci, cj, pb);
-        }
-        if (OpTraits<OP>::PBAR) {
-            const int pidx = OP == OP_RV_SRC2 ? 0 : OP == OP_RV_RX ? 1 : OP == OP_RV_RY ? 2 : 3;
-            double* part = (double*)(a.work + sM.work_off + L.off_part);
-            block_pbar<BTPB / 32>(pb, part + ((size_t)pidx * L.act_nx * L.act_ny + blk) * NPB);
-        }
+        if (OP == OP2 || k < n) block_stage<OP>(a, m, sM, sP, blk, sh);
+        else block_stage<OP2>(a, m, sM, sP, blk, sh);
         __syncthreads();
     }
 }
@@ -557,8 +580,7 @@ inline void launch_block_adjoint(const BatchArgs& a, uint32_t nblocks, char* lis
     const dim3 per_member((unsigned)gx, (unsigned)a.nmem);
     // persistent grids over the lists
     const unsigned grid = (unsigned)nsm * 2u;
-#define DC_FW(op) k_adj_blocks<op><<<grid, BTPB, 0, s>>>(a, list_dil, counts + 1)
-#define DC_RV(op) k_adj_blocks<op><<<grid, BTPB, 0, s>>>(a, list_act, counts)
+#define DC_FW(...) k_adj_blocks<__VA_ARGS__><<<grid, BTPB, 0, s>>>(a, list_dil, counts + 1)
     if (phase & PHASE_PREPARE) {
         k_adj_batch_zero<<<per_member, 256, 0, s>>>(a, counts, 1);
         k_adj_batch_scan<<<per_member, 256, 0, s>>>(a);
@@ -567,21 +589,21 @@ inline void launch_block_adjoint(const BatchArgs& a, uint32_t nblocks, char* lis
         DC_FW(OP_FW_B4);
         DC_FW(OP_FW_TAUDIR);
         DC_FW(OP_FW_SVREC);
-        DC_FW(OP_FW_RX);
-        DC_FW(OP_FW_RY);
-        DC_FW(OP_FW_FX);
-        DC_FW(OP_FW_FY);
+        DC_FW(OP_FW_RX, OP_FW_RY);
+        DC_FW(OP_FW_FX, OP_FW_FY);
     }
     if (!(phase & PHASE_REVERSE)) return;
-#undef DC_RV
-#define DC_RV(op) launch_pdl(k_adj_blocks<op>, dim3(grid), dim3(BTPB), 0, s, a, (const uint64_t*)list_act, \
+#define DC_RV(...) launch_pdl(k_adj_blocks<__VA_ARGS__>, dim3(grid), dim3(BTPB), 0, s, a, (const uint64_t*)list_act, \
                              (const unsigned int*)counts)
     launch_pdl(k_adj_batch_zero, per_member, dim3(256), 0, s, a, counts, 2);
     DC_RV(OP_RV_SRC2);
-    DC_RV(OP_RV_FX);
-    DC_RV(OP_RV_FY);
-    DC_RV(OP_RV_RX);
-    DC_RV(OP_RV_RY);
+    DC_RV(OP_RV_FX, OP_RV_FY);
+    if (nblocks <= PAIR_SOLVES_BLOCKS) {
+        DC_RV(OP_RV_RX, OP_RV_RY);
+    } else {
+        DC_RV(OP_RV_RX);
+        DC_RV(OP_RV_RY);
+    }
     DC_RV(OP_RV_TAUDIR);
     DC_RV(OP_RV_B4);
     DC_RV(OP_RV_GATHER);
