@@ -96,3 +96,25 @@ def test_patch_calls_equal_step(size, k):
         pt.src2(qp, aux, DX, DX, 0.0, 0.02)
     assert torch.equal(qp[:, MBC:-MBC, MBC:-MBC], st.state())
     assert cfl == float(st.clock[2])
+
+
+@pytest.mark.parametrize("size", [(3, 2), (31, 17), (100, 15), (380, 380), (400, 400), (900, 260)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_adjoint_equals_host_build(size):
+    """Few and many activity blocks (the reverse solves of the two directions
+    share a launch up to 600), ragged ones, and cells at rest beside moving
+    ones, which alone carry calc_taudir's and setvars' adjoints."""
+    from dclaw_b200.adjoint import StepAdjoint
+
+    from ._adj import Adj
+
+    p = DClawParams()
+    q, b = flow(*size, p, seed=3)
+    q[1:3, :, : size[0] // 2] = 0.0
+    lam = np.random.default_rng(4).standard_normal(q.shape)
+    want, _ = Adj().vjp(p, q, b, DX, DX, 0.02, lam)
+    adj = StepAdjoint(torch.tensor(b, device="cuda"), p, DX, DX)
+    got = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+    adj.vjp(torch.tensor(q, device="cuda"), torch.tensor([0.02], dtype=torch.float64, device="cuda"),
+            torch.tensor(lam, device="cuda"), got, torch.zeros(4, dtype=torch.float64, device="cuda"))
+    adj.check_status()
+    assert np.array_equal(got.cpu().numpy(), want)
