@@ -52,20 +52,14 @@ static std::mutex g_setup_mu;
 #ifndef DCLAW_SRC2_KERNEL
 #define DCLAW_SRC2_KERNEL 1
 #endif
-// the same choice for the step over tile lists: k_src2_list (1), or src2 and
-// the tick in k_tile_list (0)
-#ifndef DCLAW_LIST_SRC2_KERNEL
-#define DCLAW_LIST_SRC2_KERNEL 1
-#endif
-// and for the ensemble step: k_src2_batch (1), or src2 in k_tile_batch (0)
-#ifndef DCLAW_BATCH_SRC2_KERNEL
-#define DCLAW_BATCH_SRC2_KERNEL 1
-#endif
 constexpr int TILE_X = DCLAW_TILE_X, TILE_Y = DCLAW_TILE_Y;
 // resident blocks per SM the ensemble's streaming scan is sized for
 #ifndef DCLAW_SCAN_MINB
 #define DCLAW_SCAN_MINB 4
 #endif
+// and the single patch's, which only reads: 6 steps the 4096^2 field 0.5 %
+// faster than 4 (the ensemble's, which also writes, 4 % slower)
+constexpr int PATCH_SCAN_MINB = 6;
 // resident blocks per SM the ensemble's per-cell kernels (records of the
 // listed tiles, src2) are sized for
 #ifndef DCLAW_CELL_MINB
@@ -79,14 +73,13 @@ constexpr int TILE_X = DCLAW_TILE_X, TILE_Y = DCLAW_TILE_Y;
 #endif
 constexpr int BATCH_CELL_TPB = DCLAW_BATCH_CELL_TPB;
 constexpr int BATCH_CELL_MINB = DCLAW_CELL_MINB * 256 / DCLAW_BATCH_CELL_TPB;
-// resident blocks per SM the single-patch per-cell kernels (k_records,
-// k_src2_cells) are sized for: on the 4096^2 random field 6 (40 registers,
-// with spills) steps 1.9 % faster than 4 (64 registers), 5 1.2 % and 8
-// (32 registers) 0.8 %; 3 and 2 (80 and 110 registers, no spills) 4 % and
-// 10 % slower. The ensemble's per-cell kernels are fastest at 4 (6 is 5 %
+// resident blocks per SM the single-patch per-cell kernels (the records and
+// src2) are sized for: the 4096^2 random field steps in 3.03, 3.01, 3.05 and
+// 3.13 ms with 4, 5, 6 and 8 (64, 48, 40 and 32 registers, all with spills).
+// The ensemble's per-cell kernels are fastest at 4 (5 and 6 are 2 % and 4 %
 // slower there).
 #ifndef DCLAW_PLAIN_CELL_MINB
-#define DCLAW_PLAIN_CELL_MINB 6
+#define DCLAW_PLAIN_CELL_MINB 5
 #endif
 // threads per CTA of k_src2_list and k_src2_cells (the register budget is
 // that of DCLAW_PLAIN_CELL_MINB blocks of 256 threads whatever the CTA
@@ -899,28 +892,22 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_cells(dclaw_params
 // cells with src2 of the updated state, and its last block applies the tick.
 // Each cell's arithmetic is that of the full-grid kernels, so the results
 // are the same bits; far from the flow a cell costs its 80 bytes of scan.
-// cells [s0, s1) are scanned, cells [z0, z1) of q_out zeroed (linear
-// interior indices; the whole patch for dclaw_step, a row range and the rows
-// within 3 of it for dclaw_step_rows)
-__global__ void __launch_bounds__(TPB, DCLAW_SCAN_MINB) k_scan_patch(dclaw_params P, int mx, int my,
-                                                                    const double* __restrict__ q_in,
-                                                                    double* __restrict__ q_out, dclaw_clock* clk,
+// cells [s0, s1) are scanned (linear interior indices; the whole patch for
+// dclaw_step, a row range and the rows within 3 of it for dclaw_step_rows)
+__global__ void __launch_bounds__(TPB, PATCH_SCAN_MINB) k_scan_patch(dclaw_params P, int mx, int my,
+                                                                    const double* __restrict__ q_in, dclaw_clock* clk,
                                                                     unsigned int* counters,
                                                                     uint32_t* __restrict__ tflag, size_t s0,
-                                                                    size_t s1, size_t z0, size_t z1) {
+                                                                    size_t s1) {
     pdl_wait();
     // tile queue, list lengths, src2method 2's cell counter
     if (blockIdx.x == 0 && threadIdx.x < 6) counters[threadIdx.x] = 0u;
     const size_t n = (size_t)mx * my;
     const int ntx = (mx + TILE_X - 1) / TILE_X, nty = (my + TILE_Y - 1) / TILE_Y;
-    const size_t lo = s0 < z0 ? s0 : z0, hi = s1 > z1 ? s1 : z1;
     bool nan = false;
-    for (size_t idx = lo + (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < hi;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        if (idx >= s0 && idx < s1 && scan_cell(P, q_in, n, idx, mx, tflag, clk, TILE_X, TILE_Y, ntx, nty)) nan = true;
-        if (idx >= z0 && idx < z1)
-            for (int f = 0; f < 5; ++f) q_out[(size_t)f * n + idx] = 0.0;
-    }
+    for (size_t idx = s0 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < s1;
+         idx += (size_t)gridDim.x * blockDim.x)
+        if (scan_cell(P, q_in, n, idx, mx, tflag, clk, TILE_X, TILE_Y, ntx, nty)) nan = true;
     if (nan) flag_status(clk, DCLAW_ERR_NAN);
 }
 
@@ -969,26 +956,76 @@ __global__ void __launch_bounds__(RECORDS_TPB, RECORDS_MINB) k_records_list(dcla
     }
 }
 
-// persistent: each CTA takes active tiles from the queue until it is empty;
-// the Courant number is max-reduced once per CTA at the end. WITH_SRC2:
-// q_out receives the state after src2 and the last CTA applies the tick
-// (no k_src2_list); otherwise the pre-src2 state.
-template <bool WITH_SRC2>
+// The zero state of the cells no src2 writes, by bulk copies from a zeroed
+// block of shared memory, a few with every tile: the tile kernels leave DRAM
+// nine tenths idle and the copies cost one thread an instruction each, where
+// the scan wrote the zeros in time of its own. The 4096^2 field steps in 3.04
+// ms so and in 3.09 ms with the zeros in the scan or all at the end of the
+// tile kernel, 1000 x 731 in 231.5 and 233.4 us; the flume ensemble lost
+// 1.5 % (its narrow members make short copies, and its state mostly stays in
+// the L2) and keeps them in its scan. src2 overwrites the active tiles'
+// cells in the next launch.
+constexpr unsigned ZERO_CHUNK = 1024;  // doubles per copy
+// Zeroes n doubles from dst (a double's alignment); completed by zero_wait.
+__device__ __forceinline__ void zero_issue(double* dst, unsigned n, const double* zeros) {
+    if (((uintptr_t)dst & 8u) && n > 0) {
+        *dst++ = 0.0;
+        --n;
+    }
+    if (n & 1u) dst[n - 1] = 0.0;
+    const unsigned bytes = (n >> 1) * 16u;
+    if (bytes)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                     "r"((unsigned)__cvta_generic_to_shared(zeros)), "r"(bytes)
+                     : "memory");
+}
+__device__ __forceinline__ void zero_wait() {
+    asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+}
+// all threads, before a barrier: the block the copies read
+__device__ __forceinline__ void zero_block(double* zeros) {
+    for (unsigned k = threadIdx.x; k < ZERO_CHUNK; k += blockDim.x) zeros[k] = 0.0;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// persistent: each CTA takes active tiles from the queue until it is empty
+// (their state before src2 goes to q_star); the Courant number is max-reduced
+// once per CTA at the end. Cells [z0, z1) of every plane of q_zero are
+// zeroed on the way, each CTA its share of the copies.
 __global__ void __launch_bounds__(TILE_TPB, DCLAW_TILE_MINBLOCKS) k_tile_list(dclaw_params P, Geom g, Rec R,
                                                                              const double* __restrict__ b,
-                                                                             double* __restrict__ q_out,
+                                                                             double* __restrict__ q_star,
                                                                              dclaw_clock* clk, unsigned int* counters,
-                                                                             const uint32_t* __restrict__ list_act) {
+                                                                             const uint32_t* __restrict__ list_act,
+                                                                             double* __restrict__ q_zero, size_t z0,
+                                                                             size_t z1) {
     pdl_wait();
     extern __shared__ double smem[];
     // the tile of this pass and the next one's, claimed at the start of this
     // pass: the barrier that ends a pass also publishes the next index
     __shared__ uint32_t s_t[2];
+    __shared__ alignas(128) double s_zero[ZERO_CHUNK];
     const unsigned int nact = counters[1];
     const uint32_t ntx = (uint32_t)((g.mx + TILE_X - 1) / TILE_X);
     const double dt = clk->dt, crit = critical_root(P);
     double cfl = 0.0;
     bool nan_any = false;
+    zero_block(s_zero);
+    // this CTA's copies [zc, zend) of all the planes', and how many go out
+    // with a tile when the tiles are shared out evenly
+    const bool zeroer = threadIdx.x == blockDim.x - 32;
+    const size_t plane = (size_t)g.mx * g.my;
+    const unsigned zper = (unsigned)((z1 - z0 + ZERO_CHUNK - 1) / ZERO_CHUNK);
+    unsigned zc = (unsigned)(5ull * zper * blockIdx.x / gridDim.x);
+    const unsigned zend = (unsigned)(5ull * zper * (blockIdx.x + 1) / gridDim.x);
+    const unsigned zstep = umin((unsigned)(5ull * zper / (nact > 0 ? nact : 1u)) + 1u, 64u);
+    auto zero_some = [&](unsigned n) {
+        for (; n > 0 && zc < zend; --n, ++zc) {
+            const unsigned f = zc / zper;
+            const size_t c = z0 + (size_t)(zc - f * zper) * ZERO_CHUNK;
+            zero_issue(q_zero + f * plane + c, (unsigned)(z1 - c < ZERO_CHUNK ? z1 - c : ZERO_CHUNK), s_zero);
+        }
+    };
     if (threadIdx.x == 0) {
         const unsigned int k = atomicAdd(counters, 1u);
         s_t[0] = k < nact ? list_act[k] : 0xffffffffu;
@@ -1002,18 +1039,22 @@ __global__ void __launch_bounds__(TILE_TPB, DCLAW_TILE_MINBLOCKS) k_tile_list(dc
             const unsigned int k = atomicAdd(counters, 1u);
             s_t[(pass + 1) & 1] = k < nact ? list_act[k] : 0xffffffffu;
         }
+        if (zeroer) zero_some(zstep);
         const int i0 = 1 + (int)(t % ntx) * TILE_X, j0 = 1 + (int)(t / ntx) * TILE_Y;
         bool nan;
         const double c =
-            tile_body<TILE_X, TILE_Y, WITH_SRC2, TILE_TPB>(P, g, R, b, q_out, dt, i0, j0, smem, nullptr, nan, crit);
+            tile_body<TILE_X, TILE_Y, false, TILE_TPB>(P, g, R, b, q_star, dt, i0, j0, smem, nullptr, nan, crit);
         cfl = fmax2(cfl, c);
         nan_any = nan_any || nan;
         // the next tile's staging overwrites shared memory
         __syncthreads();
     }
+    if (zeroer) {
+        zero_some(0xffffffffu);
+        zero_wait();
+    }
     if (nan_any) flag_status(clk, DCLAW_ERR_NAN);
     block_max_to(cfl, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
-    if (WITH_SRC2) last_block_tick(P, clk);
 }
 
 __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_list(dclaw_params P, Geom g,
@@ -1269,8 +1310,7 @@ template <int TX, int TY>
 __global__ void __launch_bounds__(TPB, 2) k_tile_batch(int nmem, uint32_t ntiles, const dclaw_member* __restrict__ mem,
                                                        const dclaw_params* __restrict__ prm, dclaw_clock* clocks,
                                                        const double* __restrict__ b, double* __restrict__ work,
-                                                       unsigned int* counters, const uint32_t* __restrict__ list_act,
-                                                       double* __restrict__ q_out) {
+                                                       unsigned int* counters, const uint32_t* __restrict__ list_act) {
     pdl_wait();
     extern __shared__ double smem[];
     __shared__ dclaw_member sM;
@@ -1279,7 +1319,7 @@ __global__ void __launch_bounds__(TPB, 2) k_tile_batch(int nmem, uint32_t ntiles
     __shared__ int s_m;
     __shared__ double red[TPB / 32];
     // the queue hands out the active tiles only (inactive tiles: no wet
-    // cell within 3; src2 writes their zeros)
+    // cell within 3; their zeros are the scan's)
     const unsigned int nact = counters[1];
     int cur = -1;
     for (;;) {
@@ -1302,10 +1342,9 @@ __global__ void __launch_bounds__(TPB, 2) k_tile_batch(int nmem, uint32_t ntiles
         const unsigned int lt = t - sM.tile0;
         const int i0 = 1 + (int)(lt % sM.ntiles_x) * TX, j0 = 1 + (int)(lt / sM.ntiles_x) * TY;
         bool nan;
-        // with src2 in this kernel the tile writes the member's new state,
-        // otherwise its pre-src2 state (k_src2_batch follows)
-        double* dst = DCLAW_BATCH_SRC2_KERNEL ? work + sM.qs_off : q_out + sM.q_off;
-        double cfl = tile_body<TX, TY, !DCLAW_BATCH_SRC2_KERNEL, TPB>(sP, g, R, b + sM.b_off, dst, clocks[m].dt, i0, j0,
+        // the member's state before src2 (k_src2_batch follows)
+        double* dst = work + sM.qs_off;
+        double cfl = tile_body<TX, TY, false, TPB>(sP, g, R, b + sM.b_off, dst, clocks[m].dt, i0, j0,
                                                                      smem, nullptr, nan, critical_root(sP));
         if (nan) flag_status(clocks + m, DCLAW_ERR_NAN);
         // block max of this tile's Courant number into member m's clock
@@ -1379,12 +1418,12 @@ inline int batch_tile_attr() {
 template <int TX, int TY>
 inline int launch_tile_batch(const dclaw_batch* B, const dclaw_member* mem, const dclaw_params* prm, dclaw_clock* clocks,
                              const double* b, double* work, unsigned int* counters, const uint32_t* list_act, int nsm,
-                             cudaStream_t s, double* q_out = nullptr) {
+                             cudaStream_t s) {
     if (batch_tile_attr<TX, TY>() != DCLAW_OK) return DCLAW_ERR_CUDA;
     unsigned grid = (unsigned)(nsm * (B->tile_ctas_per_sm > 0 ? B->tile_ctas_per_sm : 2));
     if (grid > B->ntiles) grid = B->ntiles > 0 ? B->ntiles : 1;
     launch_pdl(k_tile_batch<TX, TY>, dim3(grid), dim3(TPB), TileGeom<TX, TY>::SMEM_BYTES, s, B->nmembers, B->ntiles, mem, prm, clocks, b,
-                                                                        work, counters, list_act, q_out);
+               work, counters, list_act);
     return DCLAW_OK;
 }
 
@@ -1399,9 +1438,8 @@ inline int launch_batch_tiles(const dclaw_batch* B, const dclaw_member* mem, con
     if (g1 > B->ntiles) g1 = B->ntiles > 0 ? B->ntiles : 1;
     launch_pdl(k_records_tiles_batch<TX, TY>, dim3(g1), dim3(BATCH_CELL_TPB), 0, s, B->nmembers, B->ntiles, mem, prm, q_in, b, w, counters,
                                                                  list_rec);
-    int rc = launch_tile_batch<TX, TY>(B, mem, prm, clocks, b, w, counters, list_act, nsm, s, q_out);
+    int rc = launch_tile_batch<TX, TY>(B, mem, prm, clocks, b, w, counters, list_act, nsm, s);
     if (rc != DCLAW_OK) return rc;
-    if (!DCLAW_BATCH_SRC2_KERNEL) return DCLAW_OK;
     unsigned g3 = (unsigned)(nsm * cpsm);
     if (g3 > B->ntiles) g3 = B->ntiles > 0 ? B->ntiles : 1;
     launch_pdl(k_src2_batch<TX, TY>, dim3(g3), dim3(BATCH_CELL_TPB), 0, s, B->nmembers, B->ntiles, mem, prm, clocks, q_out, w, counters,
@@ -1653,11 +1691,9 @@ inline int ensure_tile_smem_attr() {
                                      bytes) != cudaSuccess ||
                 cudaFuncSetAttribute(k_tile<TILE_X, TILE_Y, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      bytes) != cudaSuccess ||
-                cudaFuncSetAttribute(k_tile_list<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
-                    cudaSuccess ||
+                cudaFuncSetAttribute(k_tile_list, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
                 cudaFuncSetAttribute(k_tile_apart<TILE_X, TILE_Y>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)TileGeom<TILE_X, TILE_Y>::SMEM2_BYTES) != cudaSuccess ||
-                cudaFuncSetAttribute(k_tile_list<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+                                     (int)TileGeom<TILE_X, TILE_Y>::SMEM2_BYTES) != cudaSuccess)
                 return DCLAW_ERR_CUDA;
             done[dev].store(true, std::memory_order_release);
         }
@@ -1924,10 +1960,10 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
         double* qstar = (double*)((char*)work + L.off_qstar);
         const long long ncell = (long long)mx * my;
         const unsigned ntiles = (unsigned)ntx * (unsigned)nty;
-        unsigned g0 = (unsigned)(nsm * DCLAW_SCAN_MINB * 2);
+        unsigned g0 = (unsigned)(nsm * PATCH_SCAN_MINB * 2);
         if ((long long)g0 * TPB > ncell) g0 = nblocks(ncell);
-        launch_pdl(k_scan_patch, dim3(g0), dim3(TPB), 0, s, P, mx, my, q_in, q_out, clock, counters, tflag, 0, (size_t)ncell, 0,
-                                        (size_t)ncell);
+        launch_pdl(k_scan_patch, dim3(g0), dim3(TPB), 0, s, P, mx, my, q_in, clock, counters, tflag, 0,
+                   (size_t)ncell);
         launch_pdl(k_list_patch, dim3((ntiles + TPB - 1) / TPB), dim3(TPB), 0, s, ntx, nty, clock, tflag, counters, list_act, list_rec, 0,
                                                              nty - 1);
         unsigned g1 = (unsigned)(nsm * RECORDS_MINB);
@@ -1935,11 +1971,8 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
         launch_pdl(k_records_list, dim3(g1), dim3(RECORDS_TPB), 0, s, P, g, q_in, b, R, counters, list_rec);
         unsigned g2 = (unsigned)(nsm * DCLAW_TILE_MINBLOCKS);
         if (g2 > ntiles) g2 = ntiles;
-        if (!DCLAW_LIST_SRC2_KERNEL) {
-            launch_pdl(k_tile_list<true>, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, q_out, clock, counters, list_act);
-            return cuda_status();
-        }
-        launch_pdl(k_tile_list<false>, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock, counters, list_act);
+        launch_pdl(k_tile_list, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock, counters,
+                   list_act, q_out, 0, (size_t)ncell);
         unsigned g3 = (unsigned)(nsm * SRC2_MINB);
         if (g3 > ntiles) g3 = ntiles;
         launch_src2_list(P, g, qstar, q_out, clock, counters, list_act, g3, nsm, ntiles, 1, s);
@@ -2104,10 +2137,10 @@ int dclaw_step_rows(const double* q_in, double* q_out, const double* b, int mx, 
     const int ty0 = (row_first - 1) / TILE_Y, ty1 = (last - 1) / TILE_Y;
     const int sa = row_first - 3 > 1 ? row_first - 3 : 1, sb = last + 3 < my ? last + 3 : my;
     const long long nscan = (long long)(sb - sa + 1) * mx;
-    unsigned g0 = (unsigned)(sm * DCLAW_SCAN_MINB * 2);
+    unsigned g0 = (unsigned)(sm * PATCH_SCAN_MINB * 2);
     if ((long long)g0 * TPB > nscan) g0 = nblocks(nscan);
-    launch_pdl(k_scan_patch, dim3(g0), dim3(TPB), 0, s, P, mx, my, q_in, q_out, clock, counters, tflag, (size_t)(sa - 1) * mx,
-                                    (size_t)sb * mx, (size_t)(row_first - 1) * mx, (size_t)last * mx);
+    launch_pdl(k_scan_patch, dim3(g0), dim3(TPB), 0, s, P, mx, my, q_in, clock, counters, tflag,
+               (size_t)(sa - 1) * mx, (size_t)sb * mx);
     launch_pdl(k_list_patch, dim3((ntiles + TPB - 1) / TPB), dim3(TPB), 0, s, ntx, ntyp, clock, tflag, counters, list_act, list_rec, ty0,
                                                          ty1);
     unsigned g1 = (unsigned)(sm * RECORDS_MINB);
@@ -2115,7 +2148,8 @@ int dclaw_step_rows(const double* q_in, double* q_out, const double* b, int mx, 
     launch_pdl(k_records_list, dim3(g1), dim3(RECORDS_TPB), 0, s, P, g, q_in, b, R, counters, list_rec);
     unsigned g2 = (unsigned)(sm * DCLAW_TILE_MINBLOCKS);
     if (g2 > ntiles) g2 = ntiles;
-    launch_pdl(k_tile_list<false>, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock, counters, list_act);
+    launch_pdl(k_tile_list, dim3(g2), dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock, counters, list_act,
+               q_out, (size_t)(row_first - 1) * mx, (size_t)last * mx);
     unsigned g3 = (unsigned)(sm * SRC2_MINB);
     if (g3 > ntiles) g3 = ntiles;
     launch_src2_list(P, g, qstar, q_out, clock, counters, list_act, g3, sm, ntiles, 0, s);
@@ -2458,7 +2492,7 @@ int dclaw_step_batched(const dclaw_batch* batch, const dclaw_member* members, co
     unsigned g0 = (unsigned)(nsm * cpsm);
     if (g0 > batch->nschunks) g0 = batch->nschunks;
     launch_pdl(k_scan_batch, dim3(g0), dim3(TPB), 0, s, batch->nmembers, batch->nschunks, members, params, clocks, q_in, q_out, counters,
-                                    tflag, TX, TY);
+               tflag, TX, TY);
     launch_pdl(k_list_batch, dim3((unsigned)((batch->ntiles + TPB - 1) / TPB)), dim3(TPB), 0, s, batch->nmembers, batch->ntiles, members,
                                                                             clocks, tflag, counters, list_act, list_rec);
     int rc = DCLAW_OK;
