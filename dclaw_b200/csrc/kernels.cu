@@ -102,13 +102,15 @@ constexpr int RECORDS_TPB = DCLAW_RECORDS_TPB;
 constexpr int RECORDS_MINB = DCLAW_PLAIN_CELL_MINB * 256 / DCLAW_RECORDS_TPB;
 
 // Threads per CTA, and resident CTAs the registers are sized for, of the
-// staged per-interface kernels (patch calls, full state), which wait on
-// FP64 latency. Their solves and fluxes need 125-160 registers: CTAs of 256
-// threads left one CTA (8 warps) on an SM as soon as a kernel passed 128.
-// With 128 threads and 128 registers, and tau once per cell, two 1024^2
-// steps of the full state take 1.22 ms (1.68 before) and two 500 x 300
-// rounds of the patch calls 0.39 ms (0.48). 3, 5 and 6 CTAs for the solves
-// and fluxes, and 64 threads, came out 0-6 % slower.
+// staged kernels (patch calls, full state), which wait on FP64 latency. Their
+// solves and fluxes need 125-160 registers: CTAs of 256 threads left one CTA
+// (8 warps) on an SM as soon as a kernel passed 128. With 128 threads and 128
+// registers, and tau once per cell, two 1024^2 steps of the full state went
+// from 1.68 to 1.22 ms and two 500 x 300 rounds of the patch calls from 0.48
+// to 0.39; with both directions in a launch and src2 by itself at 48 registers
+// from 1.157 to 1.105 and from 0.341 to 0.324 (src2 at 4, 6, 8, 10 CTAs: 1.180,
+// 1.140, 1.114, 1.105). 3, 5 and 6 CTAs for the solves and fluxes, and 64
+// threads, came out 0-6 % slower.
 #ifndef DCLAW_STAGE_TPB
 #define DCLAW_STAGE_TPB 128
 #endif
@@ -120,6 +122,9 @@ constexpr int RECORDS_MINB = DCLAW_PLAIN_CELL_MINB * 256 / DCLAW_RECORDS_TPB;
 #endif
 #ifndef DCLAW_STAGE_FINAL_MINB
 #define DCLAW_STAGE_FINAL_MINB 4
+#endif
+#ifndef DCLAW_STAGE_SRC2_MINB
+#define DCLAW_STAGE_SRC2_MINB 10
 #endif
 constexpr int STAGE_TPB = DCLAW_STAGE_TPB;
 
@@ -272,17 +277,25 @@ __global__ void __launch_bounds__(STAGE_TPB) k_taus(dclaw_params P, Work W, doub
     if (idx < (long long)W.npad) cell_taus(P, W.qB, W.npad, (size_t)idx, tau);
 }
 
+// items (of the staged kernels' x and y index spaces) in DIR's solves and fluxes
+__host__ __device__ inline long long solve_items(const Geom& g, int dir) {
+    return dir == 0 ? (long long)(g.mx + 3) * (g.my + 2) : (long long)(g.mx + 2) * (g.my + 3);
+}
+__host__ __device__ inline long long flux_items(const Geom& g, int dir) {
+    return dir == 0 ? (long long)(g.mx + 1) * (g.my + 2) : (long long)(g.mx + 2) * (g.my + 1);
+}
+
+// solve `idx` of direction DIR; the items' Courant numbers are reduced by
+// warps, so every thread of the warp calls it
 template <int DIR>
-__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_riemann(dclaw_params P, Geom g, Work W,
-                                                                              const double* __restrict__ tau,
-                                                                              double dt, dclaw_clock* clk) {
-    pdl_wait();
+__device__ __forceinline__ void staged_solve(const dclaw_params& P, const Geom& g, const Work& W,
+                                             const double* __restrict__ tau, double dt, dclaw_clock* clk,
+                                             long long idx) {
     // DIR 0: rows r = 0..my+1, interfaces i = 0..mx+2 (x fastest)
     // DIR 1: interfaces k = 0..my+2, columns c = 0..mx+1 (column fastest)
     const int nfast = DIR == 0 ? g.mx + 3 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 3;
     const long long n = (long long)nfast * nslow;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double cflv = 0.0;
     if (idx < n) {
         int a, s;
@@ -297,20 +310,37 @@ __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_riemann(d
     warp_max_to(cflv, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
 }
 
-template <int DIR>
-__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_flux(dclaw_params P, Geom g, Work W, double dt) {
+// The x items' CTAs, then the y items' (nx of the first), in one launch: each
+// direction by itself leaves its last wave of CTAs nearly empty.
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_riemann(dclaw_params P, Geom g, Work W,
+                                                                              const double* __restrict__ tau,
+                                                                              double dt, dclaw_clock* clk,
+                                                                              unsigned nx) {
     pdl_wait();
+    if (blockIdx.x < nx) staged_solve<0>(P, g, W, tau, dt, clk, (long long)blockIdx.x * STAGE_TPB + threadIdx.x);
+    else staged_solve<1>(P, g, W, tau, dt, clk, (long long)(blockIdx.x - nx) * STAGE_TPB + threadIdx.x);
+}
+
+template <int DIR>
+__device__ __forceinline__ void staged_flux(const dclaw_params& P, const Geom& g, const Work& W, double dt,
+                                            long long idx) {
     // DIR 0: rows 0..my+1, interfaces 1..mx+1; DIR 1: interfaces 1..my+1, columns 0..mx+1
     const int nfast = DIR == 0 ? g.mx + 1 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 1;
     const long long n = (long long)nfast * nslow;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
     int a, s;
     split_index(idx, nfast, a, s);
     int r = DIR == 0 ? s : a;
     int i = DIR == 0 ? a + 1 : s + 1;
     stage_flux<DIR>(P, g, W, r, i, DIR == 0 ? dt / g.dx : dt / g.dy, nullptr);
+}
+
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_flux(dclaw_params P, Geom g, Work W, double dt,
+                                                                          unsigned nx) {
+    pdl_wait();
+    if (blockIdx.x < nx) staged_flux<0>(P, g, W, dt, (long long)blockIdx.x * STAGE_TPB + threadIdx.x);
+    else staged_flux<1>(P, g, W, dt, (long long)(blockIdx.x - nx) * STAGE_TPB + threadIdx.x);
 }
 
 // ---- the full-state step (segregation, entrainment) -------------------------
@@ -362,14 +392,12 @@ __global__ void __launch_bounds__(TPB) k_full_taudir(dclaw_params P, Geom g, Wor
 }
 
 template <int DIR>
-__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_full_riemann(dclaw_params P, Geom g, WorkF W, dclaw_clock* clk,
-                                                      uint32_t* __restrict__ brlog,
-                                                      const uint32_t* __restrict__ tflag) {
-    pdl_wait();
+__device__ __forceinline__ void full_solve(const dclaw_params& P, const Geom& g, const WorkF& W, dclaw_clock* clk,
+                                           uint32_t* __restrict__ brlog, const uint32_t* __restrict__ tflag,
+                                           long long idx) {
     const int nfast = DIR == 0 ? g.mx + 3 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 3;
     const long long n = (long long)nfast * nslow;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double cflv = 0.0;
     if (idx < n) {
         int a, s;
@@ -401,14 +429,24 @@ __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_full_riem
     warp_max_to(cflv, reinterpret_cast<unsigned long long*>(&clk->cfl_bits));
 }
 
-template <int DIR>
-__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_full_flux(dclaw_params P, Geom g, WorkF W, const dclaw_clock* clk,
-                                                   uint32_t* __restrict__ brlog, const uint32_t* __restrict__ tflag) {
+// both directions in one launch, as k_riemann
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SOLVE_MINB) k_full_riemann(dclaw_params P, Geom g, WorkF W,
+                                                                                   dclaw_clock* clk,
+                                                                                   uint32_t* __restrict__ brlog,
+                                                                                   const uint32_t* __restrict__ tflag,
+                                                                                   unsigned nx) {
     pdl_wait();
+    if (blockIdx.x < nx) full_solve<0>(P, g, W, clk, brlog, tflag, (long long)blockIdx.x * STAGE_TPB + threadIdx.x);
+    else full_solve<1>(P, g, W, clk, brlog, tflag, (long long)(blockIdx.x - nx) * STAGE_TPB + threadIdx.x);
+}
+
+template <int DIR>
+__device__ __forceinline__ void full_flux_item(const dclaw_params& P, const Geom& g, const WorkF& W,
+                                               const dclaw_clock* clk, uint32_t* __restrict__ brlog,
+                                               const uint32_t* __restrict__ tflag, long long idx) {
     const int nfast = DIR == 0 ? g.mx + 1 : g.mx + 2;
     const int nslow = DIR == 0 ? g.my + 2 : g.my + 1;
     const long long n = (long long)nfast * nslow;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
     int a, s;
     split_index(idx, nfast, a, s);
@@ -432,9 +470,15 @@ __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_full_flux(
     }
 }
 
-__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_full_final(dclaw_params P, Geom g, WorkF W, const double* __restrict__ he,
-                                                    double* __restrict__ q_out, dclaw_clock* clk,
-                                                    const uint32_t* __restrict__ tflag);
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FLUX_MINB) k_full_flux(dclaw_params P, Geom g, WorkF W,
+                                                                               const dclaw_clock* clk,
+                                                                               uint32_t* __restrict__ brlog,
+                                                                               const uint32_t* __restrict__ tflag,
+                                                                               unsigned nx) {
+    pdl_wait();
+    if (blockIdx.x < nx) full_flux_item<0>(P, g, W, clk, brlog, tflag, (long long)blockIdx.x * STAGE_TPB + threadIdx.x);
+    else full_flux_item<1>(P, g, W, clk, brlog, tflag, (long long)(blockIdx.x - nx) * STAGE_TPB + threadIdx.x);
+}
 
 // the next dt after the tick rule's choice dtn: clipped at the next
 // observation time (with the tick rule and t_obs > 0), then at t_final
@@ -529,29 +573,49 @@ __device__ __forceinline__ void last_block_tick(const dclaw_params& P, dclaw_clo
     }
 }
 
-// update + src2 of the full state; the tick is a launch of its own (a block
-// that counts itself finished holds its dry warps at a barrier until its wet
-// ones are through src2: 1.25 against 1.22 ms for two steps at 1024^2)
-__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_full_final(dclaw_params P, Geom g, WorkF W, const double* __restrict__ he,
-                                                    double* __restrict__ q_out, dclaw_clock* clk,
-                                                    const uint32_t* __restrict__ tflag) {
+// The full state's update into q_out, then src2 on it, then the tick, a launch
+// each: the update waits on memory (76 loads a cell, 128 registers), src2 on
+// FP64 latency (48 registers), and a block that counts itself finished for
+// the tick holds its dry warps at a barrier until its wet ones are through.
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_full_update(dclaw_params P, Geom g, WorkF W,
+                                                                                  double* __restrict__ q_out,
+                                                                                  dclaw_clock* clk,
+                                                                                  const uint32_t* __restrict__ tflag) {
     pdl_wait();
-    const long long n = (long long)g.mx * g.my;
+    const size_t plane = (size_t)g.mx * g.my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < n) {
-        int i, j;
-        split_index(idx, g.mx, i, j);
-        i += 1;
-        j += 1;
-        if (tflag && !full_any_active(tflag, clk->nsteps + 1u, g, i, i, j, j)) {
-            // a cell of an inactive tile: zero, its eroded depth passed through
-            const size_t plane = (size_t)g.mx * g.my;
-            for (int f = 0; f < F_BDIF; ++f) q_out[(size_t)f * plane + (size_t)idx] = 0.0;
-            q_out[(size_t)F_BDIF * plane + (size_t)idx] = W.qB[(size_t)F_BDIF * W.npad + pidx(g, i, j)];
-        } else if (full_finalize(P, g, W, he, q_out, i, j, clk->dt)) {
-            flag_status(clk, DCLAW_ERR_NAN);
-        }
+    if (idx >= (long long)plane) return;
+    int i, j;
+    split_index(idx, g.mx, i, j);
+    i += 1;
+    j += 1;
+    double qn[NQF];
+    if (tflag && !full_any_active(tflag, clk->nsteps + 1u, g, i, i, j, j)) {
+        // a cell of an inactive tile: zero, its eroded depth passed through
+        for (int f = 0; f < F_BDIF; ++f) qn[f] = 0.0;
+        qn[F_BDIF] = W.qB[(size_t)F_BDIF * W.npad + pidx(g, i, j)];
+    } else if (full_update(g, W, i, j, clk->dt, qn)) {
+        flag_status(clk, DCLAW_ERR_NAN);
     }
+    for (int f = 0; f < NQF; ++f) q_out[(size_t)f * plane + (size_t)idx] = qn[f];
+}
+
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SRC2_MINB) k_full_src2(dclaw_params P, Geom g,
+                                                                               const double* __restrict__ he,
+                                                                               double* __restrict__ q_out,
+                                                                               const dclaw_clock* clk,
+                                                                               const uint32_t* __restrict__ tflag) {
+    pdl_wait();
+    const size_t plane = (size_t)g.mx * g.my;
+    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)plane) return;
+    int i, j;
+    split_index(idx, g.mx, i, j);
+    if (tflag && !full_any_active(tflag, clk->nsteps + 1u, g, i + 1, i + 1, j + 1, j + 1)) return;
+    double q[NQF];
+    for (int f = 0; f < NQF; ++f) q[f] = q_out[(size_t)f * plane + (size_t)idx];
+    src2_cell_full(P, P.phi, clk->dt, q, he ? he[idx] : 0.0);
+    for (int f = 0; f < NQF; ++f) q_out[(size_t)f * plane + (size_t)idx] = q[f];
 }
 
 // One tile of the fused step (all threads of the CTA call it). smem holds
@@ -1545,7 +1609,7 @@ __global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_update_pa
     }
 }
 
-__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_FINAL_MINB) k_src2_padded(dclaw_params P, int mx, int my, double dt, double* q) {
+__global__ void __launch_bounds__(STAGE_TPB, DCLAW_STAGE_SRC2_MINB) k_src2_padded(dclaw_params P, int mx, int my, double dt, double* q) {
     pdl_wait();
     const long long n = (long long)mx * my;
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2218,10 +2282,9 @@ int dclaw_step2(double* q, const double* aux, int mx, int my, int mbc, double dx
     // the tau planes lie where the x-fluxes go after the solves have read them
     double* tau = W.fx;
     launch_pdl(k_taus, dim3(stage_blocks((long long)L.npad)), dim3(STAGE_TPB), 0, s, P, W, tau);
-    launch_pdl(k_riemann<0>, dim3(stage_blocks((long long)L.nxi)), dim3(STAGE_TPB), 0, s, P, g, W, tau, dt, clock);
-    launch_pdl(k_riemann<1>, dim3(stage_blocks((long long)L.nyi)), dim3(STAGE_TPB), 0, s, P, g, W, tau, dt, clock);
-    launch_pdl(k_flux<0>, dim3(stage_blocks((long long)(mx + 1) * (my + 2))), dim3(STAGE_TPB), 0, s, P, g, W, dt);
-    launch_pdl(k_flux<1>, dim3(stage_blocks((long long)(mx + 2) * (my + 1))), dim3(STAGE_TPB), 0, s, P, g, W, dt);
+    const unsigned sx = stage_blocks(solve_items(g, 0)), fx = stage_blocks(flux_items(g, 0));
+    launch_pdl(k_riemann, dim3(sx + stage_blocks(solve_items(g, 1))), dim3(STAGE_TPB), 0, s, P, g, W, tau, dt, clock, sx);
+    launch_pdl(k_flux, dim3(fx + stage_blocks(flux_items(g, 1))), dim3(STAGE_TPB), 0, s, P, g, W, dt, fx);
     launch_pdl(k_update_padded, dim3(stage_blocks((long long)mx * my)), dim3(STAGE_TPB), 0, s, g, W, dt, q, fluxes, clock);
     launch_pdl(k_cfl_from_bits, dim3(1), dim3(32), 0, s, clock);
     return cuda_status();
@@ -2333,11 +2396,13 @@ int dclaw_step_full(const double* q_in, double* q_out, const double* b, const do
     const long long npad = (long long)g.PX * g.PY;
     launch_pdl(k_full_b4, dim3(nblocks(npad)), dim3(TPB), 0, s, P, g, q_in, b, W, clock, tflag);
     launch_pdl(k_full_taudir, dim3(nblocks(npad)), dim3(TPB), 0, s, P, g, W);
-    launch_pdl(k_full_riemann<0>, dim3(stage_blocks((long long)(mx + 3) * (my + 2))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
-    launch_pdl(k_full_riemann<1>, dim3(stage_blocks((long long)(mx + 2) * (my + 3))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
-    launch_pdl(k_full_flux<0>, dim3(stage_blocks((long long)(mx + 1) * (my + 2))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
-    launch_pdl(k_full_flux<1>, dim3(stage_blocks((long long)(mx + 2) * (my + 1))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log, tflag);
-    launch_pdl(k_full_final, dim3(stage_blocks((long long)mx * my)), dim3(STAGE_TPB), 0, s, P, g, W, h_e, q_out, clock, tflag);
+    const unsigned sx = stage_blocks(solve_items(g, 0)), fx = stage_blocks(flux_items(g, 0));
+    launch_pdl(k_full_riemann, dim3(sx + stage_blocks(solve_items(g, 1))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log,
+               tflag, sx);
+    launch_pdl(k_full_flux, dim3(fx + stage_blocks(flux_items(g, 1))), dim3(STAGE_TPB), 0, s, P, g, W, clock, branch_log,
+               tflag, fx);
+    launch_pdl(k_full_update, dim3(stage_blocks((long long)mx * my)), dim3(STAGE_TPB), 0, s, P, g, W, q_out, clock, tflag);
+    launch_pdl(k_full_src2, dim3(stage_blocks((long long)mx * my)), dim3(STAGE_TPB), 0, s, P, g, h_e, q_out, clock, tflag);
     launch_pdl(k_tick, dim3(1), dim3(32), 0, s, P, clock);
     return cuda_status();
 }
