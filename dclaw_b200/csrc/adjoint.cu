@@ -537,10 +537,13 @@ __global__ void __launch_bounds__(256) k_adj_batch_list(BatchArgs a, unsigned in
 }
 
 // pbar[4 m + k] += member m's block partials of its active blocks, summed in
-// a fixed order: thread t takes blocks t, t + BTPB, ... of each stage in
-// turn, all four parameters at once; then the threads in order
-__global__ void __launch_bounds__(BTPB) k_adj_batch_pbar(BatchArgs a, double* __restrict__ pbar) {
-    __shared__ double red[NPB][BTPB];
+// a fixed order: thread t takes blocks t, t + PTPB, ... of each stage in
+// turn, all four parameters at once; then the threads by warps, in order.
+// One CTA a member, a chain of loads: with 1024 threads the reverse chain of a
+// 512^2 step takes 434 us, of a 1024^2 step 1164; with 256, 441 and 1187.
+constexpr int PTPB = 1024;
+__global__ void __launch_bounds__(PTPB) k_adj_batch_pbar(BatchArgs a, double* __restrict__ pbar) {
+    __shared__ double red[NPB][PTPB / 32];
     pdl_wait();
     const int m = blockIdx.x;
     const dclaw_adj_member M = a.mem[m];
@@ -549,19 +552,25 @@ __global__ void __launch_bounds__(BTPB) k_adj_batch_pbar(BatchArgs a, double* __
     const uint32_t* act = (const uint32_t*)(a.work + M.work_off + L.off_act);
     const int nb = L.act_nx * L.act_ny;
     double sum[NPB] = {0.0, 0.0, 0.0, 0.0};
-    for (int p = 0; p < BLK_PBAR_OPS; ++p)
-        for (int b = threadIdx.x; b < nb; b += BTPB)
-            if (act[b]) {
+    for (int b = threadIdx.x; b < nb; b += PTPB)
+        if (act[b]) {
+#pragma unroll
+            for (int p = 0; p < BLK_PBAR_OPS; ++p) {
                 const double* v = part + ((size_t)p * nb + b) * NPB;
 #pragma unroll
                 for (int k = 0; k < NPB; ++k) sum[k] += v[k];
             }
+        }
 #pragma unroll
-    for (int k = 0; k < NPB; ++k) red[k][threadIdx.x] = sum[k];
+    for (int k = 0; k < NPB; ++k) {
+        double v = sum[k];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v;
+    }
     __syncthreads();
     if (threadIdx.x < NPB) {
         double s = 0.0;
-        for (int t = 0; t < BTPB; ++t) s += red[threadIdx.x][t];
+        for (int w = 0; w < PTPB / 32; ++w) s += red[threadIdx.x][w];
         pbar[(size_t)m * NPB + threadIdx.x] += s;
     }
 }
@@ -697,7 +706,7 @@ static int single_adjoint(const double* q_in, const double* b, int mx, int my, d
     BatchArgs a{1, mem, prm, dt, q_in, b, lam_out, lam_in, bbar, base, status};
     launch_block_adjoint(a, (uint32_t)((size_t)L.act_nx * L.act_ny), base + T.off_lists,
                          (unsigned int*)(base + T.off_counts), sm_count_adj(), s, phase);
-    if (phase & PHASE_REVERSE) launch_pdl(k_adj_batch_pbar, dim3(1), dim3(BTPB), 0, s, a, pbar);
+    if (phase & PHASE_REVERSE) launch_pdl(k_adj_batch_pbar, dim3(1), dim3(PTPB), 0, s, a, pbar);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? DCLAW_OK : DCLAW_ERR_CUDA;
 }
@@ -774,7 +783,7 @@ static int batched_adjoint(const dclaw_adj_batch* batch, const dclaw_adj_member*
     char* lists = (char*)work + (batch->work_bytes - 256 - 2 * align256((size_t)batch->nblocks * 8));
     unsigned int* counts = (unsigned int*)((char*)work + (batch->work_bytes - 256));
     launch_block_adjoint(a, batch->nblocks, lists, counts, sm_count_adj(), s, phase);
-    if (phase & PHASE_REVERSE) launch_pdl(k_adj_batch_pbar, dim3((unsigned)batch->nmembers), dim3(BTPB), 0, s, a, pbar);
+    if (phase & PHASE_REVERSE) launch_pdl(k_adj_batch_pbar, dim3((unsigned)batch->nmembers), dim3(PTPB), 0, s, a, pbar);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? DCLAW_OK : DCLAW_ERR_CUDA;
 }
