@@ -1154,9 +1154,10 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_list(dclaw_params 
 // twice, the shallow ones first: the longest of them takes 300 us by itself
 // (5900 cycles a substep, a chain of divisions and roots), and a warp that
 // holds such cells takes no others until they are through. On the 777 x 1024
-// flow in motion two steps take 1.61 ms, 2.28 ms with k_src2_list (with
+// flow in motion two steps took 1.61 ms, 2.28 ms with k_src2_list (with
 // the quadrants' shared evaluations in mp_update_fe4quad; 1.68 ms without
-// them, 1.67 ms without the shallow pass). A queue of wet cells per warp, so
+// them, 1.67 ms without the shallow pass), and take 1.50 ms with the step's
+// later changes. A queue of wet cells per warp, so
 // that it starts 28 of them at once, took 1.80 ms: what is left is latency,
 // and fewer, fuller warps hide less of it.
 #ifndef DCLAW_QUAD_REFILL
