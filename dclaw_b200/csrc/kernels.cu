@@ -530,7 +530,7 @@ __global__ void k_clock_set_obs(dclaw_clock* clk, double t_obs) {
 // Records of every padded cell, and the marks. prow0 / nprow: the padded
 // rows (0 .. my+3 for j = -1 .. my+2) this launch covers, all of them by
 // default.
-template <int MINB>
+template <int MINB, int TX = TILE_X, int TY = TILE_Y>
 __global__ void __launch_bounds__(TPB, MINB) k_records(dclaw_params P, Geom g, const double* __restrict__ q_in,
                                                  const double* __restrict__ b, Rec R, dclaw_clock* clk,
                                                  uint32_t* __restrict__ tflag, int prow0 = 0, int nprow = -1) {
@@ -544,8 +544,7 @@ __global__ void __launch_bounds__(TPB, MINB) k_records(dclaw_params P, Geom g, c
     j += prow0 - 1;
     if (cell_record(P, g, q_in, b, R, i, j)) flag_status(clk, DCLAW_ERR_NAN);
     if (tflag && R.get(R_H, pidx(g, i, j)) > 0.0)
-        mark_tiles(tflag, clk->nsteps + 1u, i, j, TILE_X, TILE_Y, (g.mx + TILE_X - 1) / TILE_X,
-                   (g.my + TILE_Y - 1) / TILE_Y);
+        mark_tiles(tflag, clk->nsteps + 1u, i, j, TX, TY, (g.mx + TX - 1) / TX, (g.my + TY - 1) / TY);
 }
 
 __device__ __forceinline__ void tick_device(const dclaw_params& P, dclaw_clock* clk) {
@@ -774,20 +773,23 @@ __device__ __forceinline__ double tile_body(const dclaw_params& P, const Geom& g
     return cfl;
 }
 
-// One tile with its two sweeps side by side: threads 0..255 take the x-sweep,
-// 256..511 the y-sweep, which read the same state and meet only in the
-// update. One CTA per SM (139 KB, 512 threads at 128 registers), so a tile
+// One tile with its two sweeps side by side: threads 0..G-1 take the x-sweep,
+// G..2G-1 the y-sweep, which read the same state and meet only in the
+// update. One CTA of 14 x 13 per SM (139 KB, 512 threads at 128 registers), so a tile
 // takes one solve and one flux phase instead of two of each, and half as
 // many tiles run at once: for patches whose active tiles leave SMs idle
 // anyway, where a step lasts as long as its longest chain.
-template <int TX, int TY, bool WITH_SRC2>
+template <int TX, int TY, int G, bool WITH_SRC2>
 __device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const Geom& g, const Rec& R,
                                                   const double* __restrict__ b, double* __restrict__ q_out, double dt,
                                                   int i0, int j0, double* smem, bool& nan, double crit) {
     using TG = TileGeom<TX, TY>;
-    static_assert(TX + 1 <= 16 && TY + 1 <= 16 && (TX + 2) * 16 <= 256 && (TY + 2) * 16 <= 256, "half-warp per slice");
+    // lanes of a slice in the flux phase
+    constexpr int LANES = TX + 1 <= 8 && TY + 1 <= 8 ? 8 : 16;
+    static_assert(TX + 1 <= LANES && TY + 1 <= LANES && (TX + 2) * LANES <= G && (TY + 2) * LANES <= G && G % 32 == 0,
+                  "LANES lanes per slice");
     const int tid = threadIdx.x, lane = tid & 31;
-    const int dir = tid >> 8, gt = tid & 255;
+    const int dir = tid / G, gt = tid % G;
     TileMem M;
     M.A = smem + (size_t)dir * NW * TG::NA;
     M.B = smem + (size_t)2 * NW * TG::NA;
@@ -808,13 +810,13 @@ __device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const G
     M.hv = TX + 6;
     bool any = false;
     if (gt == 0) *M.nlist = 0;
-    for (int it = tid; it < TG::NHB; it += 512)
+    for (int it = tid; it < TG::NHB; it += 2 * G)
         if (tile_stage_hb(g, R, b, M, it)) any = true;
     any = __syncthreads_or(any) != 0;
     nan = false;
     if (!any) {
         const size_t plane = (size_t)g.mx * g.my;
-        for (int it = tid; it < TX * TY; it += 512) {
+        for (int it = tid; it < TX * TY; it += 2 * G) {
             int i = i0 + it % TX, j = j0 + it / TX;
             if (i > g.mx || j > g.my) continue;
             size_t c = (size_t)(j - 1) * g.mx + (size_t)(i - 1);
@@ -825,7 +827,7 @@ __device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const G
     const double dtdx = dt / g.dx, dtdy = dt / g.dy, dtd = dir == 0 ? dtdx : dtdy;
     // the items that need a solve, as a dense list (tile_body)
     const int nsolve = dir == 0 ? TG::NXW : TG::NYW;
-    for (int it0 = 0; it0 < nsolve; it0 += 256) {
+    for (int it0 = 0; it0 < nsolve; it0 += G) {
         const int it = it0 + gt;
         bool need = it < nsolve && tile_needs_solve(P, g, M, dir, it, i0, j0, TX);
         if (it < nsolve && !need) {
@@ -841,14 +843,14 @@ __device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const G
     __syncthreads();
     double cfl = 0.0;
     const int nneed = *M.nlist;
-    for (int w = gt; w < nneed; w += 256) {
+    for (int w = gt; w < nneed; w += G) {
         bool ok;
         double s = tile_riemann(P, g, R, M, dir, M.list[w], i0, j0, TX, TY, ok, crit);
         if (ok) cfl = fmax2(cfl, dtd * s);
     }
     __syncthreads();
     {
-        const int sl = gt >> 4, k = gt & 15;
+        const int sl = gt / LANES, k = gt % LANES;
         const int nsl = dir == 0 ? TY + 2 : TX + 2, span = dir == 0 ? TX : TY;
         const int s = (dir == 0 ? j0 : i0) - 1 + sl, a = (dir == 0 ? i0 : j0) + k;
         const int smax = dir == 0 ? g.my + 1 : g.mx + 1, amax = dir == 0 ? g.mx : g.my;
@@ -868,7 +870,7 @@ __device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const G
         }
     }
     __syncthreads();
-    for (int it = tid; it < TX * TY; it += 512)
+    for (int it = tid; it < TX * TY; it += 2 * G)
         if (tile_final<TX, TY, WITH_SRC2, true>(P, g, R, M, it, i0, j0, dt, dtdx, dtdy, q_out)) nan = true;
     if (!(cfl == cfl)) cfl = 0.0;
     return cfl;
@@ -876,8 +878,8 @@ __device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const G
 
 // the tiles of a small patch, one CTA each, with src2; the last CTA applies
 // the tick. A tile not flagged active writes its zeros.
-template <int TX, int TY>
-__global__ void __launch_bounds__(512, 1) k_tile_apart(dclaw_params P, Geom g, Rec R, const double* __restrict__ b,
+template <int TX, int TY, int G, int MINB>
+__global__ void __launch_bounds__(2 * G, MINB) k_tile_apart(dclaw_params P, Geom g, Rec R, const double* __restrict__ b,
                                                        double* __restrict__ q_out, dclaw_clock* clk,
                                                        const uint32_t* __restrict__ tflag) {
     pdl_wait();
@@ -886,10 +888,10 @@ __global__ void __launch_bounds__(512, 1) k_tile_apart(dclaw_params P, Geom g, R
     bool nan = false;
     double cfl = 0.0;
     if (tflag[blockIdx.y * gridDim.x + blockIdx.x] == clk->nsteps + 1u) {
-        cfl = tile_body_apart<TX, TY, true>(P, g, R, b, q_out, clk->dt, i0, j0, smem, nan, critical_root(P));
+        cfl = tile_body_apart<TX, TY, G, true>(P, g, R, b, q_out, clk->dt, i0, j0, smem, nan, critical_root(P));
     } else {
         const size_t plane = (size_t)g.mx * g.my;
-        for (int it = threadIdx.x; it < TX * TY; it += 512) {
+        for (int it = threadIdx.x; it < TX * TY; it += 2 * G) {
             int i = i0 + it % TX, j = j0 + it / TX;
             if (i > g.mx || j > g.my) continue;
             size_t c = (size_t)(j - 1) * g.mx + (size_t)(i - 1);
@@ -1742,6 +1744,20 @@ inline int cuda_status() {
     return e == cudaSuccess ? DCLAW_OK : DCLAW_ERR_CUDA;
 }
 
+// A patch whose 7 x 7 tiles all have a resident place (two CTAs per SM) steps
+// over those: a CTA of six warps that its SM shares with at most one other
+// takes less time for its phases than one of sixteen (solves 10,000 cycles,
+// 14,000 over 14 x 13 tiles, fluxes 7,000 and 8,000 to 11,000; the update with
+// src2, 17,000, is one thread's chain in both), although the halos' solves
+// are 1.3 times as many. A step in us, 14 x 13 and 7 x 7 tiles (share that is
+// wet): 20^2 (0.5) 31.3 and 29.1, 64^2 (0.9) 31.2 and 28.4, 96^2 (0.9) 29.8
+// and 29.3, 120^2 (0.3) 31.4 and 30.6, 120^2 (0.9) 30.8 both, 150^2 (0.9) 32.2
+// and 50.3. With three CTAs per SM (96 registers, spills) 1 us more, with
+// 5 x 5 tiles 29.2 at 64^2 (0.9) and 34.4 at 120^2 (0.9).
+constexpr int TINY_X = 7, TINY_Y = 7, TINY_G = 96, TINY_MINB = 2;
+constexpr auto k_tile_tiny = k_tile_apart<TINY_X, TINY_Y, TINY_G, TINY_MINB>;
+constexpr auto k_tile_small = k_tile_apart<TILE_X, TILE_Y, 256, 1>;
+
 // the tile kernel's dynamic shared memory above 48 KB must be opted into
 // once per device (function attributes belong to the device's context)
 inline int ensure_tile_smem_attr() {
@@ -1757,8 +1773,10 @@ inline int ensure_tile_smem_attr() {
                 cudaFuncSetAttribute(k_tile<TILE_X, TILE_Y, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      bytes) != cudaSuccess ||
                 cudaFuncSetAttribute(k_tile_list, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-                cudaFuncSetAttribute(k_tile_apart<TILE_X, TILE_Y>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)TileGeom<TILE_X, TILE_Y>::SMEM2_BYTES) != cudaSuccess)
+                cudaFuncSetAttribute(k_tile_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)TileGeom<TILE_X, TILE_Y>::SMEM2_BYTES) != cudaSuccess ||
+                cudaFuncSetAttribute(k_tile_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)TileGeom<TINY_X, TINY_Y>::SMEM2_BYTES) != cudaSuccess)
                 return DCLAW_ERR_CUDA;
             done[dev].store(true, std::memory_order_release);
         }
@@ -2045,9 +2063,23 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
     }
     dim3 grid(ntx, nty);
     if (!branch_log) {
-        launch_pdl(k_records<SMALL_RECORDS_MINB>, dim3(small_blocks((long long)L.npad)), dim3(SMALL_RECORDS_TPB), 0, s, P, g,
-                   q_in, b, R, clock, tflag, 0, -1);
-        launch_pdl(k_tile_apart<TILE_X, TILE_Y>, grid, dim3(512), TG::SMEM2_BYTES, s, P, g, R, b, q_out, clock, tflag);
+        const int nsm = sm_count();
+        if (nsm <= 0) return DCLAW_ERR_CUDA;
+        const dim3 rgrid(small_blocks((long long)L.npad));
+        const long long tnx = (mx + TINY_X - 1) / TINY_X, tny = (my + TINY_Y - 1) / TINY_Y;
+        if (tnx * tny <= (long long)nsm * TINY_MINB) {
+            // their flags stand in the place of the state before src2, which
+            // these launches do not use
+            uint32_t* sflag = (uint32_t*)((char*)work + L.off_qstar);
+            launch_pdl(k_records<SMALL_RECORDS_MINB, TINY_X, TINY_Y>, rgrid, dim3(SMALL_RECORDS_TPB), 0, s, P, g, q_in, b,
+                       R, clock, sflag, 0, -1);
+            launch_pdl(k_tile_tiny, dim3((unsigned)tnx, (unsigned)tny), dim3(2 * TINY_G),
+                       TileGeom<TINY_X, TINY_Y>::SMEM2_BYTES, s, P, g, R, b, q_out, clock, sflag);
+            return cuda_status();
+        }
+        launch_pdl(k_records<SMALL_RECORDS_MINB>, rgrid, dim3(SMALL_RECORDS_TPB), 0, s, P, g, q_in, b, R, clock, tflag, 0,
+                   -1);
+        launch_pdl(k_tile_small, grid, dim3(512), TG::SMEM2_BYTES, s, P, g, R, b, q_out, clock, tflag);
         return cuda_status();
     }
     k_records<DCLAW_PLAIN_CELL_MINB><<<nblocks((long long)L.npad), TPB, 0, s>>>(P, g, q_in, b, R, clock, tflag);

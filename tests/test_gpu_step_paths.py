@@ -1,7 +1,7 @@
 """The step's paths against each other, bit for bit.
 
-dclaw_step takes small patches through k_records and k_tile_apart, larger ones
-through the tile lists (src2method 2 always, with k_src2_quad_list), and every
+dclaw_step takes small patches through k_records and k_tile_apart (over 7 x 7
+tiles while all of them have a place on the SMs), larger ones through the tile lists (src2method 2 always, with k_src2_quad_list), and every
 patch with a branch log through the full-grid kernels, which the oracle tests
 cover; the patch calls run the staged kernels. The sizes are those where a path can go
 wrong: the smallest patches, one cell around a tile and around a CTA of the
@@ -72,6 +72,15 @@ def test_small_patch_reports_nan():
     st.init_clock(0.02)
     st.step(1)
     assert st.status() != 0
+
+
+@pytest.mark.parametrize("size", [(7, 7), (8, 6), (6, 15), (50, 48), (119, 119), (119, 126), (2, 2072), (2, 2073)],
+                         ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("k", [0, 2, 3])
+def test_tiny_tiles_equal_full_grid(size, k):
+    """Patches over 7 x 7 tiles: one cell around a tile, and both sides of the
+    296 tiles (two on each of 148 SMs) above which the 14 x 13 ones are taken."""
+    test_step_equals_full_grid(size, k)
 
 
 @pytest.mark.parametrize("size", [(2, 2), (3, 129), (127, 5), (125, 30), (60, 61)], ids=lambda s: f"{s[0]}x{s[1]}")
