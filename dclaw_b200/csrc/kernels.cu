@@ -775,10 +775,10 @@ __device__ __forceinline__ double tile_body(const dclaw_params& P, const Geom& g
 
 // One tile with its two sweeps side by side: threads 0..G-1 take the x-sweep,
 // G..2G-1 the y-sweep, which read the same state and meet only in the
-// update. One CTA of 14 x 13 per SM (139 KB, 512 threads at 128 registers), so a tile
-// takes one solve and one flux phase instead of two of each, and half as
-// many tiles run at once: for patches whose active tiles leave SMs idle
-// anyway, where a step lasts as long as its longest chain.
+// update. One CTA of a 14 x 13 tile per SM (139 KB, 512 threads at 128
+// registers), so a tile takes one solve and one flux phase instead of two of
+// each, and half as many tiles run at once: for patches whose active tiles
+// leave SMs idle anyway, where a step lasts as long as its longest chain.
 template <int TX, int TY, int G, bool WITH_SRC2>
 __device__ __forceinline__ double tile_body_apart(const dclaw_params& P, const Geom& g, const Rec& R,
                                                   const double* __restrict__ b, double* __restrict__ q_out, double dt,
@@ -947,17 +947,18 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_cells(dclaw_params
 }
 
 // ---- single patch over tile lists -------------------------------------------
-// dclaw_step without a branch log: the records, tiles and src2 run only
-// where the flow is. (1) k_scan_patch reads every interior cell's five
-// fields (the NaN check), marks the tiles whose read range holds a wet cell
-// and writes the zero state into q_out; (2) k_list_patch lists the active
-// tiles and the tiles that are active or next to one; (3) k_records_list
-// builds the records of the second list's tiles (every record an active tile
-// reads, once); (4) k_tile_list, a persistent kernel, takes the active tiles
-// from a queue; (5) k_src2_list overwrites the zeros of the active tiles'
-// cells with src2 of the updated state, and its last block applies the tick.
-// Each cell's arithmetic is that of the full-grid kernels, so the results
-// are the same bits; far from the flow a cell costs its 80 bytes of scan.
+// dclaw_step without a branch log, for patches above SMALL_CELLS: the
+// records, tiles and src2 run only where the flow is. (1) k_scan_patch reads
+// every interior cell's five fields (the NaN check) and marks the tiles whose
+// read range holds a wet cell; (2) k_list_patch lists the active tiles and
+// the tiles that are active or next to one; (3) k_records_list builds the
+// records of the second list's tiles (every record an active tile reads,
+// once); (4) k_tile_list, a persistent kernel, takes the active tiles from a
+// queue and writes the zero state into q_out beside them; (5) k_src2_list
+// overwrites the zeros of the active tiles' cells with src2 of the updated
+// state, and its last block applies the tick. Each cell's arithmetic is that
+// of the full-grid kernels, so the results are the same bits; far from the
+// flow a cell costs its 40 bytes of scan and 40 of zeros.
 // cells [s0, s1) are scanned (linear interior indices; the whole patch for
 // dclaw_step, a row range and the rows within 3 of it for dclaw_step_rows)
 __global__ void __launch_bounds__(TPB, PATCH_SCAN_MINB) k_scan_patch(dclaw_params P, int mx, int my,
@@ -1226,7 +1227,7 @@ __global__ void __launch_bounds__(DCLAW_QUAD_TPB, DCLAW_QUAD_MINB) k_src2_quad_l
                 if (i <= g.mx && j <= g.my) {
                     c = (size_t)(j - 1) * g.mx + (size_t)(i - 1);
                     double a = q_star[c];
-                    // a dry cell keeps the zeros k_scan_patch wrote
+                    // a dry cell keeps the zeros k_tile_list wrote
                     if (!(a <= P.dry_tolerance) && (a > QUAD_SHALLOW * P.dry_tolerance) == deep) {
                         double b = q_star[plane + c], d = q_star[2 * plane + c], e = q_star[3 * plane + c],
                                f = q_star[4 * plane + c];
@@ -2221,9 +2222,9 @@ int dclaw_step_rows(const double* q_in, double* q_out, const double* b, int mx, 
     double* qstar = (double*)((char*)work + L.off_qstar);
     // dclaw_step's kernels over tile lists, restricted to the range: the scan
     // of its rows and the 3 either side (the cells its tiles' marks depend
-    // on; the range's rows of q_out are zeroed), the active tiles of its
-    // tile rows, the records of those and their neighbours (one tile row
-    // beyond, 13 >= 3 rows), the tiles, their cells' src2; no tick
+    // on), the active tiles of its tile rows, the records of those and their
+    // neighbours (one tile row beyond, 13 >= 3 rows), the tiles with the
+    // zeros of the range's rows of q_out, their cells' src2; no tick
     const int sm = sm_count();
     if (sm <= 0) return DCLAW_ERR_CUDA;
     unsigned int* counters = (unsigned int*)((char*)work + L.off_counters);

@@ -5,7 +5,7 @@ particle, each with its own material parameters, batched with jax.vmap
 (gradient_particle_filter/pf_flume/flume_model.py:129-179,
 pf_flume/inference.py:96-108). `EnsembleStepper` advances an ensemble of
 patches of uneven sizes, each with its own parameters and its own adaptive
-dt, with one set of three persistent-kernel launches per ensemble step
+dt, with six launches per ensemble step
 (`dclaw_step_batched`), optionally replayed from a captured CUDA graph. The
 tile shape and the persistent grid are chosen by `autotune()`, which times
 the candidates on the ensemble itself (all candidates give the same bits).

@@ -201,7 +201,7 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
  *                    otherwise).
  * With hchi = bdif = 0 and both options off it returns dclaw_step's bits for
  * the first five fields. work holds dclaw_step_full_workspace_bytes(mx, my);
- * branch_log as for dclaw_step. One launch per stage (seven). */
+ * branch_log as for dclaw_step. Seven launches. */
 int dclaw_step_full(const double* q_in, double* q_out, const double* b, const double* h_e, int mx, int my,
                     double dx, double dy, const dclaw_params* p, dclaw_clock* clock, void* work,
                     size_t work_bytes, uint32_t* branch_log, void* stream);
@@ -293,7 +293,7 @@ int dclaw_step_host_bands(int mx, int my, int nbands, int32_t* first, int max);
  * read, those records, a persistent kernel pulling the active tiles of
  * every member from one work queue, src2, each member's tick), so a
  * sequence of ensemble steps captures into one CUDA graph. Tiles with no wet
- * cell within 3 cells are skipped (src2 writes their zeros).
+ * cell within 3 cells are skipped (the scan writes their zeros).
  * Member m's state is 5 planes [5][my][mx] at q_off in the state arenas; its
  * bed is [my][mx] at b_off in the bed arena. */
 typedef struct dclaw_member {
@@ -388,7 +388,7 @@ int dclaw_step_adjoint_reverse(const double* q_in, const double* b, int mx, int 
  * The reference differentiates its particle filters member by member with
  * jax.jacfwd / jax.grad under jax.vmap (gradient_particle_filter/pf_flume/
  * inference.py:96-108). Here the adjoint of one step of every member of an
- * ensemble of uneven patches runs as one sequence of 20 launches that work
+ * ensemble of uneven patches runs as one sequence of 16 launches that work
  * only where members are wet: a scan marks each member's 16 x 16 activity
  * blocks (a wet cell within 4), a list kernel gathers the active blocks and
  * the blocks beside them, the forward recompute and the zeroing of the
