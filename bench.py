@@ -51,11 +51,11 @@ NCU_STEP = {
                "--warmup 3 --e2e-steps 0 --no-cpu-baseline --ensemble-members 0 --grad-steps 0 "
                "--bgrad-members 0 --full-steps 0 --variant-steps 0",
     "kernels": {  # name: (DRAM bytes, warp instructions) per launch, the mean of the 6 launches
-        "k_scan_patch": (1295.4e6, 56.82e6),
-        "k_list_patch": (0.4e6, 0.59e6),
-        "k_records_list": (839.8e6, 276.57e6),
-        "k_tile_list": (754.6e6, 1410.10e6),
-        "k_src2_list": (325.6e6, 372.82e6),
+        "k_scan_patch": (671.5e6, 42.54e6),
+        "k_list_patch": (0.4e6, 0.61e6),
+        "k_records_list": (737.0e6, 230.28e6),
+        "k_tile_list": (1450.7e6, 1314.44e6),
+        "k_src2_list": (310.0e6, 368.87e6),
     },
     # k_tile_list, --set full on the 2048^2 case: active lanes per warp
     # instruction, FP64 pipe active
