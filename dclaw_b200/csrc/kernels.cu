@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_cells(dclaw_params
 }
 
 // ---- single patch over tile lists -------------------------------------------
-// dclaw_step without a branch log, for patches above SMALL_CELLS: the
+// dclaw_step without a branch log, where small_patch does not hold: the
 // records, tiles and src2 run only where the flow is. (1) k_scan_patch reads
 // every interior cell's five fields (the NaN check) and marks the tiles whose
 // read range holds a wet cell; (2) k_list_patch lists the active tiles and
@@ -1785,20 +1785,30 @@ inline int ensure_tile_smem_attr() {
     return DCLAW_OK;
 }
 
-// Patches up to this many cells step in two launches, k_records over every
-// padded cell and k_tile_apart over every tile (src2method 2 keeps the lists:
-// its lanes take cells from them). Their active tiles do not fill the SMs, so
-// a step lasts as long as its longest chain, which the lists' three more
-// launches and the tile's two sweeps in turn lengthen. A step over the lists
-// against this, in us (share of the patch that is wet): 64^2 (0.2) 55.8 and
-// 34.0, 200^2 (0.5) 61.5 and 37.0, 333 x 200 (0.3) 63.5 and 47.2, 316^2 (0.9)
-// 91.0 and 80.9, 350^2 (0.3) 64.3 and 65.3, 350^2 (0.9) 95 and 102,
-// 512^2 (0.1) 61 and 73. The records take 84 registers there, without the
-// spills that pay where occupancy counts.
-#ifndef DCLAW_SMALL_CELLS
-#define DCLAW_SMALL_CELLS 100000
-#endif
-constexpr long long SMALL_CELLS = DCLAW_SMALL_CELLS;
+// Patches of few tiles step in two launches, k_records over every padded cell
+// and k_tile_apart over every tile (src2method 2 keeps the lists: its lanes
+// take cells from them). Their active tiles do not fill the SMs, so a step
+// lasts as long as its longest chain, which the lists' three more launches
+// and the tile's two sweeps in turn lengthen. The line is drawn in 14 x 13
+// tiles, of which k_tile_apart has one on an SM, so in rounds: up to four for
+// patches at least two tiles wide, up to three for those one tile wide, whose
+// narrow tiles take the list's phases fewer passes of their threads but
+// k_tile_apart's one either way. A step of a replayed graph over the lists
+// against this, in us, on 148 SMs (tiles; share of the patch that is wet):
+// 200^2 (240; 0.31) 58.0 and 37.0, 294 x 273 (441; 0.62) 88.9 and 77.4, 316^2
+// (575; 0.15, 0.62) 53.8 and 36.6, 90.3 and 81.0, 224 x 481 (592; 0.13, 0.30,
+// 0.58) 62.2 and 39.8, 59.4 and 60.0, 93.8 and 91.0, 20 x 3845 (592; 0.53) 99.3 and 106.5,
+// 350^2 (675; 0.62) 94.7 and 100.8, 20 x 5000 (770; 0.53) 129.7 and 130.2;
+// one tile wide: 5 x 5720 (440; 0.31) 87.9 and 82.4, 14 x 5720 (440; 0.31) 96.7 and 86.0,
+// 7 x 6000 (462; 0.3, 0.9) 70.1 and 58.9, 79.9 and 89.6, 14 x 7696 (592; 0.53) 102.2 and 114.2,
+// 8288 x 5 (592; 0.31) 87.5 and 103.2, 5 x 20000 (1539; 0.31) 192.4 and 231.1.
+// The records take 84 registers there, without the spills that pay where
+// occupancy counts.
+constexpr int SMALL_ROUNDS = 4, SMALL_ROUNDS_NARROW = 3;
+inline bool small_patch(int ntx, int nty, int src2method, int nsm) {
+    const int rounds = ntx == 1 || nty == 1 ? SMALL_ROUNDS_NARROW : SMALL_ROUNDS;
+    return src2method != 2 && (long long)ntx * nty <= (long long)rounds * nsm;
+}
 constexpr int SMALL_RECORDS_MINB = 2, SMALL_RECORDS_TPB = 128;
 inline unsigned small_blocks(long long n) { return (unsigned)((n + SMALL_RECORDS_TPB - 1) / SMALL_RECORDS_TPB); }
 
@@ -2032,12 +2042,11 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
     }
     uint32_t* tflag = (uint32_t*)((char*)work + L.off_tflag);
     const int ntx = (mx + TILE_X - 1) / TILE_X, nty = (my + TILE_Y - 1) / TILE_Y;
-    const bool small = (long long)mx * my <= SMALL_CELLS && p->src2method != 2;
-    if (!branch_log && !small) {
+    const int nsm = sm_count();
+    if (nsm <= 0) return DCLAW_ERR_CUDA;
+    if (!branch_log && !small_patch(ntx, nty, p->src2method, nsm)) {
         // over the tile lists (the branch log needs every interface's bits,
         // so it keeps the full-grid kernels at the end)
-        const int nsm = sm_count();
-        if (nsm <= 0) return DCLAW_ERR_CUDA;
         unsigned int* counters = (unsigned int*)((char*)work + L.off_counters);
         uint32_t* list_act = (uint32_t*)((char*)work + L.off_list_act);
         uint32_t* list_rec = (uint32_t*)((char*)work + L.off_list_rec);
@@ -2064,8 +2073,6 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
     }
     dim3 grid(ntx, nty);
     if (!branch_log) {
-        const int nsm = sm_count();
-        if (nsm <= 0) return DCLAW_ERR_CUDA;
         const dim3 rgrid(small_blocks((long long)L.npad));
         const long long tnx = (mx + TINY_X - 1) / TINY_X, tny = (my + TINY_Y - 1) / TINY_Y;
         if (tnx * tny <= (long long)nsm * TINY_MINB) {
