@@ -84,6 +84,9 @@ class EnsembleStepper:
         self.qa = torch.zeros(self.batch.q_doubles, dtype=torch.float64, device=self.device)
         self.qb = torch.zeros_like(self.qa)
         self.bed = torch.zeros(self.batch.b_doubles, dtype=torch.float64, device=self.device)
+        # (copy_ would broadcast a smaller tensor over the arena)
+        if q is not None and q.shape != self.qa.shape:
+            raise ValueError(f"q must be the ensemble's state arena, shape {tuple(self.qa.shape)}")
         if bed is not None and bed.shape != self.bed.shape:
             raise ValueError(f"bed must be the ensemble's bed arena, shape {tuple(self.bed.shape)}")
         for k, m in enumerate(members):
