@@ -48,10 +48,6 @@ static std::mutex g_setup_mu;
 #ifndef DCLAW_TILE_MINBLOCKS
 #define DCLAW_TILE_MINBLOCKS 2
 #endif
-// src2 in its own per-cell kernel (1) or as the tile kernel's last phase (0)
-#ifndef DCLAW_SRC2_KERNEL
-#define DCLAW_SRC2_KERNEL 1
-#endif
 constexpr int TILE_X = DCLAW_TILE_X, TILE_Y = DCLAW_TILE_Y;
 // resident blocks per SM the ensemble's streaming scan is sized for
 #ifndef DCLAW_SCAN_MINB
@@ -2091,16 +2087,11 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
         return cuda_status();
     }
     k_records<DCLAW_PLAIN_CELL_MINB><<<nblocks((long long)L.npad), TPB, 0, s>>>(P, g, q_in, b, R, clock, tflag);
-    if (DCLAW_SRC2_KERNEL) {
-        double* qstar = (double*)((char*)work + L.off_qstar);
-        launch_pdl(k_tile<TILE_X, TILE_Y, false>, grid, dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock,
-                   branch_log, tflag, 0);
-        launch_pdl(k_src2_cells, dim3(src2_blocks((long long)mx * my)), dim3(SRC2_TPB), 0, s, P, g, qstar, q_out, clock,
-                   tflag, 0ll, -1ll, 1);
-    } else {
-        launch_pdl(k_tile<TILE_X, TILE_Y, true>, grid, dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, q_out, clock,
-                   branch_log, tflag, 0);
-    }
+    double* qstar = (double*)((char*)work + L.off_qstar);
+    launch_pdl(k_tile<TILE_X, TILE_Y, false>, grid, dim3(TILE_TPB), TG::SMEM_BYTES, s, P, g, R, b, qstar, clock,
+               branch_log, tflag, 0);
+    launch_pdl(k_src2_cells, dim3(src2_blocks((long long)mx * my)), dim3(SRC2_TPB), 0, s, P, g, qstar, q_out, clock,
+               tflag, 0ll, -1ll, 1);
     return cuda_status();
 }
 
