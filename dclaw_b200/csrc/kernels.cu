@@ -1352,8 +1352,7 @@ __global__ void __launch_bounds__(TPB, DCLAW_SCAN_MINB) k_scan_batch(int nmem, u
                                                     unsigned int* counters, uint32_t* __restrict__ tflag, int TX,
                                                     int TY) {
     pdl_wait();
-    // tile queue, list lengths, src2method 2's cell counter
-    if (blockIdx.x == 0 && threadIdx.x < 6) counters[threadIdx.x] = 0u;
+    if (blockIdx.x == 0 && threadIdx.x < 3) counters[threadIdx.x] = 0u;  // tile queue and list lengths
     int m = -1;
     for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         m = member_of(nmem, nchunks, ch, m, [&](int k) { return mem[k].schunk0; });
