@@ -7,8 +7,9 @@
 // theta = (phi [rad], kref, alpha_c, mu). The step's dt is data.
 //
 // One call (a single patch, or every member of an ensemble) is 16
-// launches that work only where the flow is (see "ensembles" below: a
-// single patch runs as a one-member ensemble, after a set-up launch):
+// launches, 15 up to PAIR_SOLVES_BLOCKS blocks, that work only where the flow
+// is (see "ensembles" below: a single patch runs as a one-member ensemble,
+// after a set-up launch):
 //   forward recompute  b4step2, calc_taudir, setvars records of the rpn2
 //                      states (tau and its partial derivatives, once per
 //                      cell at rest instead of once per interface side),
@@ -91,8 +92,8 @@ __host__ __device__ inline AdjLayout adj_layout(int mx, int my) {
     L.off_sv = o; o += align256((size_t)NSV * L.S.npad * 8);
     L.act_nx = (mx + 4 + ACT_TILE - 1) / ACT_TILE;
     L.act_ny = (my + 4 + ACT_TILE - 1) / ACT_TILE;
-    // block partials: per 128-item chunk (single patch) or per activity
-    // block and reverse stage (ensembles), whichever needs more
+    // parameter partials, per activity block and reverse stage (the room is
+    // for a partial per ATPB items too, more for patches of a few blocks)
     const long long nbp = 4LL * L.act_nx * L.act_ny;
     L.off_part = o; o += align256((size_t)(L.nparts > nbp ? L.nparts : nbp) * NPB * 8);
     L.off_act = o; o += align256((size_t)L.act_nx * L.act_ny * 4);
@@ -179,7 +180,7 @@ struct BatchArgs {
 //   5. k_adj_batch_pbar   each member's block partials, in block order.
 // Items are the ones the single-patch stages run; each writes its own slots,
 // so lam_in equals dclaw_step_adjoint member by member, bit for bit, and the
-// parameter adjoints agree to rounding (summed per block, not per chunk).
+// parameter adjoints agree to rounding.
 constexpr int BLK_PBAR_OPS = 4;   // src2, x solves, y solves, calc_taudir
 
 __device__ __forceinline__ void batch_member_work(const BatchArgs& a, const dclaw_adj_member& M, AdjLayout& L, Work& W,
@@ -408,7 +409,10 @@ __device__ __forceinline__ void block_stage(const BatchArgs& a, int m, const dcl
 // most, and two codes of theirs at once miss the instruction cache: they are
 // paired up to PAIR_SOLVES_BLOCKS blocks (128^2, 81: 128 us, 156 in two
 // launches; 333 x 200, 273: 220 and 223), not above (512^2, 1089: 442 and
-// 433; 1024^2: 1204 and 1168).
+// 433; 1024^2: 1204 and 1168). Ensembles of channels, about 0.6 of their
+// blocks active, whose reverse chains take, paired and not: 54 blocks 112 and
+// 129 us, 234 198 and 193, 408 225 and 215, 476 310 and 335, 594 338 and 346.
+// The host knows all the blocks, not the active ones the stages run over.
 constexpr uint32_t PAIR_SOLVES_BLOCKS = 600;
 template <int OP, int OP2 = OP>
 __global__ void __launch_bounds__(BTPB, BlkMinB<OP>::value) k_adj_blocks(BatchArgs a, const uint64_t* __restrict__ list,
@@ -666,8 +670,7 @@ int dclaw_adjoint_supported(const dclaw_params* p) {
     if (!p) return DCLAW_ERR_ARG;
     int rc = dclaw_params_check_5(p);
     if (rc) return rc;
-    // no adjoint form: the rare-wave corrector's branch structure and
-    // src2method 2's data-dependent substeps
+    // no adjoint form: src2method 2's data-dependent substeps
     if (p->src2method == 2) return DCLAW_ERR_UNSUPPORTED;
     return DCLAW_OK;
 }

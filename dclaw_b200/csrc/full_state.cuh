@@ -539,7 +539,9 @@ DC_BIG void src2_cell_full(const dclaw_params& P, double phi, double dt, double 
     q[F_H] = h; q[F_HU] = hu; q[F_HV] = hv; q[F_HM] = hm; q[F_PB] = p; q[F_HCHI] = hchi;
 }
 
-// Stage E: update + src2, written to q_out (interior layout, NQF planes)
+// Stage E: update + src2, written to q_out (interior layout, NQF planes): what
+// k_full_update and k_full_src2 do to a cell of an active tile in two launches,
+// in one call for the host build
 DC_HD bool full_finalize(const dclaw_params& P, const Geom& g, const WorkF& W, const double* __restrict__ he,
                          double* __restrict__ q_out, int i, int j, double dt) {
     double qn[NQF];

@@ -1837,7 +1837,8 @@ constexpr int MAX_HOST_BANDS = 64;
 
 inline int host_auto_bands(int mx, int my) {
     const int nty = (my + TILE_Y - 1) / TILE_Y;
-    // About 4 MB of state per band up to 10 bands, then about 28 MB: enough
+    // Bands of about 4 MB of state up to ten of them, ten bands until they
+    // are 28 MB each (280 MB of state), then bands of about 28 MB: enough
     // work per band to pay for its launches and copies, fine enough that the
     // first upload and the last download (the parts that do not overlap)
     // stay short. 512^2 in 1, 3, 6 bands takes 0.55, 0.40, 0.47 ms; 1024^2
@@ -2480,8 +2481,9 @@ int dclaw_step_noalloc(const double* q_in, double* q_out, const double* b, int m
     }
     if (ensure_tile_smem_attr() != DCLAW_OK) return DCLAW_ERR_CUDA;
     // every record plane a tile reads is written by k_records in the same
-    // call (h, fsphi and taudir for every padded cell, the other planes for
-    // every wet cell, the only cells whose other planes are read), so the
+    // call (h for every padded cell; of the wet ones all but static friction's
+    // planes; fsphi and taudir for every cell at rest or dry, tau for those
+    // at rest, the only cells whose planes of these are read), so the
     // previous call's contents need no clearing
     cudaStream_t s = (cudaStream_t)stream;
     Geom g{mx, my, mx + 4, my + 4, dx, dy};

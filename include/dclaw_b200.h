@@ -388,16 +388,15 @@ int dclaw_step_adjoint_reverse(const double* q_in, const double* b, int mx, int 
  * The reference differentiates its particle filters member by member with
  * jax.jacfwd / jax.grad under jax.vmap (gradient_particle_filter/pf_flume/
  * inference.py:96-108). Here the adjoint of one step of every member of an
- * ensemble of uneven patches runs as one sequence of 16 launches that work
- * only where members are wet: a scan marks each member's 16 x 16 activity
+ * ensemble of uneven patches runs as one sequence of 16 launches (15 up to
+ * 600 activity blocks in all) that work only where members are wet: a scan marks each member's 16 x 16 activity
  * blocks (a wet cell within 4), a list kernel gathers the active blocks and
  * the blocks beside them, the forward recompute and the zeroing of the
  * reverse planes run over the second list and the reverse stages over the
  * first, each a grid-stride loop of one CTA per listed block. Each member
  * has its own parameters, dt and parameter adjoints; member k's lam_in
  * equals dclaw_step_adjoint's on member k alone bit for bit, and its
- * parameter adjoints agree to rounding (the block sums are grouped by
- * activity block, not by 128-item chunk).
+ * parameter adjoints agree to rounding.
  * Item spaces (chunk0 / nchunk index): 0 padded cells, 1 interior cells,
  * 2 x-interface solves, 3 y-interface solves, 4 x-interface fluxes, 5 y-interface
  * fluxes. */
