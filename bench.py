@@ -59,8 +59,8 @@ NCU_STEP = {
     },
     # k_tile_list, --set full on the 2048^2 case: active lanes per warp
     # instruction, FP64 pipe active
-    "k_tile_list_lanes": 20.74,
-    "k_tile_list_fp64_pipe": 0.303,
+    "k_tile_list_lanes": 20.87,
+    "k_tile_list_fp64_pipe": 0.293,
 }
 SMS, SCHEDULERS_PER_SM = 148, 4
 METRIC = "cell-updates/sec on 1 B200 (plain vs batched); gradient/forward time ratio"

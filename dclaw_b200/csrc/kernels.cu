@@ -1,10 +1,11 @@
 // kernels.cu -- CUDA kernels (sm_100a, FP64) and the C ABI of include/dclaw_b200.h.
 //
-// One launch per stage of stages.cuh, all on the caller's stream, all
-// reading dt from the device-resident clock so that a sequence of steps can
-// be captured in a CUDA graph. The Courant number is max-reduced with warp
-// shuffles, one shared-memory pass per block and one 64-bit atomicMax per
-// block on the order-preserving bit pattern of a non-negative double.
+// The steps over tiles (tile.cuh) and the staged kernels (stages.cuh,
+// full_state.cuh), all on the caller's stream, the steps reading dt from the
+// device-resident clock so that a sequence of them can be captured in a CUDA
+// graph. The Courant number is max-reduced with warp shuffles and a 64-bit
+// atomicMax on the order-preserving bit pattern of a non-negative double, one
+// per block after a shared-memory pass or one per warp.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>
@@ -1156,9 +1157,12 @@ __global__ void __launch_bounds__(SRC2_TPB, SRC2_MINB) k_src2_list(dclaw_params 
 // flow in motion two steps took 1.61 ms, 2.28 ms with k_src2_list (with
 // the quadrants' shared evaluations in mp_update_fe4quad; 1.68 ms without
 // them, 1.67 ms without the shallow pass), and take 1.50 ms with the step's
-// later changes. A queue of wet cells per warp, so
-// that it starts 28 of them at once, took 1.80 ms: what is left is latency,
-// and fewer, fuller warps hide less of it.
+// later changes. Cells at rest take one substep each, which k_src2_list's 40
+// warps an SM do faster: a step of 1024 x 1024 of them 777 us against 734 (a
+// mass in motion over 0.3 and over 0.8 of that patch: 409 against 477, 757
+// against 820). A queue of wet cells per warp, so that it starts 28 of them at
+// once, took 1.80 ms: what is left is latency, and fewer, fuller warps hide
+// less of it.
 #ifndef DCLAW_QUAD_REFILL
 #define DCLAW_QUAD_REFILL 16
 #endif
