@@ -1784,29 +1784,31 @@ inline int ensure_tile_smem_attr() {
     return DCLAW_OK;
 }
 
-// Patches of few tiles step in two launches, k_records over every padded cell
-// and k_tile_apart over every tile (src2method 2 keeps the lists: its lanes
-// take cells from them). Their active tiles do not fill the SMs, so a step
-// lasts as long as its longest chain, which the lists' three more launches
-// and the tile's two sweeps in turn lengthen. The line is drawn in 14 x 13
-// tiles, of which k_tile_apart has one on an SM, so in rounds: up to four for
-// patches at least two tiles wide, up to three for those one tile wide, whose
-// narrow tiles take the list's phases fewer passes of their threads but
-// k_tile_apart's one either way. A step of a replayed graph over the lists
-// against this, in us, on 148 SMs (tiles; share of the patch that is wet):
-// 200^2 (240; 0.31) 58.0 and 37.0, 294 x 273 (441; 0.62) 88.9 and 77.4, 316^2
-// (575; 0.15, 0.62) 53.8 and 36.6, 90.3 and 81.0, 224 x 481 (592; 0.13, 0.30,
-// 0.58) 62.2 and 39.8, 59.4 and 60.0, 93.8 and 91.0, 20 x 3845 (592; 0.53) 99.3 and 106.5,
-// 350^2 (675; 0.62) 94.7 and 100.8, 20 x 5000 (770; 0.53) 129.7 and 130.2;
-// one tile wide: 5 x 5720 (440; 0.31) 87.9 and 82.4, 14 x 5720 (440; 0.31) 96.7 and 86.0,
-// 7 x 6000 (462; 0.3, 0.9) 70.1 and 58.9, 79.9 and 89.6, 14 x 7696 (592; 0.53) 102.2 and 114.2,
-// 8288 x 5 (592; 0.31) 87.5 and 103.2, 5 x 20000 (1539; 0.31) 192.4 and 231.1.
-// The records take 84 registers there, without the spills that pay where
-// occupancy counts.
-constexpr int SMALL_ROUNDS = 4, SMALL_ROUNDS_NARROW = 3;
-inline bool small_patch(int ntx, int nty, int src2method, int nsm) {
+// Patches up to SMALL_CELLS cells and few tiles step in two launches, k_records
+// over every padded cell and k_tile_apart over every tile (src2method 2 keeps
+// the lists: its lanes take cells from them). Their active tiles do not fill
+// the SMs, so a step lasts as long as its longest chain, which the lists' three
+// more launches and the tile's two sweeps in turn lengthen. k_tile_apart has
+// one tile on an SM and so costs the rounds of active tiles, where the lists
+// have two: five rounds of them are where it no longer gains, three for a patch
+// one tile wide, whose narrow tiles take the list's phases fewer passes of
+// their threads but k_tile_apart's one either way. A step of a replayed graph
+// over the lists against this, in us, on 148 SMs (tiles; share of the patch that
+// is wet): 200^2 (240; 0.31) 58.0 and 37.0, 294 x 273 (441; 0.62) 88.9 and
+// 77.4, 316^2 (575; 0.15, 0.62) 53.8 and 36.6, 90.3 and 81.0, 100 x 1000 (616;
+// 0.1, 0.9) 65.1 and 61.4, 105.3 and 111.7, 20 x 5000 (770; 0.3, 0.9) 86.1 and
+// 93.0, 112.3 and 132.5. Above the cells' line, where tiles are whole: 224 x 481
+// (592; 0.13, 0.9, 1) 62.2 and 39.8, 88.3 and 98.5, 76.9 and 94.1, 350^2 (675;
+// 0.62) 94.7 and 100.8. One tile wide: 5 x 5720 (440; 0.31) 87.9 and 82.4, 14 x
+// 5700 (439; 1) 77.6 and 75.6, 7 x 6000 (462; 0.3, 0.9) 70.1 and 58.9, 79.9 and
+// 89.6, 14 x 7696 (592; 0.53) 102.2 and 114.2, 8288 x 5 (592; 0.31) 87.5 and
+// 103.2, 5 x 20000 (1539; 0.31) 192.4 and 231.1. The records take 84 registers
+// there, without the spills that pay where occupancy counts.
+constexpr long long SMALL_CELLS = 100000;
+constexpr int SMALL_ROUNDS = 5, SMALL_ROUNDS_NARROW = 3;
+inline bool small_patch(int mx, int my, int ntx, int nty, int src2method, int nsm) {
     const int rounds = ntx == 1 || nty == 1 ? SMALL_ROUNDS_NARROW : SMALL_ROUNDS;
-    return src2method != 2 && (long long)ntx * nty <= (long long)rounds * nsm;
+    return src2method != 2 && (long long)mx * my <= SMALL_CELLS && (long long)ntx * nty <= (long long)rounds * nsm;
 }
 constexpr int SMALL_RECORDS_MINB = 2, SMALL_RECORDS_TPB = 128;
 inline unsigned small_blocks(long long n) { return (unsigned)((n + SMALL_RECORDS_TPB - 1) / SMALL_RECORDS_TPB); }
@@ -2044,7 +2046,7 @@ int dclaw_step(const double* q_in, double* q_out, const double* b, int mx, int m
     const int ntx = (mx + TILE_X - 1) / TILE_X, nty = (my + TILE_Y - 1) / TILE_Y;
     const int nsm = sm_count();
     if (nsm <= 0) return DCLAW_ERR_CUDA;
-    if (!branch_log && !small_patch(ntx, nty, p->src2method, nsm)) {
+    if (!branch_log && !small_patch(mx, my, ntx, nty, p->src2method, nsm)) {
         // over the tile lists (the branch log needs every interface's bits,
         // so it keeps the full-grid kernels at the end)
         unsigned int* counters = (unsigned int*)((char*)work + L.off_counters);

@@ -1,9 +1,9 @@
 """The line between the step's two-launch path and its tile lists.
 
-It is drawn in 14 x 13 tiles: a patch at least two tiles wide leaves the
-two-launch path above four tiles an SM, one a single tile wide above three.
-Drawn in cells it left thin patches, which have many tiles for their cells, on
-a path that was a fifth slower for them.
+A patch leaves the two-launch path above 100 000 cells, above five 14 x 13
+tiles an SM, and where it is one tile wide above three. Drawn in cells alone the
+line left thin patches, which have many tiles for their cells, on a path that
+was a fifth slower for them.
 """
 import pytest
 import torch
@@ -31,22 +31,22 @@ def launches_per_step(st):
     return n // 2
 
 
-def tiles(shape, nsm):
-    """(mx, my) of `shape` on either side of its line on nsm SMs."""
-    name, over = shape
+def line_size(name, over, nsm):
+    """(mx, my) at the line on nsm SMs, or (over = 1) one cell beyond it."""
     return {
         "column": (5, TY * 3 * nsm + over),
         "full column": (TX, TY * 3 * nsm + over),
         "row": (TX * 3 * nsm + over, 3),
-        "two columns": (TX + 1, TY * 2 * nsm + over),
-        "four columns": (4 * TX, TY * nsm + over),
+        "two columns": (TX + 1, TY * (5 * nsm // 2) + over),
+        "two rows": (TX * (5 * nsm // 2) + over, TY + 1),
+        "cells": (316 + over, 316),
     }[name]
 
 
 @pytest.mark.parametrize("over", [0, 1])
-@pytest.mark.parametrize("name", ["column", "full column", "row", "two columns", "four columns"])
-def test_line_in_tiles(name, over):
-    mx, my = tiles((name, over), torch.cuda.get_device_properties(0).multi_processor_count)
+@pytest.mark.parametrize("name", ["column", "full column", "row", "two columns", "two rows", "cells"])
+def test_line(name, over):
+    mx, my = line_size(name, over, torch.cuda.get_device_properties(0).multi_processor_count)
     p = DClawParams()
     q, b = flow(mx, my, p, seed=6)
     q, b = torch.tensor(q, device="cuda"), torch.tensor(b, device="cuda")
